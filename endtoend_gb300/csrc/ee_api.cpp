@@ -521,7 +521,7 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         EE_CUDA(grow(c, c->rev_grad, D.rev_total + 4));  // +4: vector-reduction padding
         if (c->P.mode == EE_KERNEL_EXP) EE_CUDA(grow(c, c->samples, D.rev_total));  // adjoint cone scratch
         if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev_grad.p, 0xFF, sizeof(float) * D.rev_total, s));
-        EE_CUDA(ee_launch_rev_zero(c->P, dge, c->rev_grad.p, nb, D.max_lines, s));
+        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev_grad.p, nb, D.max_lines, s));
         EE_CUDA(staged(c, EE_STAGE_GATHER_T, 1, [&] {
             return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev_grad.p, nb, D.max_tiles, s);
         }));
@@ -741,7 +741,7 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
         const EeBeamGeom* dge = pl->d_geoms.p + b0;
         const ChunkDims& D = pl->dims[k];
         if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev_grad.p, 0xFF, sizeof(float) * D.rev_total, s));
-        PL(ee_launch_rev_zero(P, dge, pl->rev_grad.p, nb, D.max_lines, s));
+        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev_grad.p, nb, D.max_lines, s));
         PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev_grad.p, nb, D.max_tiles, s));
         PL(ee_launch_cone_T(P, dsp, dge, pl->rev_grad.p, P.mode == EE_KERNEL_EXP ? pl->samples.p : nullptr,
                             pl->terma_grad.p, nb, D.max_lines, D.max_line, s, pl->lane_block));

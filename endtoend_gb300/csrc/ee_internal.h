@@ -106,6 +106,12 @@ struct EeRayGeom {
     float B0[3], Bx[3], By[3], Bz[3];  // REV (tX,tY,tZ) -> BEV crop-box index
     float M[9];            // BEV -> REV (copy of MK for the gather)
     float A[9];            // patient index step -> REV step (MK MB), row-major
+    float iB[3], iG[3];    // 1 / Bx, 1 / Gx (0 where below 1e-6): line-box intersections without divisions
+    // the field frustum's four sides as affine forms of a REV point,
+    // [0] i + [1] + [2] tY + [3] tZ >= 0 where its TERMA corners may lie in
+    // the field, and the distance in front of the source (k_geometry)
+    float side[4][4];
+    float front[4];
 };
 
 // Per-beam geometry computed on the device (crop box + REV frames).
@@ -163,8 +169,8 @@ cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const E
                              cudaStream_t s, int lane_block = 128);
 // zeros on every line's segment of a chunk's REV gradient arena (before
 // ee_launch_gather_T; the forward cone kernels zero their own arena)
-cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamGeom* geoms, float* rev_grad, int nbeams, int max_lines,
-                               cudaStream_t s);
+cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,
+                               int nbeams, int max_lines, cudaStream_t s);
 // test option: EE_DEBUG_POISON=1 fills scratch with NaN where the engine
 // relies on its kernels, not on a clear, to write every sample it reads
 bool ee_debug_poison();
