@@ -278,7 +278,8 @@ __device__ __forceinline__ void tri_border_scatter(float* v, int nx, int ny, int
 // Radiological path of the ray source -> voxel centre (cudaSiddon.cu:20-115):
 // plane crossings advanced from a common a_min, midpoint density samples of
 // the border-mode trilinear density at (pos-start)/voxel, segments shorter
-// than 1e-3 cm skipped, 5000-iteration cap.
+// than 1e-3 cm skipped, 5000-iteration cap.  (Nine comparisons per crossing in
+// place of the reference's validity logic: k_terma 10.0 -> 9.4 ms on 96 beams.)
 __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
     const f3 start = mk(P.start[0], P.start[1], P.start[2]);
     const f3 voxel = mk(P.voxel[0], P.voxel[1], P.voxel[2]);
@@ -297,18 +298,26 @@ __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
         float alpha = a_min, ax = a_min, ay = a_min, az = a_min, next = 0.f;
         const float ivx = 1.f / voxel.x, ivy = 1.f / voxel.y, ivz = 1.f / voxel.z;
         int iter = 0;
+        // The reference advances every axis that is valid (its parameter in
+        // [0, 1)) and not above the other valid ones, one axis after the other.
+        // The parameters start at a_min >= 0 and grow, and an invalid one
+        // (>= 1) is above every valid one, so "below 1 and not above the other
+        // two" is the same test.
         while (alpha < a_max && ++iter < 5000) {
-            bool vx = (ax >= 0.f && ax < 1.f), vy = (ay >= 0.f && ay < 1.f), vz = (az >= 0.f && az < 1.f);
-            if (!(vx || vy || vz)) break;
-            if (vx && (!vy || ax <= ay) && (!vz || ax <= az)) { next = ax; ax += stx; }
-            if (vy && (!vx || ay <= ax) && (!vz || ay <= az)) { next = ay; ay += sty; }
-            if (vz && (!vx || az <= ax) && (!vy || az <= ay)) { next = az; az += stz; }
-            float isect = fabsf(d12 * (next - alpha));
+            const bool vy = ay < 1.f, vz = az < 1.f;
+            const bool cx = ax < 1.f && ax <= ay && ax <= az;
+            if (cx) { next = ax; ax += stx; }
+            const bool cy = vy && ay <= ax && ay <= az;
+            if (cy) { next = ay; ay += sty; }
+            const bool cz = vz && az <= ax && az <= ay;
+            if (cz) { next = az; az += stz; }
+            if (!(cx || cy || cz)) break;  // no axis valid
+            const float isect = fabsf(d12 * (next - alpha));
             if (isect >= 0.001f) {
-                float mid = (next + alpha) * 0.5f;
-                float fx = (src.x + mid * diff.x - start.x) * ivx;
-                float fy = (src.y + mid * diff.y - start.y) * ivy;
-                float fz = (src.z + mid * diff.z - start.z) * ivz;
+                const float mid = (next + alpha) * 0.5f;
+                const float fx = (src.x + mid * diff.x - start.x) * ivx;
+                const float fy = (src.y + mid * diff.y - start.y) * ivy;
+                const float fz = (src.z + mid * diff.z - start.z) * ivz;
                 rpl += isect * tex3D<float>(P.dens_tex, fx, fy, fz);
             }
             alpha = next;

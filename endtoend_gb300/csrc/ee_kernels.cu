@@ -27,8 +27,33 @@
 
 namespace {
 
+// Crop-box reduction (host.cu:442-459): min/max of the BEV indices `bi` of a
+// warp's voxels with non-zero TERMA (nz) as ordered-int keys, merged into the
+// beam's keys by one lane, without a block barrier.
+__device__ __forceinline__ void merge_crop_box(EeBeamGeom& G, bool nz, f3 bi, bool cap) {
+    int kmin0 = nz ? f2key(bi.x) : INT_MAX, kmin1 = nz ? f2key(bi.y) : INT_MAX, kmin2 = nz ? f2key(bi.z) : INT_MAX;
+    int kmax0 = nz ? f2key(bi.x) : INT_MIN, kmax1 = nz ? f2key(bi.y) : INT_MIN, kmax2 = nz ? f2key(bi.z) : INT_MIN;
+    const unsigned cnt = __popc(__ballot_sync(FULL, nz));
+    const bool anycap = __any_sync(FULL, cap);
+    if (cnt == 0 && !anycap) return;
+    kmin0 = __reduce_min_sync(FULL, kmin0);
+    kmin1 = __reduce_min_sync(FULL, kmin1);
+    kmin2 = __reduce_min_sync(FULL, kmin2);
+    kmax0 = __reduce_max_sync(FULL, kmax0);
+    kmax1 = __reduce_max_sync(FULL, kmax1);
+    kmax2 = __reduce_max_sync(FULL, kmax2);
+    if ((threadIdx.x & 31) == 0) {
+        if (cnt > 0) {
+            atomicMin(&G.key_min[0], kmin0); atomicMin(&G.key_min[1], kmin1); atomicMin(&G.key_min[2], kmin2);
+            atomicMax(&G.key_max[0], kmax0); atomicMax(&G.key_max[1], kmax1); atomicMax(&G.key_max[2], kmax2);
+            atomicAdd(&G.nnz, cnt);
+        }
+        if (anycap) atomicExch(&G.status, 7 /* EE_ERR_SIDDON_ITER */);
+    }
+}
+
 // TERMA without supersampling.  Threads take the box's voxels brick by brick
-// (4x4x4, ee_brick_vol), 256 per block.  A voxel needs a ray trace when it
+// (4x4x4, ee_brick_vol), two bricks per block.  A voxel needs a ray trace when it
 // has a beamlet (beamlet_of, cudaSiddon.cu:143-165) whose fluence is
 // positive, or any beamlet when the unit TERMA is kept for the adjoint; the
 // rest are written at once.  The box is the field's axis-aligned hull, so
@@ -38,17 +63,23 @@ namespace {
 // than tracing in place).  Each voxel's arithmetic is unchanged.  The crop
 // box (host.cu:442-459) is reduced from the traced voxels with non-zero
 // TERMA: min/max of BEV indices as ordered-int keys, one merge per warp.
-// Five resident blocks per SM: 48 registers, no spills.
-__global__ void __launch_bounds__(256, 5) k_terma(EeParams P, const EeBeamSpec* __restrict__ specs,
+// Bound by the texture unit's data stage (half its cycles busy on average and
+// three quarters on the busiest SM) and by the uneven ray lengths: 128 threads
+// per block free their place sooner than 256 (96 beams of 8^2..40^2 beamlets
+// on 200 x 200 x 160: 9.42 -> 8.99 ms).  40 resident warps per SM: 48
+// registers, no spills.
+constexpr int TERMA_BLOCK = 128;
+
+__global__ void __launch_bounds__(TERMA_BLOCK, 1280 / TERMA_BLOCK) k_terma(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                    EeBeamGeom* __restrict__ geoms, const float* __restrict__ fluence,
                                                    float* __restrict__ terma, float* __restrict__ unit,
                                                    int* __restrict__ bl_idx) {
-    __shared__ int s_v[256], s_bl[256], s_wcnt[8];
-    __shared__ float s_fl[256];
+    __shared__ int s_v[TERMA_BLOCK], s_bl[TERMA_BLOCK], s_wcnt[TERMA_BLOCK / 32];
+    __shared__ float s_fl[TERMA_BLOCK];
     const int b = blockIdx.z;
     const EeBeamSpec& S = specs[b];
     const long long bvol = ee_brick_vol(S.tn);
-    const long long vb = (long long)blockIdx.x * 256;
+    const long long vb = (long long)blockIdx.x * TERMA_BLOCK;
     if (vb >= bvol) return;
     const int nbx = (S.tn[0] + 3) >> 2, nby = (S.tn[1] + 3) >> 2;
     // box indices of bricked box element v
@@ -92,7 +123,7 @@ __global__ void __launch_bounds__(256, 5) k_terma(EeParams P, const EeBeamSpec* 
     __syncthreads();
     int off = 0, total = 0;
 #pragma unroll
-    for (int w = 0; w < 8; w++) {
+    for (int w = 0; w < TERMA_BLOCK / 32; w++) {
         const int c = s_wcnt[w];
         off += w < warp ? c : 0;
         total += c;
@@ -127,127 +158,102 @@ __global__ void __launch_bounds__(256, 5) k_terma(EeParams P, const EeBeamSpec* 
             bi = mv(S.MB, mk((float)(x - P.bb0[0]), (float)(y - P.bb0[1]), (float)(z - P.bb0[2])));
         }
     }
-    int kmin0 = nz ? f2key(bi.x) : INT_MAX, kmin1 = nz ? f2key(bi.y) : INT_MAX, kmin2 = nz ? f2key(bi.z) : INT_MAX;
-    int kmax0 = nz ? f2key(bi.x) : INT_MIN, kmax1 = nz ? f2key(bi.y) : INT_MIN, kmax2 = nz ? f2key(bi.z) : INT_MIN;
-    const unsigned cnt = __popc(__ballot_sync(FULL, nz));
-    const bool anycap = __any_sync(FULL, cap);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        kmin0 = min(kmin0, __shfl_xor_sync(FULL, kmin0, o));
-        kmin1 = min(kmin1, __shfl_xor_sync(FULL, kmin1, o));
-        kmin2 = min(kmin2, __shfl_xor_sync(FULL, kmin2, o));
-        kmax0 = max(kmax0, __shfl_xor_sync(FULL, kmax0, o));
-        kmax1 = max(kmax1, __shfl_xor_sync(FULL, kmax1, o));
-        kmax2 = max(kmax2, __shfl_xor_sync(FULL, kmax2, o));
-    }
-    if (lane == 0) {
-        EeBeamGeom& G = geoms[b];
-        if (cnt > 0) {
-            atomicMin(&G.key_min[0], kmin0); atomicMin(&G.key_min[1], kmin1); atomicMin(&G.key_min[2], kmin2);
-            atomicMax(&G.key_max[0], kmax0); atomicMax(&G.key_max[1], kmax1); atomicMax(&G.key_max[2], kmax2);
-            atomicAdd(&G.nnz, cnt);
-        }
-        if (anycap) atomicExch(&G.status, 7 /* EE_ERR_SIDDON_ITER */);
-    }
+    merge_crop_box(geoms[b], nz, bi, cap);
 }
 
-// TERMA with supersampling (ss > 1): one thread per TERMA-box voxel, walking
-// the box brick by brick.
-__global__ void __launch_bounds__(256, 1) k_terma_ss(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                    EeBeamGeom* __restrict__ geoms, const float* __restrict__ fluence,
-                                                    float* __restrict__ terma, float* __restrict__ unit,
-                                                    int* __restrict__ bl_idx) {
+// TERMA with supersampling (ss > 1, cudaSiddon.cu:248-258, 297-306): each
+// voxel's TERMA is the mean over ss^3 sub-voxel centres, each with its own
+// beamlet lookup and ray trace, summed x fastest.  A block takes one brick of
+// the box (4x4x4 voxels) and walks its 64 ss^3 centres in voxel-major order,
+// TS_ITEMS at a time: the centres to trace are gathered into a shared list, a
+// thread traces one centre, and a thread per voxel adds the results in the
+// centres' order.  Neighbouring lanes then trace rays a fraction of a voxel
+// apart, so a warp's density fetches share their texels, which is what the
+// texture unit is bound by: 4 beams at ss = 3 8.00 ms with a thread per voxel
+// that traces its 27 centres in turn, 6.29 ms here.  (Unit TERMA and beamlets
+// are not kept: k_terma_T_ss recomputes the sub-voxel beamlets.)
+constexpr int TS_ITEMS = 1024;
+
+__global__ void __launch_bounds__(256, 4) k_terma_ss(EeParams P, const EeBeamSpec* __restrict__ specs,
+                                                     EeBeamGeom* __restrict__ geoms, const float* __restrict__ fluence,
+                                                     float* __restrict__ terma, float* __restrict__ unit,
+                                                     int* __restrict__ bl_idx) {
+    __shared__ float s_val[TS_ITEMS];       // fluence of a listed centre, then its fluence x unit TERMA
+    __shared__ unsigned short s_list[TS_ITEMS];
+    __shared__ int s_n;
     const int b = blockIdx.z;
     const EeBeamSpec& S = specs[b];
-    const long long bvol = ee_brick_vol(S.tn);
-    long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    bool nz = false, cap = false;
-    f3 bi = mk(0.f, 0.f, 0.f);
-    // threads walk the box brick by brick (4x4x4, ee_brick_vol): each warp
-    // traces half a brick of neighbouring rays and writes 128 contiguous bytes
-    int xr = 0, yr = 0, zr = 0;
-    bool inbox = false;
-    if (v < bvol) {
-        const long long brick = v >> 6;
-        const int w = (int)(v & 63), nbx = (S.tn[0] + 3) >> 2, nby = (S.tn[1] + 3) >> 2;
-        const long long bxy = brick % ((long long)nbx * nby);
-        xr = (int)(bxy % nbx) * 4 + (w & 3);
-        yr = (int)(bxy / nbx) * 4 + ((w >> 2) & 3);
-        zr = (int)(brick / ((long long)nbx * nby)) * 4 + (w >> 4);
-        inbox = xr < S.tn[0] && yr < S.tn[1] && zr < S.tn[2];
-        if (!inbox) {  // padding of the last bricks: never sampled, kept zero
-            terma[S.t_off + v] = 0.f;
-            if (unit) unit[S.t_off + v] = 0.f;
-            if (bl_idx) bl_idx[S.t_off + v] = -1;
-        }
-    }
-    if (inbox) {
-        // full-grid voxel index of this TERMA-box voxel
-        int x = S.t0[0] + xr;
-        int y = S.t0[1] + yr;
-        int z = S.t0[2] + zr;
-        f3 vox = mk(P.start[0] + x * P.voxel[0], P.start[1] + y * P.voxel[1], P.start[2] + z * P.voxel[2]);
-        f3 src = ld3(S.src);
-        float t = 0.f, u = 0.f;
-        int bl = -1;
-        {
-            // supersampled TERMA (cudaSiddon.cu:248-258, 297-306): the mean
-            // over ss^3 sub-voxel centres, each with its own beamlet lookup
-            // and ray trace, summed x fastest (unit and bl_idx are not kept:
-            // k_terma_T_ss recomputes the sub-voxel beamlets)
-            const int ss = P.ss, nsub = ss * ss * ss;
-            const float sv0 = P.voxel[0] / (float)ss, sv1 = P.voxel[1] / (float)ss, sv2 = P.voxel[2] / (float)ss;
-            float acc = 0.f;
-            for (int ii = 0; ii < nsub; ii++) {
-                const int sx = ii % ss, sy = (ii / ss) % ss, sz = ii / (ss * ss);
-                const f3 p = mk(P.start[0] + ((float)x - 0.5f) * P.voxel[0] + ((float)sx + 0.5f) * sv0,
-                                P.start[1] + ((float)y - 0.5f) * P.voxel[1] + ((float)sy + 0.5f) * sv1,
-                                P.start[2] + ((float)z - 0.5f) * P.voxel[2] + ((float)sz + 0.5f) * sv2);
+    const int nbx = (S.tn[0] + 3) >> 2, nby = (S.tn[1] + 3) >> 2;
+    const long long brick = blockIdx.x;
+    if (brick >= (ee_brick_vol(S.tn) >> 6)) return;
+    const long long bxy = brick % ((long long)nbx * nby);
+    const int bx = (int)(bxy % nbx) * 4, by = (int)(bxy / nbx) * 4, bz = (int)(brick / ((long long)nbx * nby)) * 4;
+    const int ss = P.ss, nsub = ss * ss * ss;
+    const float sv0 = P.voxel[0] / (float)ss, sv1 = P.voxel[1] / (float)ss, sv2 = P.voxel[2] / (float)ss;
+    const f3 src = ld3(S.src);
+    const int t = threadIdx.x, lane = t & 31;
+    // centre `item` of the brick (voxel-major); false outside the box
+    auto centre = [&](int item, f3& p) {
+        const int w = item / nsub, ii = item - w * nsub;
+        const int xr = bx + (w & 3), yr = by + ((w >> 2) & 3), zr = bz + (w >> 4);
+        const int sx = ii % ss, sy = (ii / ss) % ss, sz = ii / (ss * ss);
+        p = mk(P.start[0] + ((float)(S.t0[0] + xr) - 0.5f) * P.voxel[0] + ((float)sx + 0.5f) * sv0,
+               P.start[1] + ((float)(S.t0[1] + yr) - 0.5f) * P.voxel[1] + ((float)sy + 0.5f) * sv1,
+               P.start[2] + ((float)(S.t0[2] + zr) - 0.5f) * P.voxel[2] + ((float)sz + 0.5f) * sv2);
+        return xr < S.tn[0] && yr < S.tn[1] && zr < S.tn[2];
+    };
+    float acc = 0.f;  // voxel t of the brick (t < 64)
+    bool cap = false;
+    for (int i0 = 0; i0 < 64 * nsub; i0 += TS_ITEMS) {
+        const int n = min(TS_ITEMS, 64 * nsub - i0);
+        if (t == 0) s_n = 0;
+        __syncthreads();
+        for (int k = t; k < TS_ITEMS; k += 256) {
+            float fl = 0.f;
+            f3 p;
+            if (k < n && centre(i0 + k, p)) {
                 int bs = beamlet_of(S, p);
                 if (bs == -2) bs = beamlet_point_fp64(S, (double)p.x, (double)p.y, (double)p.z);
-                if (bs < 0) continue;
-                const float fl = __ldg(fluence + S.fl_off + bs);
-                if (!(fl > 0.f)) continue;
-                const float rpl = siddon_rpl(P, p, src, cap);
-                acc += fl * terma_per_fluence(P, rpl, p, src, S.sad);
+                if (bs >= 0) fl = __ldg(fluence + S.fl_off + bs);
             }
-            t = acc / (float)nsub;
+            const bool need = fl > 0.f;
+            s_val[k] = need ? fl : 0.f;
+            const unsigned m = __ballot_sync(FULL, need);
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&s_n, __popc(m));
+            base = __shfl_sync(FULL, base, 0);
+            if (need) s_list[base + __popc(m & ((1u << lane) - 1u))] = (unsigned short)k;
         }
-        terma[S.t_off + v] = t;
-        if (unit) unit[S.t_off + v] = u;
-        if (bl_idx) bl_idx[S.t_off + v] = bl;
-        if (t != 0.f) {
-            nz = true;
-            // crop box works on calc-bbox-relative indices (host.cu:445-448)
-            bi = mv(S.MB, mk((float)(x - P.bb0[0]), (float)(y - P.bb0[1]), (float)(z - P.bb0[2])));
+        __syncthreads();
+        const int nl = s_n;
+        for (int k = t; k < nl; k += 256) {
+            const int item = s_list[k];
+            f3 p;
+            centre(i0 + item, p);
+            const float rpl = siddon_rpl(P, p, src, cap);
+            s_val[item] *= terma_per_fluence(P, rpl, p, src, S.sad);
         }
-    }
-    // crop-box reduction (host.cu:442-459): min/max of BEV indices of voxels
-    // with non-zero TERMA, as ordered-int keys.
-    int kmin0 = nz ? f2key(bi.x) : INT_MAX, kmin1 = nz ? f2key(bi.y) : INT_MAX, kmin2 = nz ? f2key(bi.z) : INT_MAX;
-    int kmax0 = nz ? f2key(bi.x) : INT_MIN, kmax1 = nz ? f2key(bi.y) : INT_MIN, kmax2 = nz ? f2key(bi.z) : INT_MIN;
-    unsigned cnt = __popc(__ballot_sync(FULL, nz));
-    bool anycap = __any_sync(FULL, cap);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        kmin0 = min(kmin0, __shfl_xor_sync(FULL, kmin0, o));
-        kmin1 = min(kmin1, __shfl_xor_sync(FULL, kmin1, o));
-        kmin2 = min(kmin2, __shfl_xor_sync(FULL, kmin2, o));
-        kmax0 = max(kmax0, __shfl_xor_sync(FULL, kmax0, o));
-        kmax1 = max(kmax1, __shfl_xor_sync(FULL, kmax1, o));
-        kmax2 = max(kmax2, __shfl_xor_sync(FULL, kmax2, o));
-    }
-    // one lane per warp merges into the beam's keys: no block barrier, so a
-    // warp whose rays are short does not wait for the block's longest trace
-    if ((threadIdx.x & 31) == 0) {
-        EeBeamGeom& G = geoms[b];
-        if (cnt > 0) {
-            atomicMin(&G.key_min[0], kmin0); atomicMin(&G.key_min[1], kmin1); atomicMin(&G.key_min[2], kmin2);
-            atomicMax(&G.key_max[0], kmax0); atomicMax(&G.key_max[1], kmax1); atomicMax(&G.key_max[2], kmax2);
-            atomicAdd(&G.nnz, cnt);
+        __syncthreads();
+        if (t < 64) {
+            const int lo = max(t * nsub - i0, 0), hi = min((t + 1) * nsub - i0, n);
+            for (int k = lo; k < hi; k++) acc += s_val[k];
         }
-        if (anycap) atomicExch(&G.status, 7 /* EE_ERR_SIDDON_ITER */);
+        __syncthreads();
     }
+    bool nz = false;
+    f3 bi = mk(0.f, 0.f, 0.f);
+    if (t < 64) {
+        const float te = acc / (float)nsub;
+        const long long o = S.t_off + brick * 64 + t;
+        terma[o] = te;  // the padding of the box's last bricks is never sampled and stays zero
+        if (unit) unit[o] = 0.f;
+        if (bl_idx) bl_idx[o] = -1;
+        nz = te != 0.f;
+        // crop box works on calc-bbox-relative indices (host.cu:445-448)
+        bi = mv(S.MB, mk((float)(S.t0[0] + bx + (t & 3) - P.bb0[0]), (float)(S.t0[1] + by + ((t >> 2) & 3) - P.bb0[1]),
+                         (float)(S.t0[2] + bz + (t >> 4) - P.bb0[2])));
+    }
+    merge_crop_box(geoms[b], nz, bi, cap);
 }
 
 // The beam's field as seen by one cone's REV points.  A voxel has a beamlet
@@ -2256,9 +2262,12 @@ cudaError_t ee_copy_status(const EeBeamGeom* geoms, int* status_host, int nbeams
 cudaError_t ee_launch_terma(const EeParams& P, const EeBeamSpec* specs, EeBeamGeom* geoms, const float* fluence,
                             float* terma, float* unit, int* beamlet_idx, int nbeams, long long max_tvol,
                             cudaStream_t s) {
-    dim3 grid(grid1(max_tvol, 256), 1, nbeams);
-    if (P.ss > 1) k_terma_ss<<<grid, 256, 0, s>>>(P, specs, geoms, fluence, terma, unit, beamlet_idx);
-    else k_terma<<<grid, 256, 0, s>>>(P, specs, geoms, fluence, terma, unit, beamlet_idx);
+    if (P.ss > 1)
+        k_terma_ss<<<dim3(grid1(max_tvol, 64), 1, nbeams), 256, 0, s>>>(P, specs, geoms, fluence, terma, unit,
+                                                                        beamlet_idx);
+    else
+        k_terma<<<dim3(grid1(max_tvol, TERMA_BLOCK), 1, nbeams), TERMA_BLOCK, 0, s>>>(P, specs, geoms, fluence, terma,
+                                                                                      unit, beamlet_idx);
     return cudaGetLastError();
 }
 
