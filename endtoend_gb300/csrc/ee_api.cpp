@@ -1343,7 +1343,9 @@ int ee_beamlet_columns_device(ee_context* c, const ee_beam* beam, const float* f
     cudaSetDevice(c->device);
     EeBeamSpec S;
     build_specs(c->P, beam, 1, &S);
-    return ee_beamlet_run(c->P, c->rays.data(), c->stream, &c->beamlet_ws, c->bl_opt, *beam, S, fluence, thresh, out);
+    EeBeamletOptions opt = c->bl_opt;
+    opt.scratch_bytes = c->max_batch_bytes;
+    return ee_beamlet_run(c->P, c->rays.data(), c->stream, &c->beamlet_ws, opt, *beam, S, fluence, thresh, out);
 }
 
 int ee_copy_to_host(ee_context* c, void* dst, const void* src, long long bytes) {

@@ -191,6 +191,7 @@ cudaError_t ee_launch_smooth(const EeBeamSpec* specs, const float* x, float* gra
 struct EeBeamletOptions {
     float kernel_extent;  // dose kernel truncation, cm (argparser.h:27: 2 cm)
     int max_rev[3];       // REV size limit that triggers re-batching (argparser.h:29: 500^3)
+    long long scratch_bytes = 0;  // the context's scratch budget: directions whose REV arrays share a launch
 };
 int ee_beamlet_run(const EeParams& P, const EeRayConst* rays, cudaStream_t s, void** ws, const EeBeamletOptions& opt,
                    const ee_beam& beam, const EeBeamSpec& S, const float* fluence_host, float thresh, ee_csr* out);
