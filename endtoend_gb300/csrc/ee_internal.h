@@ -112,7 +112,16 @@ struct EeRayGeom {
     // the field, and the distance in front of the source (k_geometry)
     float side[4][4];
     float front[4];
+    // half-planes [0] tY + [1] tZ + [2] >= 0 that hold every line with a field
+    // span ("lit"; k_geometry), [0], [1] a unit normal (or 0, 0, 1: no bound)
+    float lit[4][3];
 };
+
+// A lit line's forms are >= 0.  The gathers visit a voxel and cone only where
+// one of the four lines around the voxel can be lit; such a line is within one
+// cell per axis of the voxel, the lines that k_gather then reads within one
+// more, so a line whose least form is below this is never read.
+constexpr float EE_LIT_READ = -2.95f;  // -2 sqrt(2), and rounding
 
 // Per-beam geometry computed on the device (crop box + REV frames).
 struct EeBeamGeom {

@@ -1,7 +1,8 @@
 """The exp cone kernels walk only the part of a line that the beam's field can
-reach: dose against the FP64 oracle and the adjoint through the dot-product
-identity, for fields that most lines miss, fields wider than the volume, and
-oblique fields at a corner.
+reach, and the gathers visit only the cones whose lines it can reach: dose
+against the FP64 oracle and the adjoint through the dot-product identity, for
+fields that most lines miss, fields wider than the volume, oblique fields at a
+corner, and voxels that are not cubes (where lines are not bounded).
 
 Tolerances: dose 1e-3 of Dmax (the engine's bound against the FP64 oracle:
 texture filter weights of 8 bits and FP32 geometry); <g, A f> = <A^T g, f> to
@@ -29,7 +30,19 @@ CASES = [
 @pytest.mark.parametrize("shape,voxel,spacing,fmap,beamlet,angles,iso,ss", CASES)
 @pytest.mark.parametrize("mode", ["exp", "table"])
 def test_dose_and_adjoint_by_field(shape, voxel, spacing, fmap, beamlet, angles, iso, ss, mode):
-    vol = inputs.head_neck_phantom(shape=shape, voxel_cm=voxel)
+    check(inputs.head_neck_phantom(shape=shape, voxel_cm=voxel), shape, spacing, fmap, beamlet, angles, iso, ss, mode)
+
+
+@pytest.mark.parametrize("mode", ["exp", "table"])
+def test_voxels_that_are_not_cubes(mode):
+    shape = (37, 30, 33)
+    vol = inputs.head_neck_phantom(shape=shape, voxel_cm=0.27)
+    vol.voxel = np.array([0.31, 0.24, 0.27])
+    vol.start = -0.5 * (np.array(shape) - 1) * vol.voxel
+    check(vol, shape, 0.27, (4, 3), 0.4, (62.0, 21.0, 9.0), inputs.ISO_OFFSET_CM, 1, mode)
+
+
+def check(vol, shape, spacing, fmap, beamlet, angles, iso, ss, mode):
     rng = np.random.default_rng(sum(shape))
     vol.density[:] = rng.uniform(0.9, 1.1, vol.density.shape)
     phys = inputs.make_physics(seed=3, spacing_cm=spacing)
