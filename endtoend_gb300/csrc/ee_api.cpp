@@ -5,13 +5,14 @@
 // beam and one cone at a time, CCCS/dosecalc-beam/nvbbRayConvolve_host.cu:376-725):
 //   H2D beam specs -> k_geom_init -> k_terma (+crop-box reduction)
 //   -> k_geometry -> [one read-back of the per-beam geometry: REV arena
-//   offsets] -> k_cone (all cones of all beams) -> k_gather (all cones of all
-//   beams accumulated per voxel).
+//   sizes] -> per chunk of beams whose arenas fit the scratch budget: k_cone
+//   (all cones of its beams) -> k_gather (all cones accumulated per voxel).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -149,6 +150,41 @@ struct PinBuf {
     }
 };
 
+// Device buffers of the lane cones (EeConeWork) for lines of max_line samples
+// and `segments` lists of `tiles` tiles in all.
+struct ConeBufs {
+    DevBuf<float4> scratch;
+    DevBuf<int> counts, tiles;
+    static size_t scratch_size(int max_line, long long limit) {
+        return (size_t)64 * ee_cone_quads(max_line) * ee_cone_warps(max_line, limit);
+    }
+    bool fits(int max_line, long long segments, long long ntiles, long long limit) const {
+        return scratch.n >= scratch_size(max_line, limit) && counts.n >= (size_t)(1 + segments) &&
+               tiles.n >= (size_t)ntiles;
+    }
+    cudaError_t ensure(int max_line, long long segments, long long ntiles, long long limit) {
+        cudaError_t e = scratch.ensure(scratch_size(max_line, limit));
+        if (e == cudaSuccess) e = counts.ensure((size_t)(1 + segments));
+        if (e == cudaSuccess) e = tiles.ensure((size_t)ntiles);
+        return e;
+    }
+    EeConeWork work(int max_line, long long limit) const {
+        EeConeWork w;
+        w.scratch = scratch.p;
+        w.counts = counts.p;
+        w.tiles = tiles.p;
+        w.quads = ee_cone_quads(max_line);
+        w.warps = ee_cone_warps(max_line, limit);
+        return w;
+    }
+    long long bytes() const { return 16ll * scratch.n + 4ll * (counts.n + tiles.n); }
+    void release() {
+        scratch.release();
+        counts.release();
+        tiles.release();
+    }
+};
+
 }  // namespace
 
 struct ee_context {
@@ -167,16 +203,16 @@ struct ee_context {
     // per-call scratch
     DevBuf<EeBeamSpec> d_specs;
     DevBuf<EeBeamGeom> d_geoms;
-    DevBuf<float> terma, unit, rev, rev_grad, terma_grad;
-    DevBuf<float2> samples;  // per-REV-sample (rho, T) / (contribution, rho) of the exp-mode cone kernels
+    DevBuf<float> terma, unit, terma_grad;
+    DevBuf<float> rev;  // a chunk's REV dose, then (adjoint) its REV gradient
+    ConeBufs cone;
     DevBuf<int> bl_idx;
     DevBuf<float> io_fluence, io_dose, io_grad;
     DevBuf<float> xf, xg, spread_w;
     DevBuf<double> acc;
     PinBuf<EeBeamSpec> h_specs;
-    PinBuf<EeBeamGeom> h_geoms;
-    std::vector<EeBeamGeom> last_geoms;
-    std::vector<EeBeamSpec> last_specs;
+    PinBuf<EeBeamGeomHead> h_geoms;
+    std::vector<ee_beam_info> last_info;  // of the last call's beams
     long long max_batch_bytes = 8ll << 30;  // scratch budget for one chunk of beams
     // profiling
     bool profiling = false;
@@ -220,7 +256,7 @@ int check_beams(const ee_beam* beams, int nbeams) {
 // convex hull of 8 vertices), widened by one voxel and clipped to the bbox.
 // TERMA is zero outside it: a voxel gets TERMA only when its projection onto
 // the isocentre plane lands inside the fluence map (cudaSiddon.cu:143-165).
-void terma_box(const EeParams& P, const EeBeamSpec& S, int t0[3], int tn[3]) {
+void terma_box(const EeParams& P, EeBeamSpec& S, int t0[3], int tn[3]) {
     const d3 src = {S.src[0], S.src[1], S.src[2]}, dir = {S.dir[0], S.dir[1], S.dir[2]};
     double dmin = 1e300, dmax = -1e300;
     for (int c = 0; c < 8; c++) {
@@ -233,6 +269,8 @@ void terma_box(const EeParams& P, const EeBeamSpec& S, int t0[3], int tn[3]) {
         dmin = std::min(dmin, d);
         dmax = std::max(dmax, d);
     }
+    S.dnear = (float)dmin;
+    S.dfar = (float)dmax;
     for (int a = 0; a < 3; a++) { t0[a] = P.bb0[a]; tn[a] = 0; }
     if (dmax <= 0) return;  // the bbox lies behind the source
     if (dmin <= 1e-3 * S.isodist) {
@@ -351,32 +389,42 @@ cudaError_t staged(ee_context* c, int stage, int nlaunch, F fn) {
 
 long long nfull_of(const ee_context* c) { return (long long)c->P.size[0] * c->P.size[1] * c->P.size[2]; }
 
-// Beams per chunk so that TERMA (+unit/index for the adjoint) fits the budget.
-// Split the beams into chunks whose REV arena fits the scratch budget
-// (estimate: nrays x 4 x the TERMA box per beam, x2 with the adjoint's REV
-// gradient).  TERMA boxes of all beams stay resident for the whole call so
-// the adjoint reuses the forward's TERMA, crop boxes and REV frames.
-std::vector<int> plan_chunks(const ee_context* c, const EeBeamSpec* specs, int nbeams, bool adjoint) {
-    std::vector<int> starts;
-    long long acc = 0;
-    // REV arena + (rho, T) sample scratch (+ REV gradient for the adjoint)
-    const long long per_vox = 4ll * (long long)c->P.nrays * 4 * (adjoint ? 4 : 3);
-    for (int b = 0; b < nbeams; b++) {
-        long long need = std::max(1ll, tvol_of(specs[b])) * per_vox;
-        if (starts.empty() || (acc + need > c->max_batch_bytes && acc > 0)) {
-            starts.push_back(b);
-            acc = 0;
-        }
-        acc += need;
+ee_beam_info beam_info(const EeBeamSpec& S, const EeBeamGeomHead& G) {
+    ee_beam_info info;
+    std::memset(&info, 0, sizeof(info));
+    for (int a = 0; a < 3; a++) {
+        info.source[a] = S.src[a];
+        info.direction[a] = S.dir[a];
+        info.b_min[a] = G.bmin[a];
+        info.bev_size[a] = G.bev[a];
+        info.lim_min[a] = G.lim_min[a];
     }
-    starts.push_back(nbeams);
-    return starts;
+    info.v_beam = G.v_beam;
+    info.rev_samples = G.rev_total;
+    info.terma_nonzero = G.nnz;
+    info.max_line = G.max_line;
+    info.status = G.status;
+    return info;
 }
+
+constexpr int kTermaBeams = 32768;  // beams per launch: a grid's z extent
 
 struct ChunkDims {
     long long rev_total = 0, max_tvol = 1;
     int max_line = 1, max_lines = 1, max_rows = 1, max_tiles = 1;
 };
+
+// The lane cones' work space for a set of chunks: the longest line, the lists
+// and their tiles of the largest chunk.
+void cone_sizes(int nrays, const std::vector<int>& starts, const std::vector<ChunkDims>& dims, int& max_line,
+                long long& segments, long long& ntiles) {
+    for (size_t k = 0; k < dims.size(); k++) {
+        const long long segs = (long long)nrays * (starts[k + 1] - starts[k]);
+        max_line = std::max(max_line, dims[k].max_line);
+        segments = std::max(segments, segs);
+        ntiles = std::max(ntiles, segs * ee_cone_tiles_cap(dims[k].max_lines));
+    }
+}
 
 // Device buffer growth: a freed buffer may still be read by queued kernels,
 // so drain the stream first when a buffer has to grow.
@@ -410,10 +458,14 @@ struct PipeArgs {
     int ngroups = 1;
 };
 
-// One call of the CCCS chain over a list of beams:
-//   geometry pass per chunk (TERMA + crop box + REV frames, one read-back)
-//   with the forward dose (REV cones + gather) when requested, then the loss
-//   gradient, then the adjoint per chunk reusing the resident TERMA/geometry.
+// One call of the CCCS chain over a list of beams: TERMA, crop boxes and REV
+// frames of all beams (one read-back of their sizes), then chunks of beams
+// whose REV arenas fit the scratch budget: the forward dose (cones + gather)
+// when requested, the loss gradient, and the adjoint, which reuses the
+// resident TERMA and geometry and the same REV arena.  A chunk should hold
+// many beams, or its kernels' last waves leave the chip idle: 96 beams of
+// 8^2..40^2 beamlets took 38.0, 28.3 and 27.4 ms in 46, 9 and 5 chunks, when
+// 8 GiB held two beams; now it holds twenty.
 int pipeline(ee_context* c, const PipeArgs& A) {
     int st = check_ready(c);
     if (st) return st;
@@ -444,52 +496,82 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         EE_CUDA(grow(c, c->terma_grad, tvol_total + 4));  // +4: vector-reduction padding
     }
     EE_CUDA(cudaMemcpyAsync(c->d_specs.p, c->h_specs.p, sizeof(EeBeamSpec) * n, cudaMemcpyHostToDevice, s));
-    std::vector<int> starts = plan_chunks(c, c->h_specs.p, n, adj);
-    const int nchunks = (int)starts.size() - 1;
-    std::vector<ChunkDims> dims(nchunks);
-    c->last_geoms.clear();
-    c->last_specs.assign(c->h_specs.p, c->h_specs.p + n);
+    c->last_info.clear();
     if (fwd && A.dose_mode == EE_DOSE_SUM)
         EE_CUDA(cudaMemsetAsync(A.d_dose, 0, sizeof(float) * nfull * (A.group ? A.ngroups : 1), s));
     if (fwd && A.dose_mode == EE_DOSE_PER_BEAM) EE_CUDA(cudaMemsetAsync(A.d_dose, 0, sizeof(float) * nfull * n, s));
 
-    // ---- geometry + forward, chunk by chunk
-    for (int k = 0; k < nchunks; k++) {
+    // ---- TERMA and geometry of all beams
+    EE_CUDA(staged(c, EE_STAGE_GEOMETRY, 1, [&] { return ee_launch_geom_init(c->d_specs.p, c->d_geoms.p, n, s); }));
+    for (int b0 = 0; b0 < n; b0 += kTermaBeams) {
+        const int nb = std::min(kTermaBeams, n - b0);
+        long long max_tvol = 1;
+        for (int b = b0; b < b0 + nb; b++) max_tvol = std::max(max_tvol, tvol_of(c->h_specs.p[b]));
+        EE_CUDA(staged(c, EE_STAGE_TERMA, 1, [&] {
+            return ee_launch_terma(c->P, c->d_specs.p + b0, c->d_geoms.p + b0, A.d_fluence, c->terma.p,
+                                   adj ? c->unit.p : nullptr, adj ? c->bl_idx.p : nullptr, nb, max_tvol, s);
+        }));
+    }
+    EE_CUDA(staged(c, EE_STAGE_GEOMETRY, 1, [&] { return ee_launch_geometry(c->P, c->d_specs.p, c->d_geoms.p, n, s); }));
+    EeBeamGeomHead* hg = c->h_geoms.p;
+    EE_CUDA(cudaMemcpy2DAsync(hg, sizeof(EeBeamGeomHead), c->d_geoms.p, sizeof(EeBeamGeom), sizeof(EeBeamGeomHead), n,
+                              cudaMemcpyDeviceToHost, s));
+    EE_CUDA(cudaStreamSynchronize(s));
+    std::vector<int> starts;
+    std::vector<ChunkDims> dims;
+    for (int b = 0; b < n; b++) {
+        EeBeamGeomHead& G = hg[b];
+        if (G.status != 0) return fail(G.status, "beam %d: %s", b, status_text(G.status));
+        c->last_info.push_back(beam_info(c->h_specs.p[b], G));
+        // a beam's share of the budget: its REV arena; the lane cones' scratch
+        // takes a quarter at most
+        if (starts.empty() || b - starts.back() >= kTermaBeams ||
+            4 * (dims.back().rev_total + G.store_total) > c->max_batch_bytes / 4 * 3) {
+            starts.push_back(b);
+            dims.push_back(ChunkDims());
+        }
+        ChunkDims& D = dims.back();
+        G.arena_off = D.rev_total;
+        G.arena_cap = G.store_total;
+        D.rev_total += G.store_total;
+        D.max_tvol = std::max(D.max_tvol, tvol_of(c->h_specs.p[b]));
+        D.max_line = std::max(D.max_line, G.max_line);
+        D.max_lines = std::max(D.max_lines, G.max_lines);
+        D.max_rows = std::max(D.max_rows, G.rows);
+        D.max_tiles = std::max(D.max_tiles, G.tiles);
+    }
+    starts.push_back(n);
+    const int nchunks = (int)starts.size() - 1;
+    constexpr size_t at = offsetof(EeBeamGeomHead, arena_off);
+    static_assert(offsetof(EeBeamGeomHead, arena_cap) == at + sizeof(long long), "one copy sets both");
+    EE_CUDA(cudaMemcpy2DAsync((char*)c->d_geoms.p + at, sizeof(EeBeamGeom), (char*)hg + at, sizeof(EeBeamGeomHead),
+                              2 * sizeof(long long), n, cudaMemcpyHostToDevice, s));
+    long long rev_max = 0;
+    for (auto& D : dims) rev_max = std::max(rev_max, D.rev_total);
+    EE_CUDA(grow(c, c->rev, rev_max + 4));  // +4: vector-reduction padding
+    EeConeWork work;
+    if (c->P.mode == EE_KERNEL_EXP) {
+        int max_line = 1;
+        long long segs = 1, ntiles = 1;
+        cone_sizes(c->P.nrays, starts, dims, max_line, segs, ntiles);
+        if (!c->cone.fits(max_line, segs, ntiles, c->max_batch_bytes)) {
+            EE_CUDA(cudaStreamSynchronize(s));  // queued kernels may still use the old buffers
+            EE_CUDA(c->cone.ensure(max_line, segs, ntiles, c->max_batch_bytes));
+        }
+        work = c->cone.work(max_line, c->max_batch_bytes);
+    }
+
+    // ---- forward, chunk by chunk
+    const int cone_launches = work.scratch ? 2 : 1;  // the lane cones list their tiles first
+    for (int k = 0; fwd && k < nchunks; k++) {
         const int b0 = starts[k], nb = starts[k + 1] - b0;
         EeBeamSpec* dsp = c->d_specs.p + b0;
         EeBeamGeom* dge = c->d_geoms.p + b0;
-        ChunkDims& D = dims[k];
-        for (int b = b0; b < b0 + nb; b++) D.max_tvol = std::max(D.max_tvol, tvol_of(c->h_specs.p[b]));
-        EE_CUDA(staged(c, EE_STAGE_GEOMETRY, 1, [&] { return ee_launch_geom_init(dsp, dge, nb, s); }));
-        EE_CUDA(staged(c, EE_STAGE_TERMA, 1, [&] {
-            return ee_launch_terma(c->P, dsp, dge, A.d_fluence, c->terma.p, adj ? c->unit.p : nullptr,
-                                   adj ? c->bl_idx.p : nullptr, nb, D.max_tvol, s);
-        }));
-        EE_CUDA(staged(c, EE_STAGE_GEOMETRY, 1, [&] { return ee_launch_geometry(c->P, dsp, dge, nb, s); }));
-        EeBeamGeom* hg = c->h_geoms.p + b0;
-        EE_CUDA(cudaMemcpyAsync(hg, dge, sizeof(EeBeamGeom) * nb, cudaMemcpyDeviceToHost, s));
-        EE_CUDA(cudaStreamSynchronize(s));
-        for (int b = 0; b < nb; b++) {
-            EeBeamGeom& G = hg[b];
-            if (G.status != 0) return fail(G.status, "beam %d: %s", b0 + b, status_text(G.status));
-            G.arena_off = D.rev_total;
-            G.arena_cap = G.rev_total;
-            D.rev_total += G.rev_total;
-            D.max_line = std::max(D.max_line, G.max_line);
-            D.max_lines = std::max(D.max_lines, G.max_lines);
-            D.max_rows = std::max(D.max_rows, G.rows);
-            D.max_tiles = std::max(D.max_tiles, G.tiles);
-        }
-        EE_CUDA(cudaMemcpyAsync(dge, hg, sizeof(EeBeamGeom) * nb, cudaMemcpyHostToDevice, s));
-        c->last_geoms.insert(c->last_geoms.end(), hg, hg + nb);
-        if (!fwd) continue;
-        EE_CUDA(grow(c, c->rev, D.rev_total));
+        const ChunkDims& D = dims[k];
         // no clear: the cone kernels write every sample k_gather reads
         if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
-        if (c->P.mode == EE_KERNEL_EXP) EE_CUDA(grow(c, c->samples, D.rev_total));
-        EE_CUDA(staged(c, EE_STAGE_CONE, 1, [&] {
-            return ee_launch_cone(c->P, dsp, dge, c->terma.p, c->rev.p,
-                                  c->P.mode == EE_KERNEL_EXP ? c->samples.p : nullptr, nb, D.max_lines, D.max_line, s);
+        EE_CUDA(staged(c, EE_STAGE_CONE, cone_launches, [&] {
+            return ee_launch_cone(c->P, dsp, dge, c->terma.p, c->rev.p, work, nb, D.max_lines, D.max_line, s);
         }));
         float* out = A.dose_mode == EE_DOSE_PER_BEAM ? A.d_dose + (long long)b0 * nfull : A.d_dose;
         const int m = A.dose_mode == EE_DOSE_PER_BEAM ? 2 : 1;
@@ -518,16 +600,13 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         const EeBeamSpec* dsp = c->d_specs.p + b0;
         const EeBeamGeom* dge = c->d_geoms.p + b0;
         const ChunkDims& D = dims[k];
-        EE_CUDA(grow(c, c->rev_grad, D.rev_total + 4));  // +4: vector-reduction padding
-        if (c->P.mode == EE_KERNEL_EXP) EE_CUDA(grow(c, c->samples, D.rev_total));  // adjoint cone scratch
-        if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev_grad.p, 0xFF, sizeof(float) * D.rev_total, s));
-        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev_grad.p, nb, D.max_lines, s));
+        if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
+        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev.p, nb, D.max_lines, s));
         EE_CUDA(staged(c, EE_STAGE_GATHER_T, 1, [&] {
-            return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev_grad.p, nb, D.max_tiles, s);
+            return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev.p, nb, D.max_tiles, s);
         }));
-        EE_CUDA(staged(c, EE_STAGE_CONE_T, 1, [&] {
-            return ee_launch_cone_T(c->P, dsp, dge, c->rev_grad.p, c->P.mode == EE_KERNEL_EXP ? c->samples.p : nullptr,
-                                    c->terma_grad.p, nb, D.max_lines, D.max_line, s);
+        EE_CUDA(staged(c, EE_STAGE_CONE_T, cone_launches, [&] {
+            return ee_launch_cone_T(c->P, dsp, dge, c->rev.p, work, c->terma_grad.p, nb, D.max_lines, D.max_line, s);
         }));
         EE_CUDA(staged(c, EE_STAGE_TERMA_T, 1, [&] {
             return ee_launch_terma_T(c->P, dsp, dge, c->unit.p, c->bl_idx.p, c->terma_grad.p, A.d_fgrad, nb,
@@ -627,6 +706,22 @@ PlanBound plan_bound(const ee_context* c, const EeBeamSpec& S) {
         double bmx = std::max(bhi[a], 0.0) + pen[a] + 1.0;
         bev[a] = std::ceil(bmx - bmn[a]) + 1.0;
     }
+    // lit frustum of the beam in BEV index coordinates (lit_planes)
+    const double vox = P.voxel[0];
+    const bool bounded = P.voxel[1] == P.voxel[0] && P.voxel[2] == P.voxel[0] && S.dnear > 0.02f * S.isodist;
+    double lc[2][3], lh[2][2];
+    if (bounded)
+        for (int e = 0; e < 2; e++) {
+            const double D = e ? (double)S.dfar + 4 * vox : (double)S.dnear - 4 * vox;
+            double p[3];
+            for (int a = 0; a < 3; a++) p[a] = (S.srcd[a] + dir[a] * D - P.start[a]) / vox - P.bb0[a];
+            for (int a = 0; a < 3; a++) lc[e][a] = S.MBd[3 * a] * p[0] + S.MBd[3 * a + 1] * p[1] + S.MBd[3 * a + 2] * p[2];
+            // 1.55 sqrt(3) sqrt(2) (1 + slope) voxels are above any raise of the sides
+            for (int a = 0; a < 2; a++) {
+                const double k = 0.5 * S.fmap[a] * S.beamlet[a] / S.isodistd;
+                lh[e][a] = k * D / vox + 4.0 * (1 + k) + 0.1 / vox;
+            }
+        }
     const double bd[3] = {bev[0] * P.lat, bev[1] * P.lng, bev[2] * P.lat};
     for (int r = 0; r < P.nrays; r++) {
         const float* M = c->rays[r].MK;
@@ -642,9 +737,45 @@ PlanBound plan_bound(const ee_context* c, const EeBeamSpec& S) {
         long long s0 = (long long)std::ceil((mx[1] - mn[1]) / P.lng) + 2;
         long long s1 = (long long)std::ceil((mx[2] - mn[2]) / P.lat) + 2;
         long long s2 = (long long)std::ceil((mx[0] - mn[0]) / P.lat) + 2;
+        B.max_line = (int)std::max<long long>(B.max_line, std::min<long long>(s0, EE_MAX_LINE));
+        // the kept part (kept_part): the lit rectangle, the same for every
+        // crop box up to its origin, and along the lines the dilated box;
+        // eight cells more for the roundings to whole cells and bricks
+        if (bounded) {
+            const double q0[3] = {0, 0, 0};
+            double lo[2] = {1e30, 1e30}, hi[2] = {-1e30, -1e30};
+            for (int axis = 0; axis < 4; axis++) {  // whichever side lines the device's rounding picks
+                double lit[4][3], l[2], h[2];
+                ee_lit_planes<double>(M, lc, lh, q0, lit, axis);
+                ee_lit_rect<double>(lit, -EE_LIT_READ, l, h);
+                for (int a = 0; a < 2; a++) {
+                    lo[a] = std::min(lo[a], l[a]);
+                    hi[a] = std::max(hi[a], h[a]);
+                }
+            }
+            s1 = std::min(s1, (long long)std::ceil(hi[0] - lo[0]) + 8);
+            s2 = std::min(s2, (long long)std::ceil(hi[1] - lo[1]) + 8);
+            const float* Mi = c->rays[r].MKi;
+            double fa = -1e30, fb = 1e30;
+            for (int k = 0; k < 3; k++) {
+                const double m = Mi[3 * k + 1], y = Mi[3 * k + 2], z = Mi[3 * k];
+                const double D = 2.1 + std::fabs(m) + std::fabs(y) + std::fabs(z);
+                if (std::fabs(m) < 1e-6) continue;
+                // lateral reach of the rectangle with its roundings
+                const double y0 = lo[0] - 4, y1 = hi[0] + 4, z0 = lo[1] - 4, z1 = hi[1] + 4;
+                const double cmin = std::min(y * y0, y * y1) + std::min(z * z0, z * z1);
+                const double cmax = std::max(y * y0, y * y1) + std::max(z * z0, z * z1);
+                const double blo = bmn[k] - D, bhi = bmn[k] + bev[k] + D;
+                const double t0 = (blo - cmax) / m, t1 = (bhi - cmin) / m;
+                fa = std::max(fa, std::min(t0, t1));
+                fb = std::min(fb, std::max(t0, t1));
+            }
+            s0 = std::max(1ll, std::min(s0, (long long)std::ceil(std::max(fb - fa, 0.0)) + 24));
+        }
+        s1 = std::max(s1, 1ll);
+        s2 = std::max(s2, 1ll);
         // bricked REV arrays and 8 x 4 lane tiles, as k_geometry sizes them
         B.rev += 64 * ((s0 + 3) / 4) * ((s1 + 3) / 4) * ((s2 + 3) / 4);
-        B.max_line = (int)std::max<long long>(B.max_line, std::min<long long>(s0, EE_MAX_LINE));
         const long long slots = std::max(((s1 + 7) / 8) * 8 * (((s2 + 3) / 4) * 4),
                                          ((s2 + 7) / 8) * 8 * (((s1 + 3) / 4) * 4));  // either lateral order
         B.max_lines = (int)std::max<long long>(B.max_lines, slots);
@@ -681,17 +812,17 @@ struct ee_plan {
     std::vector<EeBeamSpec> specs;
     std::vector<int> starts;
     std::vector<ChunkDims> dims;
-    long long tvol_total = 0, rev_max = 0, nfl = 0;
+    long long tvol_total = 0, max_tvol = 1, rev_max = 0, nfl = 0;
     DevBuf<EeBeamSpec> d_specs;
     DevBuf<EeBeamGeom> d_geoms;
-    DevBuf<float> terma, unit, terma_grad, rev, rev_grad;
+    DevBuf<float> terma, unit, terma_grad, rev;
     DevBuf<int> bl_idx;
-    DevBuf<float2> samples;
+    ConeBufs cone;
+    EeConeWork work;
     const float* d_fluence = nullptr;
     float* d_dose = nullptr;
     const float* d_grad = nullptr;
     float* d_fgrad = nullptr;
-    int lane_block = 128;
     std::vector<int> status;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -700,7 +831,7 @@ struct ee_plan {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         d_specs.release(); d_geoms.release(); terma.release(); unit.release(); terma_grad.release();
-        rev.release(); rev_grad.release(); bl_idx.release(); samples.release();
+        rev.release(); bl_idx.release(); cone.release();
     }
 };
 
@@ -717,19 +848,20 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
         if ((e = (x)) != cudaSuccess) return e; \
     } while (0)
     PL(cudaMemsetAsync(pl->d_dose, 0, sizeof(float) * nfull, s));
+    PL(ee_launch_geom_init(pl->d_specs.p, pl->d_geoms.p, pl->nbeams, s));
+    for (int b0 = 0; b0 < pl->nbeams; b0 += kTermaBeams)
+        PL(ee_launch_terma(P, pl->d_specs.p + b0, pl->d_geoms.p + b0, pl->d_fluence, pl->terma.p,
+                           pl->adjoint ? pl->unit.p : nullptr, pl->adjoint ? pl->bl_idx.p : nullptr,
+                           std::min(kTermaBeams, pl->nbeams - b0), pl->max_tvol, s));
+    PL(ee_launch_geometry(P, pl->d_specs.p, pl->d_geoms.p, pl->nbeams, s));
     const int nchunks = (int)pl->starts.size() - 1;
     for (int k = 0; k < nchunks; k++) {
         const int b0 = pl->starts[k], nb = pl->starts[k + 1] - b0;
         const EeBeamSpec* dsp = pl->d_specs.p + b0;
-        EeBeamGeom* dge = pl->d_geoms.p + b0;
+        const EeBeamGeom* dge = pl->d_geoms.p + b0;
         const ChunkDims& D = pl->dims[k];
-        PL(ee_launch_geom_init(dsp, dge, nb, s));
-        PL(ee_launch_terma(P, dsp, dge, pl->d_fluence, pl->terma.p, pl->adjoint ? pl->unit.p : nullptr,
-                           pl->adjoint ? pl->bl_idx.p : nullptr, nb, D.max_tvol, s));
-        PL(ee_launch_geometry(P, dsp, dge, nb, s));
         if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
-        PL(ee_launch_cone(P, dsp, dge, pl->terma.p, pl->rev.p, P.mode == EE_KERNEL_EXP ? pl->samples.p : nullptr, nb,
-                          D.max_lines, D.max_line, s, pl->lane_block));
+        PL(ee_launch_cone(P, dsp, dge, pl->terma.p, pl->rev.p, pl->work, nb, D.max_lines, D.max_line, s));
         PL(ee_launch_gather(P, dsp, dge, pl->rev.p, pl->d_dose, nb, 1, D.max_rows, s));
     }
     if (!pl->adjoint) return cudaSuccess;
@@ -740,11 +872,10 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
         const EeBeamSpec* dsp = pl->d_specs.p + b0;
         const EeBeamGeom* dge = pl->d_geoms.p + b0;
         const ChunkDims& D = pl->dims[k];
-        if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev_grad.p, 0xFF, sizeof(float) * D.rev_total, s));
-        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev_grad.p, nb, D.max_lines, s));
-        PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev_grad.p, nb, D.max_tiles, s));
-        PL(ee_launch_cone_T(P, dsp, dge, pl->rev_grad.p, P.mode == EE_KERNEL_EXP ? pl->samples.p : nullptr,
-                            pl->terma_grad.p, nb, D.max_lines, D.max_line, s, pl->lane_block));
+        if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
+        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev.p, nb, D.max_lines, s));
+        PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev.p, nb, D.max_tiles, s));
+        PL(ee_launch_cone_T(P, dsp, dge, pl->rev.p, pl->work, pl->terma_grad.p, nb, D.max_lines, D.max_line, s));
         PL(ee_launch_terma_T(P, dsp, dge, pl->unit.p, pl->bl_idx.p, pl->terma_grad.p, pl->d_fgrad, nb, D.max_tvol, s));
     }
 #undef PL
@@ -775,6 +906,12 @@ int ee_create(int device, ee_context** out) {
         delete c;
         return fail(EE_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     }
+    e = ee_kernel_setup();
+    if (e != cudaSuccess) {
+        cudaStreamDestroy(c->stream);
+        delete c;
+        return fail(EE_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(e));
+    }
     c->P.mode = EE_KERNEL_TABLE;
     c->P.ss = 1;
     *out = c;
@@ -789,7 +926,7 @@ int ee_destroy(ee_context* c) {
     if (c->dens_array) cudaFreeArray(c->dens_array);
     c->density.release(); c->cumkern.release(); c->expp.release(); c->d_rays.release();
     c->d_specs.release(); c->d_geoms.release(); c->terma.release(); c->unit.release(); c->rev.release();
-    c->rev_grad.release(); c->terma_grad.release(); c->bl_idx.release(); c->samples.release();
+    c->terma_grad.release(); c->bl_idx.release(); c->cone.release();
     c->io_fluence.release(); c->io_dose.release(); c->io_grad.release();
     c->xf.release(); c->xg.release(); c->spread_w.release(); c->acc.release();
     c->h_specs.release(); c->h_geoms.release();
@@ -1134,16 +1271,14 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
     pl->d_fluence = d_fluence; pl->d_dose = d_dose; pl->d_grad = d_dose_grad; pl->d_fgrad = d_fluence_grad;
     build_specs(c->P, beams, nbeams, pl->specs.data());
     const bool expm = c->P.mode == EE_KERNEL_EXP;
-    const long long per_float = 4ll * (1 + (expm ? 2 : 0) + (pl->adjoint ? 1 : 0));
-    long long acc = 0;
     for (int b = 0; b < nbeams; b++) {
         EeBeamSpec& S = pl->specs[b];
         PlanBound B = plan_bound(c, S);
-        long long need = B.rev * per_float;
-        if (pl->starts.empty() || (acc + need > c->max_batch_bytes && acc > 0)) {
+        // the REV arena in three quarters of the budget, as pipeline()
+        if (pl->starts.empty() || b - pl->starts.back() >= kTermaBeams ||
+            4 * (pl->dims.back().rev_total + B.rev) > c->max_batch_bytes / 4 * 3) {
             pl->starts.push_back(b);
             pl->dims.push_back(ChunkDims());
-            acc = 0;
         }
         ChunkDims& D = pl->dims.back();
         S.plan_off = D.rev_total;
@@ -1156,21 +1291,26 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
         D.max_rows = std::max(D.max_rows, B.rows);
         D.max_tiles = std::max(D.max_tiles, B.tiles);
         pl->tvol_total += tvol_of(S);
+        pl->max_tvol = std::max(pl->max_tvol, tvol_of(S));
         pl->rev_max = std::max(pl->rev_max, D.rev_total);
-        acc += need;
     }
     pl->starts.push_back(nbeams);
     pl->nfl = total_fluence(beams, nbeams);
     EE_CUDA(pl->d_specs.ensure(nbeams));
     EE_CUDA(pl->d_geoms.ensure(nbeams));
     EE_CUDA(pl->terma.ensure(pl->tvol_total));
-    EE_CUDA(pl->rev.ensure(pl->rev_max));
-    if (expm) EE_CUDA(pl->samples.ensure(pl->rev_max));
+    EE_CUDA(pl->rev.ensure(pl->rev_max + 4));  // +4: vector-reduction padding
+    if (expm) {
+        int max_line = 1;
+        long long segs = 1, ntiles = 1;
+        cone_sizes(c->P.nrays, pl->starts, pl->dims, max_line, segs, ntiles);
+        EE_CUDA(pl->cone.ensure(max_line, segs, ntiles, c->max_batch_bytes));
+        pl->work = pl->cone.work(max_line, c->max_batch_bytes);
+    }
     if (pl->adjoint) {
         EE_CUDA(pl->unit.ensure(pl->tvol_total));
         EE_CUDA(pl->bl_idx.ensure(pl->tvol_total));
         EE_CUDA(pl->terma_grad.ensure(pl->tvol_total + 4));
-        EE_CUDA(pl->rev_grad.ensure(pl->rev_max + 4));
     }
     EE_CUDA(cudaMemcpyAsync(pl->d_specs.p, pl->specs.data(), sizeof(EeBeamSpec) * nbeams, cudaMemcpyHostToDevice, s));
     pl->status.resize(nbeams);
@@ -1180,25 +1320,6 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
     EE_CUDA(cudaStreamSynchronize(s));
     for (int b = 0; b < nbeams; b++)
         if (pl->status[b] != 0) return fail(pl->status[b], "beam %d: %s", b, status_text(pl->status[b]));
-    // autotune the lane kernels' block size on this batch
-    if (expm) {
-        cudaEvent_t e0 = take_event(c), e1 = take_event(c);
-        float best = 1e30f;
-        int best_lb = 128;
-        for (int lb : {64, 128, 256}) {
-            pl->lane_block = lb;
-            cudaEventRecord(e0, s);
-            EE_CUDA(plan_enqueue(pl.get(), s));
-            cudaEventRecord(e1, s);
-            EE_CUDA(cudaEventSynchronize(e1));
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms < best) { best = ms; best_lb = lb; }
-        }
-        pl->lane_block = best_lb;
-        c->event_pool.push_back(e0);
-        c->event_pool.push_back(e1);
-    }
     EE_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed));
     cudaError_t ce = plan_enqueue(pl.get(), s);
     cudaGraph_t g = nullptr;
@@ -1233,11 +1354,11 @@ int ee_plan_status(ee_plan* pl, int* nfailed) {
 
 int ee_plan_info(ee_plan* pl, int* lane_block, long long* device_bytes, int* nchunks) {
     if (!pl) return fail(EE_ERR_INVALID_ARG, "null plan");
-    if (lane_block) *lane_block = pl->lane_block;
+    if (lane_block) *lane_block = EE_CONE_BLOCK_WARPS * 32;
     if (nchunks) *nchunks = (int)pl->starts.size() - 1;
     if (device_bytes) {
-        long long b = 4ll * (pl->tvol_total + pl->rev_max) + 8ll * pl->samples.n;
-        if (pl->adjoint) b += 4ll * (3 * pl->tvol_total + pl->rev_max);
+        long long b = 4ll * (pl->tvol_total + pl->rev_max) + pl->cone.bytes();
+        if (pl->adjoint) b += 4ll * 3 * pl->tvol_total;
         *device_bytes = b;
     }
     return EE_OK;
@@ -1253,22 +1374,8 @@ int ee_plan_destroy(ee_plan* pl) {
 
 int ee_get_beam_info(ee_context* c, int i, ee_beam_info* info) {
     if (!c || !info) return fail(EE_ERR_INVALID_ARG, "null argument");
-    if (i < 0 || i >= (int)c->last_geoms.size()) return fail(EE_ERR_INVALID_ARG, "beam index %d out of range", i);
-    const EeBeamGeom& G = c->last_geoms[i];
-    const EeBeamSpec& S = c->last_specs[i];
-    std::memset(info, 0, sizeof(*info));
-    for (int a = 0; a < 3; a++) {
-        info->source[a] = S.src[a];
-        info->direction[a] = S.dir[a];
-        info->b_min[a] = G.bmin[a];
-        info->bev_size[a] = G.bev[a];
-        info->lim_min[a] = G.lim_min[a];
-    }
-    info->v_beam = G.v_beam;
-    info->rev_samples = G.rev_total;
-    info->terma_nonzero = G.nnz;
-    info->max_line = G.max_line;
-    info->status = G.status;
+    if (i < 0 || i >= (int)c->last_info.size()) return fail(EE_ERR_INVALID_ARG, "beam index %d out of range", i);
+    *info = c->last_info[i];
     return EE_OK;
 }
 
@@ -1415,10 +1522,10 @@ int ee_internal_pipeline_grouped(ee_context* c, const ee_beam* beams, int nbeams
 long long ee_internal_context_bytes(ee_context* c) {
     std::lock_guard<std::mutex> lk(c->mu);
     long long b = 0;
-    b += 4ll * (c->density.n + c->cumkern.n + c->expp.n + c->terma.n + c->unit.n + c->rev.n + c->rev_grad.n +
+    b += 4ll * (c->density.n + c->cumkern.n + c->expp.n + c->terma.n + c->unit.n + c->rev.n +
                 c->terma_grad.n + c->io_fluence.n + c->io_dose.n + c->io_grad.n + c->xf.n + c->xg.n + c->spread_w.n +
                 c->bl_idx.n);
-    b += 8ll * (c->samples.n + c->acc.n);
+    b += 8ll * c->acc.n + c->cone.bytes();
     b += (long long)sizeof(EeBeamSpec) * c->d_specs.n + (long long)sizeof(EeBeamGeom) * c->d_geoms.n;
     if (c->dens_array) b += 4ll * c->density.n;
     return b;

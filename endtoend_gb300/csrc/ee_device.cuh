@@ -138,6 +138,13 @@ __device__ __forceinline__ Brick rev_brick(int n0, int n1, int n2) {  // n0 = re
     B.sz = B.sy * ((n1 + 3) >> 2);
     return B;
 }
+// A cone's REV array as it is kept (EeRayGeom::so, sn): the whole array's
+// sizes for the border tests, the kept part's brick strides.
+__device__ __forceinline__ Brick rev_store(const EeRayGeom& R) {
+    Brick B = rev_brick(R.sn[0], R.sn[1], R.sn[2]);
+    B.n0 = R.rev[0]; B.n1 = R.rev[1]; B.n2 = R.rev[2];
+    return B;
+}
 // Offset of line (tY, tZ) in a bricked REV array: its sample i sits at
 // rev_line(B, tY, tZ) + bk_x(i).
 __device__ __forceinline__ int rev_line(const Brick& B, int tY, int tZ) { return bk_y(B, tY) + bk_z(B, tZ); }

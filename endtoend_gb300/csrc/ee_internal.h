@@ -1,6 +1,7 @@
 // Internal structures shared by the CCCS host code (ee_api.cpp) and the
 // sm_103a kernels (ee_kernels.cu).  POD only, identical on host and device.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -87,6 +88,9 @@ struct EeBeamSpec {
     double dird[3];
     double MBd[9];
     double isodistd;
+    // axial distances from the source between which the calc bbox lies (its
+    // corners): every voxel with TERMA is between them
+    float dnear, dfar;
     // REV arena slot planned from geometric upper bounds (ee_plan);
     // plan_cap == 0: the arena is sized after the geometry read-back
     long long plan_off;
@@ -99,8 +103,11 @@ struct EeBeamSpec {
 // Per-cone geometry of one beam, computed on the device.
 struct EeRayGeom {
     int rev[3];            // (along-line, lateral-1, lateral-2) sizes
-    int nlines;            // rev[1]*rev[2]
-    long long offset;      // element offset in the beam's REV arena
+    // the part of the REV array that is kept: samples so[0] .. so[0]+sn[0]-1
+    // of lines so[1].. x so[2]..; so is whole bricks
+    int so[3], sn[3];
+    int nlines;            // sn[1]*sn[2]
+    long long offset;      // where sample (0, 0, 0) would sit in the beam's REV arena
     float q0[3];           // rev_min / spacing (reference vector order)
     float G0[3], Gx[3], Gy[3], Gz[3];  // REV (tX,tY,tZ) -> patient voxel index
     float B0[3], Bx[3], By[3], Bz[3];  // REV (tX,tY,tZ) -> BEV crop-box index
@@ -117,14 +124,86 @@ struct EeRayGeom {
     float lit[4][3];
 };
 
+// Lit half-planes of one cone (EeRayGeom::lit).  In the box the field is a
+// frustum; c[e] is its axis at the near (0) and far (1) plane in BEV index
+// coordinates, h[e] its half widths there along BEV x and z, q0 the REV
+// origin.  Its eight corners projected along the cone bound every lit line:
+// k = 0, 1 cut the projection off at its ends, k = 2, 3 follow its silhouette
+// from the near to the far plane, or the axis, where that turns away from it
+// (axis: bits 0, 1 take the axis for k = 2, 3 in any case).
+template <class T>
+inline __host__ __device__ void ee_lit_planes(const float* MK, const T c[2][3], const T h[2][2], const T q0[3],
+                                              T lit[4][3], int axis = 0) {
+    T v[8][2], mid[2][2];  // (tY, tZ)
+    for (int e = 0; e < 2; e++)
+        for (int a = 0; a < 2; a++) {
+            const float* M = MK + (a ? 0 : 6);  // REV vector (tZ, tX, tY)
+            const T m = M[0] * c[e][0] + M[1] * c[e][1] + M[2] * c[e][2] - q0[a ? 0 : 2];
+            mid[e][a] = m;
+            for (int i = 0; i < 4; i++)
+                v[4 * e + i][a] = m + (i & 1 ? h[e][0] : -h[e][0]) * M[0] + (i & 2 ? h[e][1] : -h[e][1]) * M[2];
+        }
+    T ey = mid[1][0] - mid[0][0], ez = mid[1][1] - mid[0][1];
+    const T l = sqrt(ey * ey + ez * ez);
+    if (l > T(1e-2)) { ey /= l; ez /= l; }
+    else { ey = 1; ez = 0; }
+    for (int k = 0; k < 4; k++) {
+        const T sg = k & 1 ? 1 : -1;
+        T ny = sg * ey, nz = sg * ez;
+        if (k >= 2) {
+            ny = -sg * ez;
+            nz = sg * ey;
+            T best[2] = {-1e30f, -1e30f}, by[2] = {0, 0}, bz[2] = {0, 0};  // near and far corner farthest along n
+            for (int i = 0; i < 8; i++) {
+                const T t = ny * v[i][0] + nz * v[i][1];
+                if (t > best[i >> 2]) { best[i >> 2] = t; by[i >> 2] = v[i][0]; bz[i >> 2] = v[i][1]; }
+            }
+            const T dy = by[1] - by[0], dz = bz[1] - bz[0], dl = sqrt(dy * dy + dz * dz);
+            const T along = -dz * ny + dy * nz;  // (dz, dy) turned onto n
+            if (!(axis >> (k - 2) & 1) && dl > T(1e-2) && fabs(along) > T(0.5) * dl) {
+                const T t = (along > 0 ? 1 : -1) / dl;
+                ny = -t * dz;
+                nz = t * dy;
+            }
+        }
+        T sup = -1e30f;
+        for (int i = 0; i < 8; i++) {
+            const T t = ny * v[i][0] + nz * v[i][1];
+            sup = t > sup ? t : sup;
+        }
+        lit[k][0] = -ny;
+        lit[k][1] = -nz;
+        lit[k][2] = sup + T(0.05);
+    }
+}
+
+// The lateral rectangle [lo, hi] around the points whose lit forms are all >=
+// -slack (the corners of an end's and a side's lines, which meet at 30 degrees
+// or more).
+template <class T>
+inline __host__ __device__ void ee_lit_rect(const T lit[4][3], T slack, T lo[2], T hi[2]) {
+    lo[0] = lo[1] = 1e30f;
+    hi[0] = hi[1] = -1e30f;
+    for (int i = 0; i < 2; i++)
+        for (int j = 2; j < 4; j++) {
+            const T det = lit[i][0] * lit[j][1] - lit[j][0] * lit[i][1], ci = lit[i][2] + slack, cj = lit[j][2] + slack;
+            const T p[2] = {(lit[i][1] * cj - lit[j][1] * ci) / det, (lit[j][0] * ci - lit[i][0] * cj) / det};
+            for (int a = 0; a < 2; a++) {
+                lo[a] = p[a] < lo[a] ? p[a] : lo[a];
+                hi[a] = p[a] > hi[a] ? p[a] : hi[a];
+            }
+        }
+}
+
 // A lit line's forms are >= 0.  The gathers visit a voxel and cone only where
 // one of the four lines around the voxel can be lit; such a line is within one
 // cell per axis of the voxel, the lines that k_gather then reads within one
 // more, so a line whose least form is below this is never read.
 constexpr float EE_LIT_READ = -2.95f;  // -2 sqrt(2), and rounding
 
-// Per-beam geometry computed on the device (crop box + REV frames).
-struct EeBeamGeom {
+// Per-beam geometry computed on the device: the crop box and the sizes that
+// the host reads back,
+struct EeBeamGeomHead {
     int key_min[3];        // ordered-int keys for atomic min/max
     int key_max[3];
     unsigned int nnz;
@@ -134,7 +213,8 @@ struct EeBeamGeom {
     float lim_off[3];      // (lim_min - start)/voxel
     float lim_min[3];
     long long v_beam;
-    long long rev_total;
+    long long rev_total;   // the cones' REV arrays (bricked)
+    long long store_total; // their kept parts: the beam's arena
     int max_line;
     int max_lines;
     // patient rows (y,z) whose voxels can see this beam's REV dose: the AABB
@@ -145,6 +225,9 @@ struct EeBeamGeom {
     int tiles;             // 8x8x4 patient tiles covering the AABB (adjoint gather)
     long long arena_off;   // element offset of this beam's REV arena
     long long arena_cap;   // elements available to this beam
+};
+// and the cones' REV frames, which stay on the device.
+struct EeBeamGeom : EeBeamGeomHead {
     EeRayGeom ray[EE_MAX_RAYS];
 };
 
@@ -157,12 +240,31 @@ cudaError_t ee_launch_terma(const EeParams& P, const EeBeamSpec* specs, EeBeamGe
                             cudaStream_t s);
 cudaError_t ee_launch_geometry(const EeParams& P, const EeBeamSpec* specs, EeBeamGeom* geoms, int nbeams,
                                cudaStream_t s);
-// exp mode writes only each line's valid segment: `rev` must be zeroed;
-// `samples` (REV-arena sized float2, exp mode) keeps (rho, T) per sample
-// between the two passes; nullptr selects the warp kernel
+// Work space of the exp mode's lane cones: each resident warp keeps one tile's
+// samples between its two passes (scratch[warp][quad][2][lane]), and takes
+// tiles from lists, one per beam and cone, of those that the gathers can see.
+struct EeConeWork {
+    float4* scratch = nullptr;
+    int warps = 0;         // resident warps, a multiple of EE_CONE_BLOCK_WARPS
+    int quads = 0;         // quads of samples per warp
+    int* counts = nullptr; // [0] tiles taken; [1 + segment] tiles listed, segment = beam * nrays + cone in list order
+    int* tiles = nullptr;  // [segment][tiles_cap] tiles of 8 x 4 lines
+};
+constexpr int EE_CONE_BLOCK_WARPS = 2, EE_CONE_SM_WARPS = 24, EE_CONE_MAX_WARPS = 152 * EE_CONE_SM_WARPS;
+inline int ee_cone_quads(int max_line) { return (max_line + 3) / 4 + 2; }
+// resident warps whose scratch stays within a quarter of `limit` bytes
+inline int ee_cone_warps(int max_line, long long limit) {
+    const long long per = 1024ll * ee_cone_quads(max_line), n = limit / 4 / per;
+    return (int)(n < 152 ? 152 : (n > EE_CONE_MAX_WARPS ? EE_CONE_MAX_WARPS : n)) & ~(EE_CONE_BLOCK_WARPS - 1);
+}
+inline int ee_cone_tiles_cap(int max_lines) { return max_lines / 32 + 1; }
+// kernel attributes of the current device; before the first launch on it
+cudaError_t ee_kernel_setup();
+// the cones write every sample that k_gather reads; without work space (exp
+// mode) the warp-per-line kernel runs
 cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* terma,
-                           float* rev, float2* samples, int nbeams, int max_lines, int max_line, cudaStream_t s,
-                           int lane_block = 128);
+                           float* rev, const EeConeWork& work, int nbeams, int max_lines, int max_line,
+                           cudaStream_t s);
 // dose_mode 0/1 accumulate atomically into dose (the caller zeroes it for
 // mode 0); mode 2 writes dose[b] rows (the caller zeroes the volumes).
 cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev,
@@ -170,12 +272,9 @@ cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const E
 // adjoint
 cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
                                const float* dose_grad, float* rev_grad, int nbeams, int max_tiles, cudaStream_t s);
-// scratch: REV-arena sized float2 (exp mode's lane kernel keeps one pass's
-// contributions and the samples' density there); nullptr selects the warp
-// kernel
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
-                             float2* scratch, float* terma_grad, int nbeams, int max_lines, int max_line,
-                             cudaStream_t s, int lane_block = 128);
+                             const EeConeWork& work, float* terma_grad, int nbeams, int max_lines, int max_line,
+                             cudaStream_t s);
 // zeros on every line's segment of a chunk's REV gradient arena (before
 // ee_launch_gather_T; the forward cone kernels zero their own arena)
 cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,

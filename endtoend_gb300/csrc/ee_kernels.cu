@@ -295,33 +295,28 @@ __device__ __forceinline__ void field_forms(const EeParams& P, const EeBeamSpec&
     }
 }
 
-// The lines of a cone that the field can reach, as half-planes of the lateral
-// REV plane.  A crop box holds the BEV origin whatever the field (host.cu:442:
-// the maximum starts at FLT_MIN), so most of it can lie off the field: of the
-// 1024-beam candidates' lines 46 % have no field span.  In the box the field
-// (raised as in field_forms) is a frustum between the planes BEV y = 0 and
-// bev[1]; its eight corners projected along the cone bound every lit line.
-// Two half-planes follow the frustum's silhouette from near to far, two cut
-// it off at its ends.  No bound where the frustum form does not hold: voxels
-// that are not cubes (the BEV planes are then not normal to the beam) and a
-// box that does not stay in front of the source.
-__device__ void lit_planes(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G, EeRayGeom& R) {
+// The lines of a cone that the field can reach (ee_lit_planes).  A crop box
+// holds the BEV origin whatever the field (host.cu:442: the maximum starts at
+// FLT_MIN), so most of it can lie off the field: of the 1024-beam candidates'
+// lines 46 % have no field span.  The field is raised as in field_forms and
+// taken between the planes through the calc bbox's nearest and farthest
+// corners, so the half-planes depend on the beam alone.  No bound where the
+// frustum form does not hold: voxels that are not cubes (the BEV planes are
+// then not normal to the beam) and a bbox that reaches the source.
+__device__ bool lit_planes(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G, EeRayGeom& R) {
     for (int k = 0; k < 4; k++) {
         R.lit[k][0] = R.lit[k][1] = 0.f;
         R.lit[k][2] = 1.f;
     }
     const float vox = P.voxel[0];
-    if (P.voxel[1] != vox || P.voxel[2] != vox) return;
+    if (P.voxel[1] != vox || P.voxel[2] != vox || !(S.dnear > 0.02f * S.isodist)) return false;
     const f3 src = ld3(S.src), dir = ld3(S.dir), start = ld3(P.start), off = ld3(G.lim_off);
     const float reach = P.ss > 1 ? 1.55f : 1.05f;
-    f3 v[8];  // REV coordinates (tZ, tX, tY) of the corners, near ones first
-    f3 mid[2];
+    float c[2][3], h[2][2];
     for (int e = 0; e < 2; e++) {
-        const f3 o = off + mv(S.MBi, mk(0.f, e ? (float)G.bev[1] : 0.f, 0.f));
-        const float D = dot(dir, start + o * vox - src);
-        if (!(D > 0.02f * S.isodist)) return;
-        const f3 c = mv(S.MB, (src + dir * D - start) * (1.f / vox) - off);
-        float h[2];
+        const float D = e ? S.dfar + 4.f * vox : S.dnear - 4.f * vox;
+        const f3 p = mv(S.MB, (src + dir * D - start) * (1.f / vox) - off);
+        c[e][0] = p.x; c[e][1] = p.y; c[e][2] = p.z;
         for (int a = 0; a < 2; a++) {
             const f3 m = ld3(S.MB + (a ? 6 : 0));
             const f3 g = m - dir * dot(m, dir);
@@ -331,39 +326,48 @@ __device__ void lit_planes(const EeParams& P, const EeBeamSpec& S, const EeBeamG
                 const f3 gl = g * (sg ? 1.f : -1.f) + dir * k;
                 M = fmaxf(M, reach * (fabsf(gl.x) + fabsf(gl.y) + fabsf(gl.z)) * vox + 1e-3f);
             }
-            h[a] = (k * D + M) / vox;
+            h[e][a] = (k * D + M) / vox;
         }
-        const f3 q0 = ld3(R.q0);
-        mid[e] = mv(R.M, c) - q0;
-        for (int i = 0; i < 4; i++) v[4 * e + i] = mv(R.M, c + mk(i & 1 ? h[0] : -h[0], 0.f, i & 2 ? h[1] : -h[1])) - q0;
     }
-    // e: the projected beam axis, n: its normal, as (tY, tZ)
-    float ey = mid[1].z - mid[0].z, ez = mid[1].x - mid[0].x;
-    const float l = sqrtf(ey * ey + ez * ez);
-    if (l > 1e-2f) { ey /= l; ez /= l; }
-    else { ey = 1.f; ez = 0.f; }
-    for (int k = 0; k < 4; k++) {
-        const float sg = k & 1 ? 1.f : -1.f;
-        float ny = sg * ey, nz = sg * ez;  // k < 2: the ends
-        if (k >= 2) {
-            ny = -sg * ez;
-            nz = sg * ey;
-            int b[2] = {0, 4};  // the near and the far corner farthest along n
-            for (int i = 0; i < 8; i++)
-                if (ny * v[i].z + nz * v[i].x > ny * v[b[i >> 2]].z + nz * v[b[i >> 2]].x) b[i >> 2] = i;
-            const float dy = v[b[1]].z - v[b[0]].z, dz = v[b[1]].x - v[b[0]].x, dl = sqrtf(dy * dy + dz * dz);
-            if (dl > 1e-2f) {
-                const float t = -dz * ny + dy * nz > 0.f ? 1.f : -1.f;
-                ny = -t * dz / dl;
-                nz = t * dy / dl;
-            }
+    ee_lit_planes<float>(R.M, c, h, R.q0, R.lit);
+    return true;
+}
+
+// The part of a cone's REV array that the gathers reach: the lines whose lit
+// forms are at least EE_LIT_READ, and along them the crop box dilated as in
+// line_read_span.  The cells outside it are neither written nor read (of the
+// arrays' 84..142 cells per crop-box voxel a little over half remain), so more
+// beams share a chunk.
+__device__ void kept_part(const EeBeamGeom& G, EeRayGeom& R, bool bounded) {
+    float lo[2] = {0.f, 0.f}, hi[2] = {(float)(R.rev[1] - 1), (float)(R.rev[2] - 1)};
+    if (bounded) {
+        float a[2], b[2];
+        ee_lit_rect<float>(R.lit, -EE_LIT_READ, a, b);
+        for (int i = 0; i < 2; i++) {
+            lo[i] = fmaxf(lo[i], floorf(a[i] - 0.1f));
+            hi[i] = fminf(hi[i], ceilf(b[i] + 0.1f));
         }
-        float sup = -1e30f;
-        for (int i = 0; i < 8; i++) sup = fmaxf(sup, ny * v[i].z + nz * v[i].x);
-        R.lit[k][0] = -ny;
-        R.lit[k][1] = -nz;
-        R.lit[k][2] = sup + 0.05f;
     }
+    float fa = 0.f, fb = (float)(R.rev[0] - 1);
+    for (int k = 0; k < 3; k++) {
+        const float D = 2.05f + fabsf(R.Bx[k]) + fabsf(R.By[k]) + fabsf(R.Bz[k]), m = R.Bx[k];
+        if (fabsf(m) < 1e-6f) continue;
+        const float y = R.By[k], z = R.Bz[k];
+        const float cmin = R.B0[k] + fminf(y * lo[0], y * hi[0]) + fminf(z * lo[1], z * hi[1]);
+        const float cmax = R.B0[k] + fmaxf(y * lo[0], y * hi[0]) + fmaxf(z * lo[1], z * hi[1]);
+        const float t0 = (-D - cmax) / m, t1 = ((float)G.bev[k] + D - cmin) / m;
+        fa = fmaxf(fa, fminf(t0, t1));
+        fb = fminf(fb, fmaxf(t0, t1));
+    }
+    const bool none = hi[0] < lo[0] || hi[1] < lo[1] || fb < fa - 4.f;
+    const int i0 = max(0, (int)floorf(fa) - 4), i1 = min(R.rev[0] - 1, (int)ceilf(fb) + 4);
+    R.so[0] = none ? 0 : i0 & ~3;
+    R.sn[0] = none ? 0 : i1 - R.so[0] + 1;
+    for (int i = 0; i < 2; i++) {
+        R.so[1 + i] = none ? 0 : (int)lo[i] & ~3;
+        R.sn[1 + i] = none ? 0 : (int)hi[i] - R.so[1 + i] + 1;
+    }
+    R.nlines = R.sn[1] * R.sn[2];
 }
 
 // The least of a cone's lit forms at lateral REV point (tY, tZ).
@@ -447,7 +451,6 @@ __global__ void k_geometry(EeParams P, const EeBeamSpec* __restrict__ specs, EeB
         }
         if (sz[0] > EE_MAX_LINE || sz[0] <= 0 || sz[1] <= 0 || sz[2] <= 0) bad = true;
         if (bad) atomicExch(&G.status, 4);
-        R.nlines = sz[1] * sz[2];
         f3 q0 = mk(mn[0] / P.lat, mn[1] / P.lng, mn[2] / P.lat);
         R.q0[0] = q0.x; R.q0[1] = q0.y; R.q0[2] = q0.z;
         // REV vector (tZ, tX, tY) + q0 -> BEV (inverseRotateKernel)
@@ -474,7 +477,7 @@ __global__ void k_geometry(EeParams P, const EeBeamSpec* __restrict__ specs, EeB
             R.iG[a] = fabsf(R.Gx[a]) < 1e-6f ? 0.f : 1.f / R.Gx[a];
         }
         field_forms(P, S, R);
-        lit_planes(P, S, G, R);
+        kept_part(G, R, lit_planes(P, S, G, R));
     }
     __syncthreads();
     if (threadIdx.x == 0 && G.status == 0) {
@@ -494,19 +497,23 @@ __global__ void k_geometry(EeParams P, const EeBeamSpec* __restrict__ specs, EeB
         G.gnx = max(0, x1 - x0 + 1); G.gny = max(0, y1 - y0 + 1); G.gnz = max(0, z1 - z0 + 1);
         G.rows = (int)ee_gather_groups(G.gny, G.gnz);
         G.tiles = ((G.gnx + 7) / 8) * ((G.gny + 7) / 8) * ((G.gnz + 3) / 4);
-        long long off = 0;
+        long long off = 0, all = 0;
         int ml = 0, mls = 0;
         for (int r = 0; r < P.nrays; r++) {
             // bricked REV arrays (rev_brick); the lane kernels run one lane
             // slot per line of an 8 (tY) x 4 (tZ) tile
-            G.ray[r].offset = off;
-            off += ee_brick_vol(G.ray[r].rev);
-            ml = max(ml, G.ray[r].rev[0]);
-            mls = max(mls, ((G.ray[r].rev[1] + 7) >> 3) * 8 * (((G.ray[r].rev[2] + 3) >> 2) * 4));
+            EeRayGeom& R = G.ray[r];
+            const Brick B = rev_store(R);
+            R.offset = off - (bk_x(R.so[0]) + bk_y(B, R.so[1]) + bk_z(B, R.so[2]));
+            off += ee_brick_vol(R.sn);
+            all += ee_brick_vol(R.rev);
+            ml = max(ml, R.rev[0]);
+            mls = max(mls, ((R.sn[1] + 7) >> 3) * 8 * (((R.sn[2] + 3) >> 2) * 4));
         }
-        G.rev_total = off;
+        G.rev_total = all;
+        G.store_total = off;
         // the gather addresses a cone's REV array with a 32-bit offset
-        if (off > 2147483647ll) G.status = 4;  // EE_ERR_REV_SIZE
+        if (all > 2147483647ll) G.status = 4;  // EE_ERR_REV_SIZE
         G.max_line = ml;
         G.max_lines = mls;
         if (G.arena_cap > 0 && off > G.arena_cap) G.status = 8;
@@ -541,8 +548,8 @@ __device__ __forceinline__ void line_segment(const EeParams& P, const EeBeamGeom
         }
     }
     if (!(a <= b + 2.f)) { n = 0; i0 = 0; return; }
-    i0 = max(0, (int)floorf(a) - 1);
-    int i1 = min(L - 1, (int)ceilf(b) + 1);
+    i0 = max(R.so[0], (int)floorf(a) - 1);
+    int i1 = min(R.so[0] + R.sn[0] - 1, (int)ceilf(b) + 1);
     n = max(0, i1 - i0 + 1);
 }
 
@@ -573,8 +580,15 @@ __device__ __forceinline__ void line_read_span(const EeBeamGeom& G, const EeRayG
         }
     }
     if (!(a <= b + 2.f)) return;
-    z0 = max(0, (int)floorf(a) - 1);
-    z1 = min(L - 1, (int)ceilf(b) + 1);
+    z0 = max(R.so[0], (int)floorf(a) - 1);
+    z1 = min(R.so[0] + R.sn[0] - 1, (int)ceilf(b) + 1);
+}
+
+// Line `line` of a cone's kept part (R.nlines).
+__device__ __forceinline__ void kept_line(const EeRayGeom& R, int line, int& tY, int& tZ) {
+    tZ = line / R.sn[1];
+    tY = R.so[1] + line - tZ * R.sn[1];
+    tZ += R.so[2];
 }
 
 // Zero the samples of a line's read span outside [i0, i0 + n) (the cone
@@ -811,12 +825,14 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone(EeParams P, const EeBe
     const int line = blockIdx.x * CONE_WARPS + warp;
     if (line >= R.nlines) return;
     const int L = R.rev[0];
-    const int tY = line % R.rev[1], tZ = line / R.rev[1];
+    int tY, tZ;
+    kept_line(R, line, tY, tZ);
+    if (lit_form(R, (float)tY, (float)tZ) < EE_LIT_READ) return;
     float* rho = sm + (size_t)warp * 3 * maxL;
     float* T = rho + maxL;
     float* D = T + maxL;
     // bricked REV arena (rev_brick): sample i at out + bk_x(i)
-    const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
+    const Brick Bv = rev_store(R);
     float* out = rev + G.arena_off + R.offset + rev_line(Bv, tY, tZ);
     int i0, n, z0, z1;
     line_segment(P, G, R, tY, tZ, L, i0, n);
@@ -1241,8 +1257,9 @@ __device__ __forceinline__ void tab_fwd_line(const EeParams& P, const EeBeamSpec
     int nn = 0;
     if (line >= 0) {
         const int L = R.rev[0];
-        const int tY = line % R.rev[1], tZ = line / R.rev[1];
-        const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
+        int tY, tZ;
+        kept_line(R, line, tY, tZ);
+        const Brick Bv = rev_store(R);
         out = rev_beam + R.offset + rev_line(Bv, tY, tZ);
         int z0, z1;
         line_read_span(G, R, tY, tZ, L, z0, z1);
@@ -1263,6 +1280,18 @@ __device__ __forceinline__ void tab_fwd_line(const EeParams& P, const EeBeamSpec
     tab_receivers<false, W>(Mv, Pv, SVv, SVMv, rho, nn, lane, tab_row(tab, false), X, D, nphi);
     __syncwarp();
     for (int k = lane; k < nn; k += W) out[bk_x(i0 + k)] = D[k];
+}
+
+// The segment of kept line `line`; line = -1 (n = 0) where its lit forms are
+// below `least`.
+__device__ __forceinline__ void tab_line(const EeParams& P, const EeBeamGeom& G, const EeRayGeom& R, float least,
+                                         int& line, int& i0, int& n) {
+    i0 = n = 0;
+    if (line < 0) return;
+    int tY, tZ;
+    kept_line(R, line, tY, tZ);
+    if (lit_form(R, (float)tY, (float)tZ) < least) line = -1;
+    else line_segment(P, G, R, tY, tZ, R.rev[0], i0, n);
 }
 
 // A warp takes two neighbouring lines.  When both fit half of its arrays
@@ -1287,13 +1316,13 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_tab(EeParams P, const E
     const EeBeamGeom& G = geoms[b];
     if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
-    const int la = 2 * (blockIdx.x * TAB_WARPS + warp);
+    int la = 2 * (blockIdx.x * TAB_WARPS + warp);
     if (la >= R.nlines) return;
-    const int lb = la + 1 < R.nlines ? la + 1 : -1;
-    const int L = R.rev[0];
+    int lb = la + 1 < R.nlines ? la + 1 : -1;
     int i0a, na, i0b = 0, nb = 0;
-    line_segment(P, G, R, la % R.rev[1], la / R.rev[1], L, i0a, na);
-    if (lb >= 0) line_segment(P, G, R, lb % R.rev[1], lb / R.rev[1], L, i0b, nb);
+    tab_line(P, G, R, EE_LIT_READ, la, i0a, na);
+    tab_line(P, G, R, EE_LIT_READ, lb, i0b, nb);
+    if (la < 0 && lb < 0) return;
     float* arr = sm + (size_t)warp * tab_fwd_stride(maxL);
     int* X = reinterpret_cast<int*>(arr + 7 * Lp) + lane;
     const EeBeamSpec& S = specs[b];
@@ -1307,7 +1336,7 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_tab(EeParams P, const E
         tab_fwd_line<16>(P, S, G, R, terma_b, rev_beam, sub ? lb : la, sub ? i0b : i0a, sub ? nb : na, lane & 15,
                          arr + sub * (half + 1), Lp, tab, X);
     } else {
-        tab_fwd_line<32>(P, S, G, R, terma_b, rev_beam, la, i0a, na, lane, arr, Lp, tab, X);
+        if (la >= 0) tab_fwd_line<32>(P, S, G, R, terma_b, rev_beam, la, i0a, na, lane, arr, Lp, tab, X);
         if (lb >= 0) {
             __syncwarp();
             tab_fwd_line<32>(P, S, G, R, terma_b, rev_beam, lb, i0b, nb, lane, arr, Lp, tab, X);
@@ -1332,14 +1361,13 @@ __device__ __forceinline__ void tab_adj_line(const EeParams& P, const EeBeamSpec
     float* Uk = Wk + Lp;
     int nn = 0, tY = 0, tZ = 0;
     if (line >= 0 && n > 0) {
-        tY = line % R.rev[1];
-        tZ = line / R.rev[1];
+        kept_line(R, line, tY, tZ);
         gather_line(P, S, G, R, nullptr, tY, tZ, i0, n, lane, rho, nullptr, W);
         nn = n;
     }
     __syncwarp();
     if (nn > 0) {
-        const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
+        const Brick Bv = rev_store(R);
         const float* gin = grad_beam + R.offset + rev_line(Bv, tY, tZ);
         const float inv_nphi = 1.f / (float)P.nphi;
         for (int k = lane; k < nn; k += W) {
@@ -1395,13 +1423,13 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_T_tab(EeParams P, const
     const EeBeamGeom& G = geoms[b];
     if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
-    const int la = 2 * (blockIdx.x * TAB_WARPS + warp);
+    int la = 2 * (blockIdx.x * TAB_WARPS + warp);
     if (la >= R.nlines) return;
-    const int lb = la + 1 < R.nlines ? la + 1 : -1;
-    const int L = R.rev[0];
+    int lb = la + 1 < R.nlines ? la + 1 : -1;
     int i0a, na, i0b = 0, nb = 0;
-    line_segment(P, G, R, la % R.rev[1], la / R.rev[1], L, i0a, na);
-    if (lb >= 0) line_segment(P, G, R, lb % R.rev[1], lb / R.rev[1], L, i0b, nb);
+    tab_line(P, G, R, 0.f, la, i0a, na);
+    tab_line(P, G, R, 0.f, lb, i0b, nb);
+    if (la < 0 && lb < 0) return;
     float* arr = sm + (size_t)warp * tab_adj_stride(maxL);
     int* Y = reinterpret_cast<int*>(arr + 9 * Lp) + lane;
     const EeBeamSpec& S = specs[b];
@@ -1412,7 +1440,7 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_T_tab(EeParams P, const
         tab_adj_line<16>(P, S, G, R, grad_beam, terma_grad, sub ? lb : la, sub ? i0b : i0a, sub ? nb : na,
                          lane & 15, arr + sub * (half + 1), Lp, tab, Y);
     } else {
-        tab_adj_line<32>(P, S, G, R, grad_beam, terma_grad, la, i0a, na, lane, arr, Lp, tab, Y);
+        if (la >= 0) tab_adj_line<32>(P, S, G, R, grad_beam, terma_grad, la, i0a, na, lane, arr, Lp, tab, Y);
         if (lb >= 0) {
             __syncwarp();
             tab_adj_line<32>(P, S, G, R, grad_beam, terma_grad, lb, i0b, nb, lane, arr, Lp, tab, Y);
@@ -1502,10 +1530,115 @@ __device__ __forceinline__ LaneSpan lane_span(const EeParams& P, const EeBeamSpe
 // slabs.  False for slots of a tile that lie outside the cone's array.
 __device__ __forceinline__ bool lane_line(const EeRayGeom& R, int slot, int& tY, int& tZ) {
     const int wt = slot >> 5, l = slot & 31;
-    const int nty = (R.rev[1] + 7) >> 3;
+    const int nty = (R.sn[1] + 7) >> 3;
+    if (nty == 0) return false;
     tY = (wt % nty) * 8 + (l & 7);
     tZ = (wt / nty) * 4 + (l >> 3);
-    return tY < R.rev[1] && tZ < R.rev[2];
+    const bool in = tY < R.sn[1] && tZ < R.sn[2];
+    tY += R.so[1];
+    tZ += R.so[2];
+    return in;
+}
+
+// Cone y of a beam's lists: cones with small angles to the beam axis, whose
+// lines are the longest, come first.
+__device__ __forceinline__ int list_cone(const EeParams& P, int y) {
+    return (y % P.nphi) * (P.ntheta / 2) + y / P.nphi;
+}
+
+// The tiles of 8 x 4 lines that may hold a line with lit forms of at least
+// `least` in the dilated crop box: the lane cones' work lists, a block per
+// beam and cone.
+__global__ void __launch_bounds__(256) k_cone_tiles(EeParams P, const EeBeamGeom* __restrict__ geoms, float least,
+                                                    int* __restrict__ counts, int* __restrict__ tiles, int cap) {
+    __shared__ int s_n;
+    const int b = blockIdx.y, seg = b * P.nrays + blockIdx.x;
+    const EeBeamGeom& G = geoms[b];
+    if (seg == 0 && threadIdx.x == 0) counts[0] = 0;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    if (G.status == 0) {
+        const EeRayGeom& R = G.ray[list_cone(P, blockIdx.x)];
+        const int nty = (R.sn[1] + 7) >> 3, n = nty * ((R.sn[2] + 3) >> 2);
+        for (int t0 = 0; t0 < n; t0 += 256) {
+            const int tile = t0 + threadIdx.x;
+            bool live = tile < n;
+            if (live) {
+                const float cy = (float)(R.so[1] + (tile % nty) * 8) + 3.5f, cz = (float)(R.so[2] + (tile / nty) * 4) + 1.5f;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const float a = R.lit[k][0], b2 = R.lit[k][1];
+                    if (fmaf(a, cy, fmaf(b2, cz, R.lit[k][2])) + 3.5f * fabsf(a) + 1.5f * fabsf(b2) < least) live = false;
+                }
+                float a = 0.f, e = (float)(R.rev[0] - 1);
+#pragma unroll
+                for (int k = 0; k < 3; k++) {  // line_read_span, for all lines of the tile
+                    const float c = R.B0[k] + R.By[k] * cy + R.Bz[k] * cz;
+                    const float D = 2.1f + fabsf(R.Bx[k]) + 4.5f * fabsf(R.By[k]) + 2.5f * fabsf(R.Bz[k]);
+                    const float lo = -D - c, hi = (float)G.bev[k] + D - c;
+                    if (R.iB[k] == 0.f) {
+                        if (lo > 0.f || hi < 0.f) live = false;
+                    } else {
+                        a = fmaxf(a, fminf(lo * R.iB[k], hi * R.iB[k]));
+                        e = fminf(e, fmaxf(lo * R.iB[k], hi * R.iB[k]));
+                    }
+                }
+                if (a > e + 3.f) live = false;
+            }
+            const unsigned m = __ballot_sync(FULL, live);
+            int base = 0;
+            if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(&s_n, __popc(m));
+            base = __shfl_sync(FULL, base, 0);
+            if (live) tiles[(size_t)seg * cap + base + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = tile;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) counts[1 + seg] = s_n;
+}
+
+// Runs `line` for every listed tile, a lane per line.  The warps are resident
+// (24 per SM at 80 registers; 28 and 32 measured the same and 4 % slower, 20 and
+// 16 3 % and 6 % slower): each starts on the tile of its number and takes the
+// next from the counter when it is done, not before, or the last tiles wait
+// behind long ones while other warps idle (one 24 x 24 beam 1.03 against
+// 1.15 ms).  Tiles are taken beam by beam, so that the beams in work stay in L2
+// (one list of all beams, filled in the order the blocks happened to run: 96
+// beams of 8^2..40^2 beamlets 11.1 against 10.5 ms).  So the scratch of a
+// tile's samples is a warp's and not a REV array's: 8 of the 12 to 16 bytes
+// that a REV cell took, and it stays in L2.  On the same chunks the cones run
+// as fast as one block per 128 lines did; more beams fit a chunk.
+template <class F>
+__device__ __forceinline__ void cone_tiles_run(const EeParams& P, const EeConeWork& W, int nbeams, int cap, F line) {
+    const int lane = threadIdx.x & 31, slot = blockIdx.x * EE_CONE_BLOCK_WARPS + (threadIdx.x >> 5);
+    float4* scratch = W.scratch + (size_t)slot * W.quads * 64 + lane;
+    const int nseg = nbeams * P.nrays;
+    // a window of 32 lists: items before it, this lane's list and the items up
+    // to and with it
+    int seg0 = 0, base = 0, upto = 0, mine = 0;
+    auto load = [&]() {
+        mine = seg0 + lane < nseg ? W.counts[1 + seg0 + lane] : 0;
+        upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(FULL, upto, o);
+            if (lane >= o) upto += y;
+        }
+    };
+    load();
+    for (int item = slot;;) {
+        int total;
+        while (item >= base + (total = __shfl_sync(FULL, upto, 31))) {
+            base += total;
+            seg0 += 32;
+            if (seg0 >= nseg) return;
+            load();
+        }
+        const int l = __ffs((int)__ballot_sync(FULL, item < base + upto)) - 1, seg = seg0 + l;
+        const int first = base + __shfl_sync(FULL, upto - mine, l);
+        line(seg / P.nrays, list_cone(P, seg % P.nrays), W.tiles[(size_t)seg * cap + item - first] * 32 + lane, scratch);
+        if (lane == 0) item = W.warps + atomicAdd(W.counts, 1);
+        item = __shfl_sync(FULL, item, 0);
+    }
 }
 
 // Forward cone, one lane per line.  Both passes walk whole quads of samples
@@ -1526,25 +1659,20 @@ __device__ __forceinline__ bool lane_line(const EeRayGeom& R, int slot, int& tY,
 // Samples of an end quad outside [i0, i1] get dose 0 (they are inside the
 // read span or never read); their zero TERMA and unit factors leave the
 // recurrence as it is.
-template <int LANE_BLOCK>
-__global__ void __launch_bounds__(LANE_BLOCK) k_cone_lane(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                          const EeBeamGeom* __restrict__ geoms,
-                                                          const float* __restrict__ terma, float* __restrict__ rev,
-                                                          float2* __restrict__ samples) {
-    const int ray = blockIdx.y, b = blockIdx.z;
+__device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* __restrict__ specs,
+                                          const EeBeamGeom* __restrict__ geoms, const float* __restrict__ terma,
+                                          float* __restrict__ rev, int b, int ray, int slot,
+                                          float4* __restrict__ smp) {
     const EeBeamGeom& G = geoms[b];
-    if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
     int tY, tZ;
-    if (!lane_line(R, blockIdx.x * LANE_BLOCK + threadIdx.x, tY, tZ)) return;
+    if (!lane_line(R, slot, tY, tZ)) return;
     if (lit_form(R, (float)tY, (float)tZ) < EE_LIT_READ) return;  // dark, and never read
     const EeBeamSpec& S = specs[b];
     LineFrame F;
     const LaneSpan s = lane_span(P, S, G, R, tY, tZ, F);
     // bricked REV arena (rev_brick): this line's sample i sits at out + bk_x(i)
-    const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
-    const long long base = G.arena_off + R.offset + rev_line(Bv, tY, tZ);
-    float* out = rev + base;
+    float* out = rev + G.arena_off + R.offset + rev_line(rev_store(R), tY, tZ);
     const bool lit = s.q0 <= s.q1;
     {   // zeros on the rest of the read span, or all of it on a dark line
         int z0, z1;
@@ -1559,7 +1687,6 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_lane(EeParams P, const EeBe
     const float* tb = terma + S.t_off;
     const Brick Bt = brick_of(S.tn);
     const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
-    float2* smp = samples + base;  // (rho, T), bricked like the REV arena
     const EeRayConst& RC = P.rays[ray];
     const float inv_nphi = 1.f / (float)P.nphi;
     const int qe = s.i1 >> 2, qs = s.i0 >> 2;
@@ -1593,9 +1720,9 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_lane(EeParams P, const EeBe
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) dq[j] = step(rr[j], tt[j]);
-            float4* sq = reinterpret_cast<float4*>(smp + 64 * q);
+            float4* sq = smp + 64 * (q - s.q0);  // (rho, T)
             sq[0] = make_float4(rr[0], tt[0], rr[1], tt[1]);
-            sq[1] = make_float4(rr[2], tt[2], rr[3], tt[3]);
+            sq[32] = make_float4(rr[2], tt[2], rr[3], tt[3]);
             *reinterpret_cast<float4*>(out + 64 * q) = make_float4(dq[0], dq[1], dq[2], dq[3]);
         }
         for (int q = s.q1 + 1; q <= qe; q++) {
@@ -1626,8 +1753,8 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_lane(EeParams P, const EeBe
             return v ? (below + d) * inv_nphi : 0.f;
         };
         for (int q = s.q1; q >= s.q0; q--) {
-            const float4* sq = reinterpret_cast<const float4*>(smp + 64 * q);
-            const float4 s01 = sq[0], s23 = sq[1];
+            const float4* sq = smp + 64 * (q - s.q0);
+            const float4 s01 = sq[0], s23 = sq[32];
             const float4 o4 = *reinterpret_cast<const float4*>(out + 64 * q);
             float4 dq;
             dq.w = step(s23.z, s23.w, o4.w);
@@ -1649,6 +1776,14 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_lane(EeParams P, const EeBe
             *reinterpret_cast<float4*>(out + 64 * q) = make_float4(dq[0], dq[1], dq[2], dq[3]);
         }
     }
+}
+
+__global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / EE_CONE_BLOCK_WARPS)
+    k_cone_lane(EeParams P, const EeBeamSpec* __restrict__ specs, const EeBeamGeom* __restrict__ geoms,
+                const float* __restrict__ terma, float* __restrict__ rev, EeConeWork W, int nbeams, int cap) {
+    cone_tiles_run(P, W, nbeams, cap, [&](int b, int ray, int slot, float4* scratch) {
+        cone_line(P, specs, geoms, terma, rev, b, ray, slot, scratch);
+    });
 }
 
 // Zero the samples of the chunk's REV gradient arena that the adjoint cone
@@ -1674,12 +1809,12 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
         i0 = s.i0;
         i1 = s.i1;
     } else {
+        if (lit_form(R, (float)tY, (float)tZ) < 0.f) return;
         int n;
         line_segment(P, G, R, tY, tZ, R.rev[0], i0, n);
         i1 = i0 + n - 1;
     }
-    const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
-    float* row = rev_grad + G.arena_off + R.offset + rev_line(Bv, tY, tZ);
+    float* row = rev_grad + G.arena_off + R.offset + rev_line(rev_store(R), tY, tZ);
     for (int ib = i0 & ~3; ib <= i1; ib += 4)
         *reinterpret_cast<float4*>(row + bk_x(ib)) = make_float4(0.f, 0.f, 0.f, 0.f);
 }
@@ -1689,31 +1824,25 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
 // neighbour it came from (g, h and Z of sample m's neighbour i):
 //   Tbar_m += c g_i (1 - h_m) + Z h_i (1 - h_m h_i),   Z <- h_i^2 Z + c g_i.
 // Pass A walks down (transpose of the walk up) and keeps its part of Tbar
-// with rho in `scratch` (the REV-arena layout); pass B walks up, adds its
+// with rho in the warp's scratch; pass B walks up, adds its
 // part and scatters Tbar into the TERMA-box gradient.  Only the quads [q0, q1]
 // of the field span have a TERMA gradient: pass A stops below q0, pass B
 // above q1, and outside the span each only updates Z, with the densities of
 // the texture; the scratch holds the span alone.  One 24 x 24 beam 0.428 ->
 // 0.301 ms, 20 beams of 128^2 pixels 8.1 -> 5.4 ms.
-template <int LANE_BLOCK>
-__global__ void __launch_bounds__(LANE_BLOCK) k_cone_T_lane(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                            const EeBeamGeom* __restrict__ geoms,
-                                                            const float* __restrict__ rev_grad,
-                                                            float2* __restrict__ scratch, float* __restrict__ terma_grad) {
-    const int ray = blockIdx.y, b = blockIdx.z;
+__device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec* __restrict__ specs,
+                                            const EeBeamGeom* __restrict__ geoms, const float* __restrict__ rev_grad,
+                                            float* __restrict__ terma_grad, int b, int ray, int slot,
+                                            float4* __restrict__ sA) {
     const EeBeamGeom& G = geoms[b];
-    if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
     int tY, tZ;
-    if (!lane_line(R, blockIdx.x * LANE_BLOCK + threadIdx.x, tY, tZ)) return;
+    if (!lane_line(R, slot, tY, tZ)) return;
     const EeBeamSpec& S = specs[b];
     LineFrame F;
     const LaneSpan s = lane_span(P, S, G, R, tY, tZ, F);
     if (s.q1 < s.q0) return;
-    const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
-    const long long base = G.arena_off + R.offset + rev_line(Bv, tY, tZ);
-    const float* gin = rev_grad + base;
-    float2* sA = scratch + base;  // (pass-A part of Tbar, rho), bricked like the REV arena
+    const float* gin = rev_grad + G.arena_off + R.offset + rev_line(rev_store(R), tY, tZ);
     const EeRayConst& RC = P.rays[ray];
     const float inv_nphi = 1.f / (float)P.nphi;
     // the neighbour's state; Z before the neighbour's own update
@@ -1753,9 +1882,9 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_T_lane(EeParams P, const Ee
 #pragma unroll
             for (int j = 3; j >= 0; j--) e[j] = step(rl[j], gl[j]);
             if (q <= s.q1) {
-                float4* sq = reinterpret_cast<float4*>(sA + 64 * q);
+                float4* sq = sA + 64 * (q - s.q0);  // (pass-A part of Tbar, rho)
                 sq[0] = make_float4(e[0], rl[0], e[1], rl[1]);
-                sq[1] = make_float4(e[2], rl[2], e[3], rl[3]);
+                sq[32] = make_float4(e[2], rl[2], e[3], rl[3]);
             }
         }
     }
@@ -1778,8 +1907,8 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_T_lane(EeParams P, const Ee
         const Brick Bt = brick_of(S.tn);
         const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
         for (int q = s.q0; q <= s.q1; q++) {
-            const float4* sq = reinterpret_cast<const float4*>(sA + 64 * q);
-            const float4 s01 = sq[0], s23 = sq[1];
+            const float4* sq = sA + 64 * (q - s.q0);
+            const float4 s01 = sq[0], s23 = sq[32];
             const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
             const float al[4] = {s01.x, s01.z, s23.x, s23.z}, rl[4] = {s01.y, s01.w, s23.y, s23.w};
             const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
@@ -1793,6 +1922,15 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_cone_T_lane(EeParams P, const Ee
             }
         }
     }
+}
+
+__global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / EE_CONE_BLOCK_WARPS)
+    k_cone_T_lane(EeParams P, const EeBeamSpec* __restrict__ specs, const EeBeamGeom* __restrict__ geoms,
+                  const float* __restrict__ rev_grad, EeConeWork W, int nbeams, int cap,
+                  float* __restrict__ terma_grad) {
+    cone_tiles_run(P, W, nbeams, cap, [&](int b, int ray, int slot, float4* scratch) {
+        cone_T_line(P, specs, geoms, rev_grad, terma_grad, b, ray, slot, scratch);
+    });
 }
 
 // Adjoint of k_cone followed by the transpose of the REV TERMA resample:
@@ -1821,7 +1959,9 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
     const int line = blockIdx.x * CONE_WARPS + warp;
     if (line >= R.nlines) return;
     const int L = R.rev[0];
-    const int tY = line % R.rev[1], tZ = line / R.rev[1];
+    int tY, tZ;
+    kept_line(R, line, tY, tZ);
+    if (lit_form(R, (float)tY, (float)tZ) < 0.f) return;
     float* rho = sm + (size_t)warp * 3 * maxL;
     float* g = rho + maxL;
     float* Tb = g + maxL;
@@ -1830,7 +1970,7 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
     line_segment(P, G, R, tY, tZ, L, i0, n);
     if (n == 0) return;
     gather_line(P, S, G, R, nullptr, tY, tZ, i0, n, lane, rho, nullptr);
-    const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);  // bricked REV gradient
+    const Brick Bv = rev_store(R);  // bricked REV gradient
     const float* gin = rev_grad + G.arena_off + R.offset + rev_line(Bv, tY, tZ);
     const float inv_nphi = 1.f / (float)P.nphi;
     __syncwarp();
@@ -1931,7 +2071,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
         if (c < 3) {
             v = make_float4(R.A[3 * c], R.A[3 * c + 1], R.A[3 * c + 2], -R.q0[c]);
         } else if (c == 4) {
-            const Brick Bq = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
+            const Brick Bq = rev_store(R);
             v = make_float4(__int_as_float(Bq.sy), __int_as_float(Bq.sz), 0.f, 0.f);
         } else {
             v = make_float4(__int_as_float(R.rev[0]), __int_as_float(R.rev[1]), __int_as_float(R.rev[2]),
@@ -2077,7 +2217,9 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
     // read with two vector loads before the scatter, and {sy, sz, offset lo,
     // offset hi} (the REV gradient's brick strides and the cone's arena
     // offset), read with one before the flush
-    __shared__ int4 s_p[EE_MAX_RAYS][3];
+    // and {k0, k1, k2 | k each, lo | hi << 16}: the box cells inside the kept
+    // part, which the flush sends
+    __shared__ int4 s_p[EE_MAX_RAYS][4];
     __shared__ float4 s_A[EE_MAX_RAYS][3];
     const int b = blockIdx.z;
     const EeBeamGeom& G = geoms[b];
@@ -2163,9 +2305,11 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
             }
             sp[3] = s0;
         }
-        sp[a == 1 ? 0 : (a == 2 ? 1 : 2)] = l | (max(w, 0) << 16);
+        const int d = a == 1 ? 0 : (a == 2 ? 1 : 2);
+        sp[d] = l | (max(w, 0) << 16);
+        sp[12 + d] = max(0, R.so[d] - l) | max(0, R.so[d] + R.sn[d] - l) << 16;
         if (a == 0) {
-            const Brick Bv = rev_brick(R.rev[0], R.rev[1], R.rev[2]);
+            const Brick Bv = rev_store(R);
             sp[4] = Bv.sy;
             sp[5] = Bv.sz;
             sp[6] = (int)(unsigned)(R.offset & 0xffffffffll);
@@ -2267,11 +2411,13 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
                     const int k2 = __float2int_rd(((float)q1 + 0.5f) * inv1);
                     const int k1 = q1 - k2 * n1p;
                     // rows and slabs past the array's end and quads that
-                    // start past it hold the forward's border corners (0):
-                    // cleared, not sent; a quad that starts inside the array
-                    // ends in its last brick, whose padding nothing reads
-                    const int4 pv = s_p[r][2];
-                    if (4 * kq < pv.x && k1 < pv.y && k2 < pv.z)
+                    // start past it hold the forward's border corners (0), and
+                    // cells outside the kept part are not read: cleared, not
+                    // sent; a quad that starts inside ends in its last brick,
+                    // whose padding nothing reads
+                    const int4 pk = s_p[r][3];
+                    if (4 * kq >= (pk.x & 0xffff) && 4 * kq < (pk.x >> 16) && k1 >= (pk.y & 0xffff) &&
+                        k1 < (pk.y >> 16) && k2 >= (pk.z & 0xffff) && k2 < (pk.z >> 16))
                         red_v4(rb + bk_x(l0 + 4 * kq) + bk_y(Bv, l1 + k1) + bk_z(Bv, l2 + k2), (float)v.x * fx_inv,
                                (float)v.y * fx_inv, (float)v.z * fx_inv, (float)v.w * fx_inv);
                 }
@@ -2285,8 +2431,9 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
                             fmaf(a1.x, dx, fmaf(a1.y, dy, fmaf(a1.z, dz, a1.w))),
                             fmaf(a2.x, dx, fmaf(a2.y, dy, fmaf(a2.z, dz, a2.w))));
             if (!(q.y >= (float)R.rev[0] || q.z >= (float)R.rev[1] || q.x >= (float)R.rev[2] || q.x < 0.f ||
-                  q.y < 0.f || q.z < 0.f))
-                tri_brick_scatter(base + R.offset, rev_brick(R.rev[0], R.rev[1], R.rev[2]), q.y, q.z, q.x, gd);
+                  q.y < 0.f || q.z < 0.f) &&
+                lit_form(R, q.z, q.x) >= 0.5f * EE_LIT_READ)  // a line around the voxel can be lit, so all are kept
+                tri_brick_scatter(base + R.offset, rev_store(R), q.y, q.z, q.x, gd);
         }
     }
 }
@@ -2413,7 +2560,7 @@ cudaError_t ee_launch_geom_init(const EeBeamSpec* specs, EeBeamGeom* g, int nbea
 }
 
 cudaError_t ee_copy_status(const EeBeamGeom* geoms, int* status_host, int nbeams, cudaStream_t s) {
-    return cudaMemcpy2DAsync(status_host, sizeof(int), (const char*)geoms + offsetof(EeBeamGeom, status),
+    return cudaMemcpy2DAsync(status_host, sizeof(int), (const char*)geoms + offsetof(EeBeamGeomHead, status),
                              sizeof(EeBeamGeom), sizeof(int), nbeams, cudaMemcpyDeviceToHost, s);
 }
 
@@ -2433,6 +2580,24 @@ cudaError_t ee_launch_geometry(const EeParams& P, const EeBeamSpec* specs, EeBea
                                cudaStream_t s) {
     k_geometry<<<nbeams, 64, 0, s>>>(P, specs, geoms);
     return cudaGetLastError();
+}
+
+// The split of an SM's L1 between shared memory and cache that the kernels ask
+// for, on the current device.  An SM takes blocks of another kernel only at
+// the split that it has, so the TERMA and the cones, which would ask for 0 to
+// 16 KB, ask for the 100 KB that k_gather needs anyway: with three engines on
+// their own streams a 24 x 24 beam takes 0.697 against 0.727 ms a pass, 96
+// beams of 8^2..40^2 beamlets 26.9 against 27.3 ms; one engine alone loses 1 %
+// on the large batches (128 KB and more: 4 % and up; 64 KB: the three engines
+// gain nothing on the batches).
+cudaError_t ee_kernel_setup() {
+    const void* const fn[] = {(const void*)k_terma, (const void*)k_cone_tiles, (const void*)k_cone_lane,
+                              (const void*)k_cone_T_lane};
+    for (const void* f : fn) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 static size_t cone_smem(int maxL) { return sizeof(float) * ((size_t)CONE_WARPS * 3 * maxL + 2 * EE_MAX_RADII + EE_MAX_RADII); }
@@ -2471,13 +2636,13 @@ static cudaError_t smem_attr(const void* fn, size_t smem) {
 }
 
 cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* terma,
-                           float* rev, float2* samples, int nbeams, int max_lines, int max_line, cudaStream_t s,
-                           int lane_block) {
-    if (P.mode == 1 && samples) {  // exp kernel: one lane per line; the caller zeroed `rev`
-        dim3 grid(grid1(max_lines, lane_block), P.nrays, nbeams);
-        if (lane_block == 64) k_cone_lane<64><<<grid, 64, 0, s>>>(P, specs, geoms, terma, rev, samples);
-        else if (lane_block == 256) k_cone_lane<256><<<grid, 256, 0, s>>>(P, specs, geoms, terma, rev, samples);
-        else k_cone_lane<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, specs, geoms, terma, rev, samples);
+                           float* rev, const EeConeWork& work, int nbeams, int max_lines, int max_line,
+                           cudaStream_t s) {
+    if (P.mode == 1 && work.scratch) {  // exp kernel: one lane per line
+        const int cap = ee_cone_tiles_cap(max_lines);
+        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, EE_LIT_READ, work.counts, work.tiles, cap);
+        k_cone_lane<<<work.warps / EE_CONE_BLOCK_WARPS, EE_CONE_BLOCK_WARPS * 32, 0, s>>>(P, specs, geoms, terma, rev,
+                                                                                        work, nbeams, cap);
         return cudaGetLastError();
     }
     if (P.mode == EE_KERNEL_TABLE && P.nradii == TAB_NR) {  // exact O(n nr) table scan
@@ -2521,15 +2686,13 @@ cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const
 }
 
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
-                             float2* scratch, float* terma_grad, int nbeams, int max_lines, int max_line,
-                             cudaStream_t s, int lane_block) {
-    if (P.mode == 1 && scratch) {
-        dim3 grid(grid1(max_lines, lane_block), P.nrays, nbeams);
-        if (lane_block == 64) k_cone_T_lane<64><<<grid, 64, 0, s>>>(P, specs, geoms, rev_grad, scratch, terma_grad);
-        else if (lane_block == 256) k_cone_T_lane<256><<<grid, 256, 0, s>>>(P, specs, geoms, rev_grad, scratch, terma_grad);
-        else
-            k_cone_T_lane<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, specs, geoms, rev_grad,
-                                                                                          scratch, terma_grad);
+                             const EeConeWork& work, float* terma_grad, int nbeams, int max_lines, int max_line,
+                             cudaStream_t s) {
+    if (P.mode == 1 && work.scratch) {
+        const int cap = ee_cone_tiles_cap(max_lines);
+        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, 0.f, work.counts, work.tiles, cap);
+        k_cone_T_lane<<<work.warps / EE_CONE_BLOCK_WARPS, EE_CONE_BLOCK_WARPS * 32, 0, s>>>(
+            P, specs, geoms, rev_grad, work, nbeams, cap, terma_grad);
         return cudaGetLastError();
     }
     if (P.mode == EE_KERNEL_TABLE && P.nradii == TAB_NR) {

@@ -123,7 +123,7 @@ extern "C" int ee_beam_dose_noalloc(ee_context* ctx, const ee_beam* beam, const 
         cudaSuccess)
         return cuda_fail(e, "k_terma");
     if ((e = ee_launch_geometry(P, d_spec, d_geom, 1, s)) != cudaSuccess) return cuda_fail(e, "k_geometry");
-    EeBeamGeom G;  // host copy of the geometry (about 11 KB on the stack)
+    EeBeamGeomHead G;  // the sizes; the cones' frames stay on the device
     if ((e = cudaMemcpyAsync(&G, d_geom, sizeof(G), cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_fail(e, "geometry read-back");
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
@@ -135,17 +135,16 @@ extern "C" int ee_beam_dose_noalloc(ee_context* ctx, const ee_beam* beam, const 
         return ee_internal_fail(EE_ERR_CAPACITY, m);
     }
     G.arena_off = 0;
-    G.arena_cap = G.rev_total;
+    G.arena_cap = G.store_total;
     if ((e = cudaMemcpyAsync(d_geom, &G, sizeof(G), cudaMemcpyHostToDevice, s)) != cudaSuccess)
         return cuda_fail(e, "geometry upload");
     float* d_rev = d_terma + tvol;
     const long long nfull = (long long)P.size[0] * P.size[1] * P.size[2];
     if ((e = cudaMemsetAsync(d_dose, 0, sizeof(float) * nfull, s)) != cudaSuccess) return cuda_fail(e, "dose clear");
-    if ((e = cudaMemsetAsync(d_rev, 0, sizeof(float) * G.rev_total, s)) != cudaSuccess) return cuda_fail(e, "REV clear");
-    // no (rho, T) sample scratch here: the warp-per-line cone kernel keeps a
-    // line's samples in shared memory instead
-    float2* d_smp = nullptr;
-    if ((e = ee_launch_cone(P, d_spec, d_geom, d_terma, d_rev, d_smp, 1, G.max_lines, G.max_line, s)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(d_rev, 0, sizeof(float) * G.store_total, s)) != cudaSuccess) return cuda_fail(e, "REV clear");
+    // no work space for the lane cones here: the warp-per-line cone kernel
+    // keeps a line's samples in shared memory instead
+    if ((e = ee_launch_cone(P, d_spec, d_geom, d_terma, d_rev, EeConeWork(), 1, G.max_lines, G.max_line, s)) != cudaSuccess)
         return cuda_fail(e, "k_cone");
     if ((e = ee_launch_gather(P, d_spec, d_geom, d_rev, d_dose, 1, 1, G.rows > 0 ? G.rows : 1, s)) != cudaSuccess)
         return cuda_fail(e, "k_gather");

@@ -223,8 +223,8 @@ int ee_beam_dose_noalloc(ee_context *ctx, const ee_beam *beam, const float *d_fl
  * ee_plan_create fixes a batch of beams and the device buffers it reads and
  * writes (fluence in, dose out, and optionally dose gradient in / fluence
  * gradient out), sizes every intermediate from geometric upper bounds, runs
- * the batch once to validate them, autotunes the cone kernels' block shape
- * on it and captures the whole forward(+adjoint) chain into one CUDA graph.
+ * the batch once to validate them and captures the whole forward(+adjoint)
+ * chain into one CUDA graph.
  * ee_plan_launch replays that graph on the context stream with no host
  * synchronisation (new fluence / gradient values are read from the same
  * buffers); ee_plan_status then reports per-beam failures. */
