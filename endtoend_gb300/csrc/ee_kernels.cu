@@ -2038,7 +2038,7 @@ constexpr int ROW_WARPS = 8;
 // REV2XYZdose (device.cu:222-261) for all cones at once, a cone only at the
 // voxels whose lines it can light (lit_planes): the others read zeros.  A warp
 // takes a group of PY x PZ patient rows (EE_GATHER_*) of one beam's AABB and sweeps
-// the union of their spans in PX x PY x PZ patches, GATHER_V of them at a time
+// the union of their spans in PX x PY x PZ patches, V of them at a time
 // (one voxel of each per lane): a compact patch of voxels maps to a compact
 // patch of REV cells, so a corner load of the warp touches fewer cache lines
 // than a run of 32 voxels along x would.  A voxel sums the trilinear REV dose
@@ -2047,12 +2047,13 @@ constexpr int ROW_WARPS = 8;
 //
 // Bound by the load/store unit's data pipe (three quarters of its cycles): a
 // corner load of 32 scattered words takes two to three passes over the banks.
-// One read of a cone's map serves GATHER_V voxels; five resident blocks (48
-// registers, a few spilled words) beat four without spills, and six.  96 beams
-// of 8^2..40^2 beamlets on 200 x 200 x 160: 18.1 ms with one voxel per lane
-// (40 registers), 17.5 with two, 17.1 with four; 12.6 without the dark cones.
-constexpr int GATHER_V = 4;
-
+// One read of a cone's map serves V voxels; five resident blocks (48 registers,
+// a few spilled words) beat four without spills, and six.  96 beams of 8^2..40^2
+// beamlets on 200 x 200 x 160: 18.1 ms with one voxel per lane (40 registers),
+// 17.5 with two, 17.1 with four; 12.6 without the dark cones, 8.8 in chunks of
+// 15 beams and more.  gridDim.y blocks share a group's patches, every
+// gridDim.y-th V of them each (ee_launch_gather).
+template <int V>
 __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                            const EeBeamGeom* __restrict__ geoms,
                                                            const float* __restrict__ rev, float* __restrict__ dose,
@@ -2102,6 +2103,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
     const long long rbase = (long long)P.size[0] * (y + (long long)P.size[1] * z);
     const float* base = rev + G.arena_off;
     const float dy = (float)y - G.lim_off[1], dz = (float)z - G.lim_off[2];
+    if (wx0 + (int)blockIdx.y * V * PX > wx1) return;
     const float dx0 = (float)wx0 - G.lim_off[0];
     for (int r = lx; r < P.nrays; r += PX) {  // a row's eight lanes take its cones in turn
         float lo = 0.f, hi = 65535.f;
@@ -2121,11 +2123,11 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
         s_lit[warp][r][row] = e < 0 ? make_ushort2(1, 0) : make_ushort2((unsigned short)max(a, 0), (unsigned short)min(e, 65535));
     }
     __syncwarp();
-    for (int xs = wx0 + lx; xs - lx <= wx1; xs += GATHER_V * PX) {
-        float dx[GATHER_V], acc[GATHER_V];
-        int rel[GATHER_V];  // from the group's first voxel; -1: nothing to sum
+    for (int xs = wx0 + lx + blockIdx.y * V * PX; xs - lx <= wx1; xs += gridDim.y * V * PX) {
+        float dx[V], acc[V];
+        int rel[V];  // from the group's first voxel; -1: nothing to sum
 #pragma unroll
-        for (int v = 0; v < GATHER_V; v++) {
+        for (int v = 0; v < V; v++) {
             const int x = xs + v * PX;
             dx[v] = (float)x - G.lim_off[0];
             acc[v] = 0.f;
@@ -2138,9 +2140,9 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
         }
         for (int r = 0; r < P.nrays; r++) {
             const ushort2 lit = s_lit[warp][r][row];
-            bool on[GATHER_V], any = false;
+            bool on[V], any = false;
 #pragma unroll
-            for (int v = 0; v < GATHER_V; v++) {
+            for (int v = 0; v < V; v++) {
                 on[v] = rel[v] >= (int)lit.x && rel[v] <= (int)lit.y;
                 any |= on[v];
             }
@@ -2155,7 +2157,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
             const float cx = fmaf(a0.y, dy, fmaf(a0.z, dz, a0.w)), cy = fmaf(a1.y, dy, fmaf(a1.z, dz, a1.w)),
                         cz = fmaf(a2.y, dy, fmaf(a2.z, dz, a2.w));
 #pragma unroll
-            for (int v = 0; v < GATHER_V; v++) {
+            for (int v = 0; v < V; v++) {
                 const float qx = fmaf(a0.x, dx[v], cx), qy = fmaf(a1.x, dx[v], cy), qz = fmaf(a2.x, dx[v], cz);
                 if (on[v] && !(qy >= (float)Bq.n0 || qz >= (float)Bq.n1 || qx >= (float)Bq.n2 || qx < 0.f ||
                                qy < 0.f || qz < 0.f))
@@ -2163,7 +2165,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
             }
         }
 #pragma unroll
-        for (int v = 0; v < GATHER_V; v++) {
+        for (int v = 0; v < V; v++) {
             const int x = xs + v * PX;
             if (x < x0 || x > x1) continue;
             if (mode == 2) out[rbase + x] = acc[v];
@@ -2669,9 +2671,22 @@ cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const
 
 cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev,
                              float* dose, int nbeams, int dose_mode, int max_rows, cudaStream_t s) {
-    long long nfull = (long long)P.size[0] * P.size[1] * P.size[2];
-    dim3 grid(grid1(max_rows, ROW_WARPS), 1, nbeams);
-    k_gather<<<grid, ROW_WARPS * 32, 0, s>>>(P, specs, geoms, rev, dose, dose_mode, nfull);
+    const long long nfull = (long long)P.size[0] * P.size[1] * P.size[2];
+    // A warp's patches are a chain of loads, and five blocks are resident per SM.
+    // Up to 12 rounds of resident blocks, two blocks share the patches of a
+    // group, or the last round is long (one 24 x 24 beam, 1000 blocks: 0.199 ->
+    // 0.143 ms; six beams, 6000: 0.565 -> 0.477); above, the set-up that each
+    // repeats costs more than that (12 beams, 12000: 1.03 -> 1.07; 96: 8.8 ->
+    // 9.3).  Below three blocks per SM four blocks take two patches at a time
+    // (a 64^3 slab, 96 blocks: 0.086 -> 0.038 ms, 0.058 with two blocks of four
+    // patches; 384: 0.119 -> 0.102; 1000: 0.150 against 0.143).
+    const int blocks = grid1(max_rows, ROW_WARPS);
+    const long long all = (long long)blocks * nbeams;
+    if (all < 456)
+        k_gather<2><<<dim3(blocks, 4, nbeams), ROW_WARPS * 32, 0, s>>>(P, specs, geoms, rev, dose, dose_mode, nfull);
+    else
+        k_gather<4><<<dim3(blocks, all < 9120 ? 2 : 1, nbeams), ROW_WARPS * 32, 0, s>>>(P, specs, geoms, rev, dose,
+                                                                                       dose_mode, nfull);
     return cudaGetLastError();
 }
 
