@@ -149,27 +149,43 @@ __device__ __forceinline__ Brick rev_store(const EeRayGeom& R) {
 // rev_line(B, tY, tZ) + bk_x(i).
 __device__ __forceinline__ int rev_line(const Brick& B, int tY, int tZ) { return bk_y(B, tY) + bk_z(B, tZ); }
 
-// tri_border on a bricked box: the same weights, products and order, so the
-// value is bit-identical to tri_border on the x-fastest box.
-__device__ __forceinline__ float tri_brick(const float* __restrict__ v, const Brick& B, float x, float y, float z) {
+// The cell of a point and whether all its corners lie in the box; the float to
+// integer conversion saturates, so a point far outside is outside here too.
+__device__ __forceinline__ bool brick_cell(const Brick& B, float x, float y, float z, int& i, int& j, int& k) {
+    i = __float2int_rd(x);
+    j = __float2int_rd(y);
+    k = __float2int_rd(z);
+    return (unsigned)i < (unsigned)(B.n0 - 1) && (unsigned)j < (unsigned)(B.n1 - 1) && (unsigned)k < (unsigned)(B.n2 - 1);
+}
+
+// tri_border on a bricked box at a point whose corners all lie in it: the same
+// weights and order.  The corners are addressed from the first one by per-axis
+// steps (+1, +4, +16 inside a brick; +61, +sy - 12, +sz - 48 across a brick
+// face), which with one range test per axis saves the forward cone 7 % against a
+// brick offset per corner and tri_border's tests.
+__device__ __forceinline__ float tri_brick_cell(const float* __restrict__ v, const Brick& B, float x, float y, float z,
+                                                int i, int j, int k) {
+    const float ax = x - (float)i, ay = y - (float)j, az = z - (float)k;
+    const float* p = v + (i + 60 * (i >> 2) + 4 * j + (j >> 2) * (B.sy - 16) + 16 * k + (k >> 2) * (B.sz - 64));
+    const int dx = (i & 3) == 3 ? 61 : 1, dy = (j & 3) == 3 ? B.sy - 12 : 4, dz = (k & 3) == 3 ? B.sz - 48 : 16;
+    const float c000 = __ldg(p), c100 = __ldg(p + dx), c010 = __ldg(p + dy), c110 = __ldg(p + dy + dx);
+    const float c001 = __ldg(p + dz), c101 = __ldg(p + dz + dx), c011 = __ldg(p + dz + dy),
+                c111 = __ldg(p + dz + dy + dx);
+    const float c00 = c000 + ax * (c100 - c000), c10 = c010 + ax * (c110 - c010);
+    const float c01 = c001 + ax * (c101 - c001), c11 = c011 + ax * (c111 - c011);
+    const float c0 = c00 + ay * (c10 - c00), c1 = c01 + ay * (c11 - c01);
+    return c0 + az * (c1 - c0);
+}
+
+// tri_border on a bricked box at any other point: the corner values that
+// exist, weighted; 0 from one cell outside the box on.  Callers keep it out of
+// their unrolled samples: there it was a quarter of the forward cone's code and
+// a third of the gather's, more than the instruction cache holds.
+__device__ __forceinline__ float tri_brick_edge(const float* __restrict__ v, const Brick B, float x, float y, float z) {
     if (!(x > -1.f && x < (float)B.n0 && y > -1.f && y < (float)B.n1 && z > -1.f && z < (float)B.n2)) return 0.f;
-    float fx = floorf(x), fy = floorf(y), fz = floorf(z);
-    int i = (int)fx, j = (int)fy, k = (int)fz;
-    float ax = x - fx, ay = y - fy, az = z - fz;
-    if (i >= 0 && j >= 0 && k >= 0 && i + 1 < B.n0 && j + 1 < B.n1 && k + 1 < B.n2) {
-        const int x0 = bk_x(i), x1 = bk_x(i + 1), y0 = bk_y(B, j), y1 = bk_y(B, j + 1);
-        const int z0 = bk_z(B, k), z1 = bk_z(B, k + 1);
-        const float* p0 = v + z0;
-        const float* p1 = v + z1;
-        float c000 = __ldg(p0 + y0 + x0), c100 = __ldg(p0 + y0 + x1), c010 = __ldg(p0 + y1 + x0),
-              c110 = __ldg(p0 + y1 + x1);
-        float c001 = __ldg(p1 + y0 + x0), c101 = __ldg(p1 + y0 + x1), c011 = __ldg(p1 + y1 + x0),
-              c111 = __ldg(p1 + y1 + x1);
-        float c00 = c000 + ax * (c100 - c000), c10 = c010 + ax * (c110 - c010);
-        float c01 = c001 + ax * (c101 - c001), c11 = c011 + ax * (c111 - c011);
-        float c0 = c00 + ay * (c10 - c00), c1 = c01 + ay * (c11 - c01);
-        return c0 + az * (c1 - c0);
-    }
+    const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
+    const int i = (int)fx, j = (int)fy, k = (int)fz;
+    const float ax = x - fx, ay = y - fy, az = z - fz;
     float acc = 0.f;
 #pragma unroll
     for (int dk = 0; dk < 2; dk++) {
@@ -193,11 +209,20 @@ __device__ __forceinline__ float tri_brick(const float* __restrict__ v, const Br
     return acc;
 }
 
-// tri_brick for a point the caller has placed in [0, n0) x [0, n1) x [0, n2)
-// (B's sizes and brick strides): no entry or lower-bound tests, and the
-// corners addressed from the first one by per-axis steps (+1, +4, +16 inside
-// a brick; +61, +sy - 12, +sz - 48 across a brick face).  The same loads,
-// weights and order as tri_brick.
+// tri_border on a bricked box.
+__device__ __forceinline__ float tri_brick(const float* __restrict__ v, const Brick& B, float x, float y, float z) {
+    int i, j, k;
+    return brick_cell(B, x, y, z, i, j, k) ? tri_brick_cell(v, B, x, y, z, i, j, k) : tri_brick_edge(v, B, x, y, z);
+}
+
+// tri_brick for a point the caller has placed in [0, n0) x [0, n1) x [0, n2):
+// no entry or lower-bound tests.  The last cell of an axis goes out of line:
+// inlined for four voxels it is a third of the gather's code.  (With
+// tri_brick_cell's body the gather at 48 registers spills twice as much: 96
+// beams 8.7 -> 9.1 ms.)
+__device__ __noinline__ float tri_brick_last(const float* __restrict__ v, const Brick B, float x, float y, float z) {
+    return tri_brick_edge(v, B, x, y, z);
+}
 __device__ __forceinline__ float tri_brick_in(const float* __restrict__ v, const Brick& B, float x, float y, float z) {
     const float fx = floorf(x), fy = floorf(y), fz = floorf(z);
     const int i = (int)fx, j = (int)fy, k = (int)fz;
@@ -213,7 +238,7 @@ __device__ __forceinline__ float tri_brick_in(const float* __restrict__ v, const
         float c0 = c00 + ay * (c10 - c00), c1 = c01 + ay * (c11 - c01);
         return c0 + az * (c1 - c0);
     }
-    return tri_brick(v, B, x, y, z);  // the last cell of an axis: border corners
+    return tri_brick_last(v, B, x, y, z);
 }
 
 // Transpose of tri_brick (same weights as tri_border_scatter).  Each (y, z)
@@ -222,7 +247,8 @@ __device__ __forceinline__ float tri_brick_in(const float* __restrict__ v, const
 // 3), and a second one on slot 0 of the next brick row only then (or when
 // corner i is outside the box).  The other slots of a quad receive +0.  No
 // branch on the slot, so the lanes of a warp issue the same two reductions.
-__device__ __forceinline__ void tri_brick_scatter(float* v, const Brick& B, float x, float y, float z, float g) {
+// Points with corners outside the box:
+__device__ __forceinline__ void tri_brick_scatter_edge(float* v, const Brick B, float x, float y, float z, float g) {
     if (!(x > -1.f && x < (float)B.n0 && y > -1.f && y < (float)B.n1 && z > -1.f && z < (float)B.n2)) return;
     float fx = floorf(x), fy = floorf(y), fz = floorf(z);
     int i = (int)fx, j = (int)fy, k = (int)fz;
@@ -250,6 +276,29 @@ __device__ __forceinline__ void tri_brick_scatter(float* v, const Brick& B, floa
             float* row = v + bk_y(B, jj) + bk_z(B, kk);
             if (in0) red_v4(row + xa, w * p0, w * p1, w * p2, w * p3);
             if (in1 && !both) red_v4(row + xb, w * ax, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
+// All corners in the box, of cell (i, j, k): no tests per corner row.
+__device__ __forceinline__ void tri_brick_scatter_cell(float* v, const Brick& B, float x, float y, float z, float g,
+                                                       int i, int j, int k) {
+    const float ax = x - (float)i, ay = y - (float)j, az = z - (float)k;
+    const int o = i & 3;
+    float* const p = v + (((i >> 2) << 6) + 4 * j + (j >> 2) * (B.sy - 16) + 16 * k + (k >> 2) * (B.sz - 64));
+    const int dy = (j & 3) == 3 ? B.sy - 12 : 4, dz = (k & 3) == 3 ? B.sz - 48 : 16;
+    const float a0 = 1.f - ax;
+    const float p0 = o == 0 ? a0 : 0.f, p1 = o == 1 ? a0 : (o == 0 ? ax : 0.f);
+    const float p2 = o == 2 ? a0 : (o == 1 ? ax : 0.f), p3 = o == 3 ? a0 : (o == 2 ? ax : 0.f);
+#pragma unroll
+    for (int dk = 0; dk < 2; dk++) {
+        const float wz = dk ? az : 1.f - az;
+#pragma unroll
+        for (int dj = 0; dj < 2; dj++) {
+            const float w = (dj ? ay : 1.f - ay) * wz * g;
+            float* const row = p + (dj ? dy : 0) + (dk ? dz : 0);
+            red_v4(row, w * p0, w * p1, w * p2, w * p3);
+            if (o == 3) red_v4(row + 64, w * ax, 0.f, 0.f, 0.f);
         }
     }
 }

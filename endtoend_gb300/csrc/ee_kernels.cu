@@ -1399,7 +1399,7 @@ __device__ __forceinline__ void tab_adj_line(const EeParams& P, const EeBeamSpec
             const float v = Tb[k];
             if (rho[k] < 0.f || v == 0.f) continue;
             const f3 gp = gl + gx * (float)(i0 + k);
-            tri_brick_scatter(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
+            tri_brick_scatter_edge(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
                               gp.z - (float)S.t0[2], v);
         }
     }
@@ -1516,7 +1516,9 @@ __device__ __forceinline__ LaneSpan lane_span(const EeParams& P, const EeBeamSpe
                  g.y < (float)P.bb0[1] || g.y >= (float)(P.bb0[1] + P.bbs[1]) || g.z < (float)P.bb0[2] ||
                  g.z >= (float)(P.bb0[2] + P.bbs[2]));
     };
+#pragma unroll 1
     while (s.i0 <= s.i1 && !valid(s.i0)) s.i0++;
+#pragma unroll 1
     while (s.i1 > s.i0 && !valid(s.i1)) s.i1--;
     if (max(f0, s.i0) > min(f1, s.i1)) return s;
     s.q0 = max(f0, s.i0) >> 2;
@@ -1651,11 +1653,13 @@ __device__ __forceinline__ void cone_tiles_run(const EeParams& P, const EeConeWo
 // reaches down to it; the walk down the line starts at q1 and takes its
 // densities past q0 from the texture.  So each walk visits 0.42 of the
 // samples, and the (rho, T) scratch and the partial dose only the span.
-// Bound by latency (long-scoreboard stalls at 22 resident warps per SM, issue
-// 27 % on one beam).  Against both walks over the whole segment with the box
-// tests at every sample: one 24 x 24 beam 0.427 -> 0.254 ms, 96 beams of
-// 8^2..40^2 beamlets 27.8 -> 15.0 ms, 20 beams of 128^2 pixels 9.7 -> 6.1 ms
-// (200 x 200 x 160 at 2 mm).
+// Bound by latency and by the instruction cache (24 warps of 80 registers per
+// SM; half of the issue slots; a sample's corners in the TERMA box are
+// addressed by steps, and samples at its faces share one loop per quad: 50 ->
+// 41 KB of code, 96 beams 10.5 -> 9.4 ms).  Against both walks over the whole
+// segment with the box tests at every sample: one 24 x 24 beam 0.427 -> 0.183
+// ms, 96 beams of 8^2..40^2 beamlets 27.8 -> 9.4 ms, 20 beams of 128^2 pixels
+// 9.7 -> 4.0 ms (200 x 200 x 160 at 2 mm).
 // Samples of an end quad outside [i0, i1] get dose 0 (they are inside the
 // read span or never read); their zero TERMA and unit factors leave the
 // recurrence as it is.
@@ -1678,6 +1682,7 @@ __device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* _
         int z0, z1;
         line_read_span(G, R, tY, tZ, R.rev[0], z0, z1);
         const int e0 = lit ? s.i0 >> 2 : 0x3fffffff, e1 = lit ? s.i1 >> 2 : 0x3fffffff;
+#pragma unroll 1
         for (int q = z0 >> 2; q <= (z1 >> 2); q++) {
             if (q == e0) q = e1;
             else *reinterpret_cast<float4*>(out + 64 * q) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1704,19 +1709,34 @@ __device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* _
             tm = t; hm1 = h1; hm2 = h2;
             return d;
         };
+#pragma unroll 1
         for (int q = s.q0; q <= s.q1; q++) {
             // the quad's samples gathered before the recurrence consumes
             // them, so each lane keeps several independent loads in flight
             float rr[4], tt[4], dq[4];
+            unsigned edge = 0;  // samples with corners outside the TERMA box
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int i = 4 * q + j;
                 const bool in = i >= s.i0 && i <= s.i1;
                 const f3 g = sample_point(F, i);
                 rr[j] = rho_at(P, g);
-                tt[j] = tri_brick(tb, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z);
                 if (!in) rr[j] = -1.f;
+                const f3 p = mk(g.x - t0.x, g.y - t0.y, g.z - t0.z);
+                int ci, cj, ck;
+                const bool cell = brick_cell(Bt, p.x, p.y, p.z, ci, cj, ck);
+                tt[j] = cell ? tri_brick_cell(tb, Bt, p.x, p.y, p.z, ci, cj, ck) : 0.f;
+                edge |= cell ? 0u : 1u << j;
                 if (!(rr[j] >= 0.f)) tt[j] = 0.f;
+            }
+#pragma unroll 1
+            for (; edge; edge &= edge - 1) {
+                const int w = __ffs((int)edge) - 1;
+                const f3 g = sample_point(F, 4 * q + w);
+                const float e = tri_brick_edge(tb, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (j == w && rr[j] >= 0.f) tt[j] = e;
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) dq[j] = step(rr[j], tt[j]);
@@ -1725,6 +1745,7 @@ __device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* _
             sq[32] = make_float4(rr[2], tt[2], rr[3], tt[3]);
             *reinterpret_cast<float4*>(out + 64 * q) = make_float4(dq[0], dq[1], dq[2], dq[3]);
         }
+#pragma unroll 1
         for (int q = s.q1 + 1; q <= qe; q++) {
             float rr[4], dq[4];
 #pragma unroll
@@ -1752,6 +1773,7 @@ __device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* _
             tm = t; hm1 = h1; hm2 = h2;
             return v ? (below + d) * inv_nphi : 0.f;
         };
+#pragma unroll 1
         for (int q = s.q1; q >= s.q0; q--) {
             const float4* sq = smp + 64 * (q - s.q0);
             const float4 s01 = sq[0], s23 = sq[32];
@@ -1763,6 +1785,7 @@ __device__ __forceinline__ void cone_line(const EeParams& P, const EeBeamSpec* _
             dq.x = step(s01.x, s01.y, o4.x);
             *reinterpret_cast<float4*>(out + 64 * q) = dq;
         }
+#pragma unroll 1
         for (int q = s.q0 - 1; q >= qs; q--) {
             float rr[4], dq[4];
 #pragma unroll
@@ -1829,7 +1852,9 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
 // of the field span have a TERMA gradient: pass A stops below q0, pass B
 // above q1, and outside the span each only updates Z, with the densities of
 // the texture; the scratch holds the span alone.  One 24 x 24 beam 0.428 ->
-// 0.301 ms, 20 beams of 128^2 pixels 8.1 -> 5.4 ms.
+// 0.242 ms, 20 beams of 128^2 pixels 8.1 -> 2.9 ms; of that 0.265 -> 0.242 by
+// scattering interior samples without tests per corner row and those at the
+// box's faces in one loop per quad.
 __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec* __restrict__ specs,
                                             const EeBeamGeom* __restrict__ geoms, const float* __restrict__ rev_grad,
                                             float* __restrict__ terma_grad, int b, int ray, int slot,
@@ -1869,6 +1894,7 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
     };
     {   // pass A, down from i1
         begin(RC.row_fwd);
+#pragma unroll 1
         for (int q = s.i1 >> 2; q >= s.q0; q--) {
             const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
             const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
@@ -1890,6 +1916,7 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
     }
     {   // pass B, up from i0; scatter
         begin(RC.row_rev);
+#pragma unroll 1
         for (int q = s.i0 >> 2; q < s.q0; q++) {
             const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
             const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
@@ -1906,19 +1933,34 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
         float* tg = terma_grad + S.t_off;
         const Brick Bt = brick_of(S.tn);
         const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
+#pragma unroll 1
         for (int q = s.q0; q <= s.q1; q++) {
             const float4* sq = sA + 64 * (q - s.q0);
             const float4 s01 = sq[0], s23 = sq[32];
             const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
             const float al[4] = {s01.x, s01.z, s23.x, s23.z}, rl[4] = {s01.y, s01.w, s23.y, s23.w};
             const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
+            float tot[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float tot = al[j] + step(rl[j], gl[j]);
-                if (rl[j] >= 0.f && tot != 0.f) {
-                    const f3 g = sample_point(F, 4 * q + j);
-                    tri_brick_scatter(tg, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z, tot);
-                }
+                const float e = al[j] + step(rl[j], gl[j]);
+                tot[j] = rl[j] >= 0.f ? e : 0.f;
+            }
+            unsigned edge = 0;  // samples with corners outside the TERMA box
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const f3 g = sample_point(F, 4 * q + j), p = mk(g.x - t0.x, g.y - t0.y, g.z - t0.z);
+                int ci, cj, ck;
+                const bool cell = brick_cell(Bt, p.x, p.y, p.z, ci, cj, ck);
+                if (tot[j] != 0.f && cell) tri_brick_scatter_cell(tg, Bt, p.x, p.y, p.z, tot[j], ci, cj, ck);
+                edge |= tot[j] != 0.f && !cell ? 1u << j : 0u;
+            }
+#pragma unroll 1
+            for (; edge; edge &= edge - 1) {
+                const int w = __ffs((int)edge) - 1;
+                const f3 g = sample_point(F, 4 * q + w);
+                const float e = w == 0 ? tot[0] : w == 1 ? tot[1] : w == 2 ? tot[2] : tot[3];
+                tri_brick_scatter_edge(tg, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z, e);
             }
         }
     }
@@ -2001,7 +2043,7 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
         float v = Tb[k];
         if (rho[k] < 0.f || v == 0.f) continue;
         f3 gp = gl + gx * (float)(i0 + k);
-        tri_brick_scatter(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
+        tri_brick_scatter_edge(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
                            gp.z - (float)S.t0[2], v);
     }
 }
@@ -2050,7 +2092,7 @@ constexpr int ROW_WARPS = 8;
 // One read of a cone's map serves V voxels; five resident blocks (48 registers,
 // a few spilled words) beat four without spills, and six.  96 beams of 8^2..40^2
 // beamlets on 200 x 200 x 160: 18.1 ms with one voxel per lane (40 registers),
-// 17.5 with two, 17.1 with four; 12.6 without the dark cones, 8.8 in chunks of
+// 17.5 with two, 17.1 with four; 12.6 without the dark cones, 8.7 in chunks of
 // 15 beams and more.  gridDim.y blocks share a group's patches, every
 // gridDim.y-th V of them each (ee_launch_gather).
 template <int V>
@@ -2435,7 +2477,7 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
             if (!(q.y >= (float)R.rev[0] || q.z >= (float)R.rev[1] || q.x >= (float)R.rev[2] || q.x < 0.f ||
                   q.y < 0.f || q.z < 0.f) &&
                 lit_form(R, q.z, q.x) >= 0.5f * EE_LIT_READ)  // a line around the voxel can be lit, so all are kept
-                tri_brick_scatter(base + R.offset, rev_store(R), q.y, q.z, q.x, gd);
+                tri_brick_scatter_edge(base + R.offset, rev_store(R), q.y, q.z, q.x, gd);
         }
     }
 }
