@@ -863,6 +863,79 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone(EeParams P, const EeBe
     for (int k = lane; k < n; k += 32) out[bk_x(i0 + k)] = D[k];
 }
 
+struct LineFrame {
+    f3 gl, gx;  // patient voxel index of sample 0, and its step per sample
+};
+
+__device__ __forceinline__ f3 sample_point(const LineFrame& F, int i) { return F.gl + F.gx * (float)i; }
+
+__device__ __forceinline__ float rho_at(const EeParams& P, f3 g) {
+    return tex3D<float>(P.dens_tex, g.x + 0.5f, g.y + 0.5f, g.z + 0.5f);
+}
+
+// What a lane needs of its line.  [i0, i1]: the samples inside the BEV crop
+// box and the calc bbox by the reference's own tests (device.cu:51-70).  Every
+// test is a comparison of an affine function of i, which stays monotone in
+// FP32, so the samples that pass are one interval: the analytic segment
+// trimmed at its ends by the tests themselves, and no sample in between needs
+// them again.  [q0, q1]: the quads of [i0, i1] that hold the samples whose
+// TERMA corners can lie in the field (field_forms); q1 < q0: no such sample,
+// so neither dose nor TERMA gradient.
+struct LaneSpan {
+    int i0, i1, q0, q1;
+};
+
+__device__ __forceinline__ LaneSpan lane_span(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
+                                              const EeRayGeom& R, int tY, int tZ, LineFrame& F) {
+    const float fy = (float)tY, fz = (float)tZ;
+    F.gl = ld3(R.G0) + ld3(R.Gy) * fy + ld3(R.Gz) * fz;
+    F.gx = ld3(R.Gx);
+    LaneSpan s{0, -1, 0, -1};
+    if (lit_form(R, fy, fz) < 0.f) return s;
+    int n;
+    line_segment(P, G, R, tY, tZ, R.rev[0], s.i0, n);
+    s.i1 = s.i0 + n - 1;
+    if (n <= 0) return s;
+    // field span: the four sides, raised by more than their rounding, cut the
+    // line to one interval.  The forms hold in front of the source; beamlet_of
+    // takes |depth|, so a segment that does not stay in front of it is not
+    // restricted
+    float lo = -1e9f, hi = 1e9f;
+    const float pr = fmaf(R.front[2], fy, fmaf(R.front[3], fz, R.front[1]));
+    const bool front = fminf(fmaf(R.front[0], (float)s.i0, pr), fmaf(R.front[0], (float)s.i1, pr)) > 1e-2f * S.isodist;
+    if (front) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float al = R.side[k][0], be = fmaf(R.side[k][2], fy, fmaf(R.side[k][3], fz, R.side[k][1]));
+            if (fabsf(al) < 1e-20f) {
+                if (be < 0.f) { lo = 1e9f; hi = -1e9f; }
+            } else {
+                const float t = fminf(fmaxf(__fdividef(-be, al), -1e9f), 1e9f);
+                if (al > 0.f) lo = fmaxf(lo, t);
+                else hi = fminf(hi, t);
+            }
+        }
+    }
+    const int f0 = max(s.i0, (int)ceilf(lo - 0.01f)), f1 = min(s.i1, (int)floorf(hi + 0.01f));
+    if (f0 > f1) return s;
+    const f3 bl = ld3(R.B0) + ld3(R.By) * fy + ld3(R.Bz) * fz, bx = ld3(R.Bx);
+    auto valid = [&](int i) {
+        const f3 bev = bl + bx * (float)i, g = sample_point(F, i);
+        return !(bev.x < 0.f || bev.y < 0.f || bev.z < 0.f || bev.x >= (float)G.bev[0] || bev.y >= (float)G.bev[1] ||
+                 bev.z >= (float)G.bev[2] || g.x < (float)P.bb0[0] || g.x >= (float)(P.bb0[0] + P.bbs[0]) ||
+                 g.y < (float)P.bb0[1] || g.y >= (float)(P.bb0[1] + P.bbs[1]) || g.z < (float)P.bb0[2] ||
+                 g.z >= (float)(P.bb0[2] + P.bbs[2]));
+    };
+#pragma unroll 1
+    while (s.i0 <= s.i1 && !valid(s.i0)) s.i0++;
+#pragma unroll 1
+    while (s.i1 > s.i0 && !valid(s.i1)) s.i1--;
+    if (max(f0, s.i0) > min(f1, s.i1)) return s;
+    s.q0 = max(f0, s.i0) >> 2;
+    s.q1 = min(f1, s.i1) >> 2;
+    return s;
+}
+
 // ------------------------------------- cone: exact table scan, O(n nr) ----
 // The reference's RowConvolve walk (device.cu:126-211) with the cumulative
 // kernel interpolated linearly between its nr = 24 radial boundaries (the
@@ -963,61 +1036,60 @@ __device__ __forceinline__ TabRow tab_row(const float* t, bool fwd) {
 
 // exclusive prefix sum over the W-lane group of `lane` (W = 32: the warp; W =
 // 16: each half separately); all 32 lanes take part
-template <int W = 32>
-__device__ __forceinline__ float warp_excl_scan(float x, int lane) {
+__device__ __forceinline__ float warp_excl_scan(float x, int lane, int W) {
     float s = x;
 #pragma unroll
-    for (int off = 1; off < W; off <<= 1) {
+    for (int off = 1; off < 32; off <<= 1) {  // lane < W: the last step adds nothing when W = 16
         const float y = __shfl_up_sync(FULL, s, off, W);
         if (lane >= off) s += y;
     }
     return s - x;
 }
 
-template <bool FWD>
-__device__ __forceinline__ int wmap(int w, int n) { return FWD ? w : n - 1 - w; }
+__device__ __forceinline__ int wmap(bool fwd, int w, int n) { return fwd ? w : n - 1 - w; }
 
 // lane chunks of a line over the W lanes that share it: the shortest length
 // that covers it, so that as many lanes as possible work (measured faster
 // than odd lengths, which spread the lanes' strided shared-memory accesses
 // over all the banks but leave up to a third of the lanes idle)
-template <int W = 32>
-__device__ __forceinline__ void tab_chunk(int n, int lane, int& w0, int& w1) {
+__device__ __forceinline__ void tab_chunk(int W, int n, int lane, int& w0, int& w1) {
     const int cs = max(1, (n + W - 1) / W);
     w0 = min(n, lane * cs);
     w1 = min(n, w0 + cs);
 }
 
-// M_w, P_w, SV_w = T_{w-1} and SVM_w in walk order (separate arrays: lanes
-// reading scattered samples then spread over all the banks); T is 0 at
-// sentinels.
-template <bool FWD, int W = 32>
-__device__ __forceinline__ void tab_build(const float* rho, const float* T, int n, int lane, float delr, float* Mv,
-                                          float* Pv, float* SVv, float* SVMv) {
+// M_w, P_w and SVM_w for w >= a in walk order, P from sample a on (separate
+// arrays: lanes reading scattered samples then spread over all the banks); T is
+// 0 below a.  SV_w = T_{w-1} is read from T, which has a zero at T[-1] and T[n].
+__device__ __forceinline__ void tab_build(bool fwd, int W, const float* rho, const float* T, int n, int a, int lane,
+                                          float delr, float* Mv, float* Pv, float* SVMv) {
     int w0, w1;
-    tab_chunk<W>(n, lane, w0, w1);
-    const float tp0 = (w0 > 0 && w0 < w1) ? T[wmap<FWD>(w0 - 1, n)] : 0.f;
+    tab_chunk(W, n - a, lane, w0, w1);
+    w0 += a;
+    w1 += a;
+    const float tp0 = (w0 > a && w0 < w1) ? T[wmap(fwd, w0 - 1, n)] : 0.f;
     float sd = 0.f, svm = 0.f, tp = tp0;
+#pragma unroll 1
     for (int w = w0; w < w1; w++) {  // chunk sums, P local to the chunk
-        const int i = wmap<FWD>(w, n);
+        const int i = wmap(fwd, w, n);
         const float r = rho[i], t = T[i];
         const float d = r >= 0.f ? delr * r : 0.f;
         svm = fmaf(t - tp, fmaf(0.5f, d, sd), svm);
         sd += d;
         tp = t;
     }
-    const float Pst = warp_excl_scan<W>(sd, lane);
-    float S = warp_excl_scan<W>(fmaf(Pst, tp - tp0, svm), lane);
+    const float Pst = warp_excl_scan(sd, lane, W);
+    float S = warp_excl_scan(fmaf(Pst, tp - tp0, svm), lane, W);
     float Pw = Pst;
     tp = tp0;
+#pragma unroll 1
     for (int w = w0; w < w1; w++) {
-        const int i = wmap<FWD>(w, n);
+        const int i = wmap(fwd, w, n);
         const float r = rho[i], t = T[i];
         const float d = r >= 0.f ? delr * r : 0.f;
         const float M = fmaf(0.5f, d, Pw);
         Mv[w] = M;
         Pv[w] = Pw;
-        SVv[w] = tp;
         SVMv[w] = S;
         S = fmaf(t - tp, M, S);
         Pw += d;
@@ -1025,105 +1097,130 @@ __device__ __forceinline__ void tab_build(const float* rho, const float* T, int 
     }
 }
 
-// Receivers of one walk direction.  FWD writes D[i]; the reverse direction
-// adds its part, divides by nphi and zeroes sentinel samples.  X: this lane's
-// window ends, X[32 j] = x_j (shared memory, so the loops over the window
-// ends stay loops).
-template <bool FWD, int W = 32>
-__device__ __forceinline__ void tab_receivers(const float* Mv, const float* Pv, const float* SVv, const float* SVMv,
-                                              const float* rho, int n, int lane, const TabRow& K, int* X, float* D,
-                                              float nphi) {
+// Receivers of one walk direction, added to D (sources in [a, e], a lane's
+// receivers a contiguous chunk of (a, n)).  X: this lane's window ends, X[32 j]
+// = x_j (shared memory, so the loops over the window ends stay loops).
+//
+// Only the ends inside the sources' range cost a step: an end with R_j >= P_w -
+// M_a has not left a, where the prefix sums are 0; one past e + 1 (js of them)
+// has every source behind it, SV is 0 there and the ends' SVM terms add up to
+// beta_js.  So a receiver inside the range visits the radii up to its distance
+// from a and one beyond it those between the range's two ends: 5 of the 20 that
+// a 40 cm line has, on average, and receivers at and before a none.  Neither
+// s nor the clip matter before R_{nr-2} reaches past a: the general form runs
+// only there.
+__device__ __forceinline__ void tab_receivers(bool fwd, int W, const float* Mv, const float* Pv, const float* T,
+                                              const float* SVMv, int n, int a, int e, int lane, const TabRow& K,
+                                              unsigned short* X, float* D) {
     int w0, w1;
-    tab_chunk<W>(n, lane, w0, w1);
+    tab_chunk(W, n - 1 - a, lane, w0, w1);
     if (w0 >= w1) return;
-    const float Rl = K.R[TAB_NR - 1];
-    // window ends with R_j >= M_{n-1} - M_0 stay at 0 for every receiver
-    const float span = Mv[n - 1] - Mv[0];
-    int ja = 0;
-    while (ja < TAB_NB && K.R[ja] < span) ++ja;
-    const int jm = min(ja, TAB_NB - 1);  // moving middle window ends: j < jm
-    // closed form of the fixed middle ends j in [jm, nr-3]
-    const float sgf = K.SG[jm] - K.SG[TAB_NB - 1], sgrf = K.SGR[jm] - K.SGR[TAB_NB - 1];
+    w0 += a + 1;
+    w1 += a + 1;
+    const float Rl = K.R[TAB_NR - 1], m0 = Mv[a];
+    auto SV = [&](int w) { return T[wmap(fwd, w - 1, n)]; };
+    int ja = 0, js = 0;  // ends that have left a; ends past e + 1
     {   // the chunk's first receiver: binary searches (x_j <= x_{j-1})
         const float Pw = Pv[w0];
-        int hi = w0;
-        for (int j = 0; j < ja; j++) {
-            const float t = Pw - K.R[j];
-            int lo = 0, h = hi;
+        int hi = min(w0, e + 2);
+        for (; ja < TAB_NB && K.R[ja] < Pw - m0; ++ja) {
+            const float t = Pw - K.R[ja];
+            int lo = a, h = hi;
+#pragma unroll 1
             while (lo < h) {
                 const int mid = (lo + h) >> 1;
                 if (Mv[mid] >= t) h = mid;
                 else lo = mid + 1;
             }
-            X[32 * j] = lo;
+            X[32 * ja] = (unsigned short)lo;
             hi = lo;
         }
-        for (int j = ja; j < TAB_NB; j++) X[32 * j] = 0;
     }
+#pragma unroll 1
     for (int w = w0; w < w1; w++) {
         const float Pw = Pv[w];
-        // the last window end (radius R_{nr-2}) decides the last included source s
-        int xs = X[32 * (TAB_NB - 1)];
-        if (TAB_NB - 1 < ja) {
-            const float t = Pw - K.R[TAB_NB - 1];
-            while (xs < w && Mv[xs] < t) ++xs;
-            X[32 * (TAB_NB - 1)] = xs;
-        }
-        const bool back = xs >= 1 && Pw - Mv[xs - 1] <= Rl;
-        const int s = back ? xs - 1 : xs;
-        const int clip = s + 1;  // window ends are clipped below at s + 1
-        float tot = 0.f;
-        int seg = 0;
+        const int hi = min(w, e + 2);
+        for (; ja < TAB_NB && K.R[ja] < Pw - m0; ++ja) X[32 * ja] = (unsigned short)a;
+        float tot;
+        if (ja < TAB_NB) {
+            if (hi == e + 2)
+                while (js < ja && X[32 * js] == hi) ++js;
+            tot = K.B[js] * fmaf(Pw, SV(hi), -SVMv[hi]);
 #pragma unroll 1
-        for (int j = 0; j < jm; j++) {
-            const float t = Pw - K.R[j];
-            int xx = X[32 * j];
-            while (xx < w && Mv[xx] < t) ++xx;
-            X[32 * j] = xx;
+            for (int j = js; j < ja; j++) {
+                const float t = Pw - K.R[j];
+                int xx = X[32 * j];
+#pragma unroll 1
+                while (xx < hi && Mv[xx] < t) ++xx;
+                X[32 * j] = (unsigned short)xx;
+                tot = fmaf(K.G[j + 1], fmaf(t, SV(xx), -SVMv[xx]), tot);
+            }
+        } else {
+            // the last window end (radius R_{nr-2}) decides the last included source s
+            tot = 0.f;
+            int xs = X[32 * (TAB_NB - 1)];
+            {
+                const float t = Pw - K.R[TAB_NB - 1];
+#pragma unroll 1
+                while (xs < hi && Mv[xs] < t) ++xs;
+                X[32 * (TAB_NB - 1)] = (unsigned short)xs;
+            }
+            const bool back = xs > a && Pw - Mv[xs - 1] <= Rl;
+            const int s = back ? xs - 1 : xs;
+            const int clip = s + 1;  // window ends are clipped below at s + 1
+            int seg = 0;
+#pragma unroll 1
+            for (int j = 0; j < TAB_NB - 1; j++) {
+                const float t = Pw - K.R[j];
+                int xx = X[32 * j];
+#pragma unroll 1
+                while (xx < hi && Mv[xx] < t) ++xx;
+                X[32 * j] = (unsigned short)xx;
+                if (s < w) {
+                    seg += xx > s ? 1 : 0;
+                    const int lo = max(xx, clip);
+                    tot = fmaf(K.G[j + 1], fmaf(t, SV(lo), -SVMv[lo]), tot);
+                }
+            }
             if (s < w) {
-                seg += xx > s ? 1 : 0;
-                const int lo = max(xx, clip);
-                tot = fmaf(K.G[j + 1], fmaf(t, SVv[lo], -SVMv[lo]), tot);
+                tot = fmaf(K.B[0], fmaf(Pw, SV(hi), -SVMv[hi]), tot);  // top end
+                {   // the lowest window's lower end
+                    seg += xs > s ? 1 : 0;
+                    const int lo = max(xs, clip);
+                    const float coef = fmaf(K.B[TAB_NB - 1], Pw - K.Rm[TAB_NB - 1], K.Km[TAB_NB - 1]);
+                    tot = fmaf(K.B[TAB_NB - 1], SVMv[lo], fmaf(-coef, SV(lo), tot));
+                }
+                const int sg = back ? TAB_NR - 1 : seg;  // segment of c_s
+                tot = fmaf(SV(clip), fmaf(K.B[sg], (Pw - Mv[s]) - K.Rm[sg], K.Km[sg]), tot);
             }
         }
-        if (s < w) {
-            const float svc = SVv[clip], svmc = SVMv[clip];
-            tot += fmaf(svc, fmaf(Pw, sgf, -sgrf), -svmc * sgf);  // fixed middle ends
-            tot = fmaf(K.B[0], fmaf(Pw, SVv[w], -SVMv[w]), tot);   // top end w
-            {   // the lowest window's lower end
-                seg += xs > s ? 1 : 0;
-                const int lo = max(xs, clip);
-                const float coef = fmaf(K.B[TAB_NB - 1], Pw - K.Rm[TAB_NB - 1], K.Km[TAB_NB - 1]);
-                tot = fmaf(K.B[TAB_NB - 1], SVMv[lo], fmaf(-coef, SVv[lo], tot));
-            }
-            const int sg = back ? TAB_NR - 1 : seg;  // segment of c_s
-            tot = fmaf(svc, fmaf(K.B[sg], (Pw - Mv[s]) - K.Rm[sg], K.Km[sg]), tot);
-        }
-        const int i = wmap<FWD>(w, n);
-        if (FWD) D[i] = tot;
-        else D[i] = rho[i] >= 0.f ? __fdiv_rn(D[i] + tot, nphi) : 0.f;
+        D[wmap(fwd, w, n)] += tot;
     }
 }
 
-// P_w, Sg_w, SgP_w (w = 0..n, P_n = +inf: pointer stop) and M_w in walk order.
-template <bool FWD, int W = 32>
-__device__ __forceinline__ void tab_build_T(const float* rho, const float* g, int n, int lane, float delr, float* Pv,
-                                            float* Sgv, float* SgPv, float* Mv) {
+// P_w, Sg_w, SgP_w (w = a..n, P_n = +inf: pointer stop) and M_w in walk order,
+// the sums from sample a on.
+__device__ __forceinline__ void tab_build_T(bool fwd, int W, const float* rho, const float* g, int n, int a, int lane,
+                                            float delr, float* Pv, float* Sgv, float* SgPv, float* Mv) {
     int w0, w1;
-    tab_chunk<W>(n, lane, w0, w1);
+    tab_chunk(W, n - a, lane, w0, w1);
+    w0 += a;
+    w1 += a;
     float sd = 0.f, sg = 0.f, sgp = 0.f;
+#pragma unroll 1
     for (int w = w0; w < w1; w++) {
-        const int i = wmap<FWD>(w, n);
+        const int i = wmap(fwd, w, n);
         const float r = rho[i], gi = g[i];
         sgp = fmaf(gi, sd, sgp);
         sg += gi;
         sd += r >= 0.f ? delr * r : 0.f;
     }
-    float Pw = warp_excl_scan<W>(sd, lane);
-    float Sg = warp_excl_scan<W>(sg, lane);
-    float SgP = warp_excl_scan<W>(fmaf(Pw, sg, sgp), lane);
+    float Pw = warp_excl_scan(sd, lane, W);
+    float Sg = warp_excl_scan(sg, lane, W);
+    float SgP = warp_excl_scan(fmaf(Pw, sg, sgp), lane, W);
+#pragma unroll 1
     for (int w = w0; w < w1; w++) {
-        const int i = wmap<FWD>(w, n);
+        const int i = wmap(fwd, w, n);
         const float r = rho[i], gi = g[i];
         const float d = r >= 0.f ? delr * r : 0.f;
         Pv[w] = Pw;
@@ -1141,92 +1238,108 @@ __device__ __forceinline__ void tab_build_T(const float* rho, const float* g, in
     }
 }
 
-// Sources of one walk direction: W[k] = Phi_{b_k}(M_k), U[k] = Phi_{b_{k-1}}(M_k),
-// with the window ends y_j (Y[32 j], shared memory) clipped above at cap + 1
-// for each cap.
-template <bool FWD, int W = 32>
-__device__ __forceinline__ void tab_sources(const float* Pv, const float* Sgv, const float* SgPv, const float* Mv,
-                                            int n, int lane, const TabRow& K, int* Y, float* Wk, float* Uk) {
+// Sources [a, e] of one walk direction, and e + 1 for its U: Tbar_k = W_k -
+// U_{k+1} added to Tb, with W_k = Phi_{b_k}(M_k), U_k = Phi_{b_{k-1}}(M_k) and
+// the window ends y_j (Y[32 j], shared memory) clipped above at cap + 1 for each
+// cap.  A lane's sources are a contiguous chunk; its first U goes to the lane
+// before it (all lanes take part).
+__device__ __forceinline__ void tab_sources(bool fwd, int W, const float* Pv, const float* Sgv, const float* SgPv,
+                                            const float* Mv, int n, int a, int e, int lane, const TabRow& K,
+                                            unsigned short* Y, float* Tb) {
     int w0, w1;
-    tab_chunk<W>(n, lane, w0, w1);
-    if (w0 >= w1) return;
-    const float Rl = K.R[TAB_NR - 1], Rl2 = K.R[TAB_NR - 2];
-    // window ends with R_j >= P_{n-1} - M_0 stay at n for every source
-    const float span = Pv[n - 1] - Mv[0];
-    int ja = 0;
-    while (ja < TAB_NR && K.R[ja] < span) ++ja;
-    const int jm = min(ja, TAB_NR - 1);  // moving middle window ends: j < jm
-    auto lim_of = [&](int k) {
-        float l = Mv[k] + Rl;
-        if (k + 1 < n) l = fminf(l, Mv[k + 1] + Rl2);
-        return l;
-    };
-    // the first receiver i in [lo, n] with P_i > v (P_n = +inf)
-    auto ub = [&](float v, int lo) {
-        int h = n;
-        while (lo < h) {
-            const int mid = (lo + h) >> 1;
-            if (Pv[mid] > v) h = mid;
-            else lo = mid + 1;
-        }
-        return lo;
-    };
-    {   // the chunk's first source: binary searches (y_j >= y_{j-1})
-        const float m = Mv[w0];
-        int lo = min(w0 + 1, n);
-        for (int j = 0; j < ja; j++) {
-            lo = ub(m + K.R[j], lo);
-            Y[32 * j] = lo;
-        }
-        for (int j = ja; j < TAB_NR; j++) Y[32 * j] = n;
-    }
-    int ylim = ub(lim_of(w0), min(w0 + 1, n));
-    int capU = w0 >= 1 ? min(max(ub(lim_of(w0 - 1), w0) - 1, w0), n - 1) : w0;  // b_{w0-1}
-    for (int k = w0; k < w1; k++) {
-        const float m = Mv[k];
-        {
-            const float l = lim_of(k);
-            while (Pv[ylim] <= l) ++ylim;
-        }
-        const int capW = min(max(ylim - 1, k + 1), n - 1);  // b_k
-        float W = 0.f, U = 0.f;
-        if (k + 1 < n) {
-            const float sW = Sgv[capW + 1], sWp = SgPv[capW + 1], sU = Sgv[capU + 1], sUp = SgPv[capU + 1];
-            // bottom end k + 1: beta_0 (m Sg - SgP)
-            W = K.B[0] * fmaf(m, Sgv[k + 1], -SgPv[k + 1]);
-            U = W;
+    tab_chunk(W, min(e + 2, n) - a, lane, w0, w1);
+    w0 += a;
+    w1 += a;
+    float first = 0.f;  // U of the chunk's first source
+    if (w0 < w1) {
+        const float Rl = K.R[TAB_NR - 1], Rl2 = K.R[TAB_NR - 2];
+        // window ends with R_j >= P_{n-1} - M_{w0} stay at n for every source
+        const float span = Pv[n - 1] - Mv[w0];
+        int ja = 0;
+        while (ja < TAB_NR && K.R[ja] < span) ++ja;
+        int jm = min(ja, TAB_NR - 1);  // moving middle window ends: j < jm
+        auto lim_of = [&](int k) {
+            float l = Mv[k] + Rl;
+            if (k + 1 < n) l = fminf(l, Mv[k + 1] + Rl2);
+            return l;
+        };
+        // the first receiver i in [lo, n] with P_i > v (P_n = +inf)
+        auto ub = [&](float v, int lo) {
+            int h = n;
 #pragma unroll 1
-            for (int j = 0; j < jm; j++) {
-                const float t = m + K.R[j];
-                int yy = Y[32 * j];
-                while (Pv[yy] <= t) ++yy;
-                Y[32 * j] = yy;
-                const float a = Sgv[yy], ap = SgPv[yy];
-                const bool inW = yy <= capW + 1, inU = yy <= capU + 1;
-                W = fmaf(K.G[j + 1], fmaf(t, inW ? a : sW, -(inW ? ap : sWp)), W);
-                U = fmaf(K.G[j + 1], fmaf(t, inU ? a : sU, -(inU ? ap : sUp)), U);
+            while (lo < h) {
+                const int mid = (lo + h) >> 1;
+                if (Pv[mid] > v) h = mid;
+                else lo = mid + 1;
             }
-            // fixed middle ends j in [jm, nr-2] sit at n: past both caps
-            const float sg = K.SG[jm], sgr = K.SGR[jm];
-            W += fmaf(sW, fmaf(m, sg, sgr), -sWp * sg);
-            U += fmaf(sU, fmaf(m, sg, sgr), -sUp * sg);
-            {   // top end (radius R_{nr-1}): coef'_{nr-1} Sg + beta_{nr-1} SgP
-                const int j = TAB_NR - 1;
-                int yy = Y[32 * j];
-                if (j < ja) {
-                    while (Pv[yy] <= m + K.R[j]) ++yy;
-                    Y[32 * j] = yy;
-                }
-                const float coef = K.Km[j] - K.B[j] * (m + K.Rm[j]);
-                const bool inW = yy <= capW + 1, inU = yy <= capU + 1;
-                W = fmaf(coef, inW ? Sgv[yy] : sW, fmaf(K.B[j], inW ? SgPv[yy] : sWp, W));
-                U = fmaf(coef, inU ? Sgv[yy] : sU, fmaf(K.B[j], inU ? SgPv[yy] : sUp, U));
+            return lo;
+        };
+        {   // the chunk's first source: binary searches (y_j >= y_{j-1})
+            const float m = Mv[w0];
+            int lo = min(w0 + 1, n);
+            for (int j = 0; j < ja; j++) {
+                lo = ub(m + K.R[j], lo);
+                Y[32 * j] = (unsigned short)lo;
             }
+            for (int j = ja; j < TAB_NR; j++) Y[32 * j] = (unsigned short)n;
         }
-        Wk[k] = W;
-        Uk[k] = U;
-        capU = capW;
+        int ylim = ub(lim_of(w0), min(w0 + 1, n));
+        int capU = w0 > a ? min(max(ub(lim_of(w0 - 1), w0) - 1, w0), n - 1) : w0;  // b_{w0-1}
+#pragma unroll 1
+        for (int k = w0; k < w1; k++) {
+            const float m = Mv[k];
+            {
+                const float l = lim_of(k);
+#pragma unroll 1
+                while (Pv[ylim] <= l) ++ylim;
+            }
+            const int capW = min(max(ylim - 1, k + 1), n - 1);  // b_k
+            float wk = 0.f, uk = 0.f;
+            if (k + 1 < n) {
+                const float sW = Sgv[capW + 1], sWp = SgPv[capW + 1], sU = Sgv[capU + 1], sUp = SgPv[capU + 1];
+                while (jm > 0 && Y[32 * (jm - 1)] == n) --jm;
+                // bottom end k + 1: beta_0 (m Sg - SgP)
+                wk = K.B[0] * fmaf(m, Sgv[k + 1], -SgPv[k + 1]);
+                uk = wk;
+#pragma unroll 1
+                for (int j = 0; j < jm; j++) {
+                    const float t = m + K.R[j];
+                    int yy = Y[32 * j];
+#pragma unroll 1
+                    while (Pv[yy] <= t) ++yy;
+                    Y[32 * j] = (unsigned short)yy;
+                    const float a = Sgv[yy], ap = SgPv[yy];
+                    const bool inW = yy <= capW + 1, inU = yy <= capU + 1;
+                    wk = fmaf(K.G[j + 1], fmaf(t, inW ? a : sW, -(inW ? ap : sWp)), wk);
+                    uk = fmaf(K.G[j + 1], fmaf(t, inU ? a : sU, -(inU ? ap : sUp)), uk);
+                }
+                // fixed middle ends j in [jm, nr-2] sit at n: past both caps
+                const float sg = K.SG[jm], sgr = K.SGR[jm];
+                wk += fmaf(sW, fmaf(m, sg, sgr), -sWp * sg);
+                uk += fmaf(sU, fmaf(m, sg, sgr), -sUp * sg);
+                {   // top end (radius R_{nr-1}): coef'_{nr-1} Sg + beta_{nr-1} SgP
+                    const int j = TAB_NR - 1;
+                    int yy = Y[32 * j];
+                    if (j < ja) {
+#pragma unroll 1
+                        while (Pv[yy] <= m + K.R[j]) ++yy;
+                        Y[32 * j] = (unsigned short)yy;
+                    }
+                    const float coef = K.Km[j] - K.B[j] * (m + K.Rm[j]);
+                    const bool inW = yy <= capW + 1, inU = yy <= capU + 1;
+                    wk = fmaf(coef, inW ? Sgv[yy] : sW, fmaf(K.B[j], inW ? SgPv[yy] : sWp, wk));
+                    uk = fmaf(coef, inU ? Sgv[yy] : sU, fmaf(K.B[j], inU ? SgPv[yy] : sUp, uk));
+                }
+            }
+            if (k == w0) first = uk;
+            else Tb[wmap(fwd, k - 1, n)] -= uk;
+            if (k <= e) Tb[wmap(fwd, k, n)] += wk;
+            capU = capW;
+        }
     }
+    __syncwarp();
+    const float next = __shfl_down_sync(FULL, first, 1, W);
+    if (w0 < w1 && w1 <= min(e + 1, n - 1)) Tb[wmap(fwd, w1 - 1, n)] -= next;
 }
 
 // Exact-table cone kernel (mode EE_KERNEL_TABLE, nr = 24): REV resample of a
@@ -1234,72 +1347,96 @@ __device__ __forceinline__ void tab_sources(const float* Pv, const float* Sgv, c
 constexpr int TAB_WARPS = 4;
 
 __host__ __device__ constexpr int tab_lp(int maxL) { return ((maxL + 3) & ~3) + 4; }
-__host__ __device__ constexpr int tab_fwd_stride(int maxL) { return 7 * tab_lp(maxL) + 32 * TAB_NB; }
-__host__ __device__ constexpr int tab_adj_stride(int maxL) { return 9 * tab_lp(maxL) + 32 * TAB_NR; }
+__host__ __device__ constexpr int tab_fwd_stride(int maxL) { return 6 * tab_lp(maxL) + 16 * TAB_NB; }
+__host__ __device__ constexpr int tab_adj_stride(int maxL) { return 7 * tab_lp(maxL) + 16 * TAB_NR; }
+
+// A line of the table kernels: its samples [i0, i0 + n), of which [a, e]
+// (from i0) can have TERMA; line = -1: nothing to write, n = 0: zeros only.
+struct TabLine {
+    int line, i0, n, a, e, tY, tZ;
+    LineFrame F;
+};
+
+// Kept line `line`; -1 where its lit forms are below `least`.
+__device__ __forceinline__ TabLine tab_line(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
+                                            const EeRayGeom& R, float least, int line) {
+    TabLine t;
+    t.line = -1;
+    t.i0 = t.n = t.a = t.tY = t.tZ = 0;
+    t.e = -1;
+    if (line < 0) return t;
+    kept_line(R, line, t.tY, t.tZ);
+    if (lit_form(R, (float)t.tY, (float)t.tZ) < least) return t;
+    t.line = line;
+    const LaneSpan s = lane_span(P, S, G, R, t.tY, t.tZ, t.F);
+    if (s.q1 < s.q0) return t;
+    t.i0 = s.i0;
+    t.n = s.i1 - s.i0 + 1;
+    t.a = max(4 * s.q0, s.i0) - s.i0;
+    t.e = min(4 * s.q1 + 3, s.i1) - s.i0;
+    return t;
+}
 
 // One line of k_cone_tab on the W lanes of its group (`lane` counts within
 // the group; W = 32: the whole warp, W = 16: half of it), with the group's
-// arrays at `arr`.  line < 0 or n <= 0: nothing to write, but the group still
-// takes part in the scans, which all 32 lanes execute.
-template <int W>
-__device__ __forceinline__ void tab_fwd_line(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
+// arrays at `arr`.  A line without samples still takes part in the scans, which
+// all 32 lanes execute.
+__device__ __forceinline__ void tab_fwd_line(int W, const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
                                              const EeRayGeom& R, const float* __restrict__ terma_b,
-                                             float* __restrict__ rev_beam, int line, int i0, int n, int lane,
-                                             float* arr, int Lp, const float* tab, int* X) {
+                                             float* __restrict__ rev_beam, const TabLine& L, int lane, float* arr,
+                                             int Lp, const float* tab, unsigned short* X) {
     float* Mv = arr;
     float* Pv = Mv + Lp;
-    float* SVv = Pv + Lp;
-    float* SVMv = SVv + Lp;
+    float* SVMv = Pv + Lp;
     float* rho = SVMv + Lp;
-    float* T = rho + Lp;
-    float* D = T + Lp;
+    float* D = rho + Lp;
+    float* T = D + Lp + 1;  // T[-1] = T[n] = 0
     float* out = nullptr;
-    int nn = 0;
-    if (line >= 0) {
-        const int L = R.rev[0];
-        int tY, tZ;
-        kept_line(R, line, tY, tZ);
+    const int n = L.n;
+    if (L.line >= 0) {
         const Brick Bv = rev_store(R);
-        out = rev_beam + R.offset + rev_line(Bv, tY, tZ);
+        out = rev_beam + R.offset + rev_line(Bv, L.tY, L.tZ);
         int z0, z1;
-        line_read_span(G, R, tY, tZ, L, z0, z1);
-        zero_outside_segment(out, Bv, z0, z1, i0, n, lane, W);
-        if (n > 0) {
-            gather_line(P, S, G, R, terma_b, tY, tZ, i0, n, lane, rho, T, W);
-            nn = n;
-        }
+        line_read_span(G, R, L.tY, L.tZ, R.rev[0], z0, z1);
+        zero_outside_segment(out, Bv, z0, z1, L.i0, n, lane, W);
     }
+    const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
+    const Brick Bt = brick_of(S.tn);
+    for (int k = lane; k < n; k += W) {
+        const f3 g = sample_point(L.F, L.i0 + k);
+        rho[k] = rho_at(P, g);
+        T[k] = k >= L.a && k <= L.e ? tri_brick(terma_b, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z) : 0.f;
+        D[k] = 0.f;
+    }
+    if (lane == 0) T[-1] = T[n] = 0.f;
     __syncwarp();
+#pragma unroll 1
+    for (int dir = 0; dir < 2; dir++) {
+        const bool fwd = dir == 0;
+        const int a = fwd ? L.a : max(0, n - 1 - L.e), e = fwd ? L.e : n - 1 - L.a;  // the sources in walk order
+        tab_build(fwd, W, rho, T, n, a, lane, P.lng, Mv, Pv, SVMv);
+        __syncwarp();
+        tab_receivers(fwd, W, Mv, Pv, T, SVMv, n, a, e, lane, tab_row(tab, fwd), X, D);
+        __syncwarp();
+    }
     const float nphi = (float)P.nphi;
-    tab_build<true, W>(rho, T, nn, lane, P.lng, Mv, Pv, SVv, SVMv);
-    __syncwarp();
-    tab_receivers<true, W>(Mv, Pv, SVv, SVMv, rho, nn, lane, tab_row(tab, true), X, D, nphi);
-    __syncwarp();
-    tab_build<false, W>(rho, T, nn, lane, P.lng, Mv, Pv, SVv, SVMv);
-    __syncwarp();
-    tab_receivers<false, W>(Mv, Pv, SVv, SVMv, rho, nn, lane, tab_row(tab, false), X, D, nphi);
-    __syncwarp();
-    for (int k = lane; k < nn; k += W) out[bk_x(i0 + k)] = D[k];
-}
-
-// The segment of kept line `line`; line = -1 (n = 0) where its lit forms are
-// below `least`.
-__device__ __forceinline__ void tab_line(const EeParams& P, const EeBeamGeom& G, const EeRayGeom& R, float least,
-                                         int& line, int& i0, int& n) {
-    i0 = n = 0;
-    if (line < 0) return;
-    int tY, tZ;
-    kept_line(R, line, tY, tZ);
-    if (lit_form(R, (float)tY, (float)tZ) < least) line = -1;
-    else line_segment(P, G, R, tY, tZ, R.rev[0], i0, n);
+    for (int k = lane; k < n; k += W) out[bk_x(L.i0 + k)] = rho[k] >= 0.f ? __fdiv_rn(D[k], nphi) : 0.f;
 }
 
 // A warp takes two neighbouring lines.  When both fit half of its arrays
-// (n below Lp / 2 - 1), each half-warp runs one of them, 16 lanes per line;
+// (n below Lp / 2 - 1, or - 2), each half-warp runs one of them, 16 lanes per line;
 // else the whole warp runs one after the other.  A lane's first receiver costs a
 // binary search per window end, so a lane that runs one chunk of a line
 // instead of two shorter chunks of two lines saves one set of searches, and
 // short lines keep more lanes busy.
+//
+// Bound by instruction issue and fixed latencies (40 % of the issue slots at 20
+// to 24 warps per SM, which the shared arrays allow).  Two 24 x 24 beams on 200 x
+// 200 x 160: 6.8 ms with every radius of the line's length at every receiver,
+// 3.3 with the ends inside the sources' range only, TERMA sampled there only and
+// one copy of the code for both directions and group widths (129 -> 43 KB), 2.45
+// with 16-bit window ends and T in place of an SV array (4 -> 6 blocks per SM);
+// the adjoint likewise 5.4, 3.0, 2.6 ms.
 __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_tab(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                              const EeBeamGeom* __restrict__ geoms,
                                                              const float* __restrict__ terma, float* __restrict__ rev,
@@ -1318,38 +1455,33 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_tab(EeParams P, const E
     const EeRayGeom& R = G.ray[ray];
     int la = 2 * (blockIdx.x * TAB_WARPS + warp);
     if (la >= R.nlines) return;
-    int lb = la + 1 < R.nlines ? la + 1 : -1;
-    int i0a, na, i0b = 0, nb = 0;
-    tab_line(P, G, R, EE_LIT_READ, la, i0a, na);
-    tab_line(P, G, R, EE_LIT_READ, lb, i0b, nb);
-    if (la < 0 && lb < 0) return;
-    float* arr = sm + (size_t)warp * tab_fwd_stride(maxL);
-    int* X = reinterpret_cast<int*>(arr + 7 * Lp) + lane;
     const EeBeamSpec& S = specs[b];
+    const TabLine A = tab_line(P, S, G, R, EE_LIT_READ, la),
+                  B = tab_line(P, S, G, R, EE_LIT_READ, la + 1 < R.nlines ? la + 1 : -1);
+    if (A.line < 0 && B.line < 0) return;
+    float* arr = sm + (size_t)warp * tab_fwd_stride(maxL);
+    unsigned short* X = reinterpret_cast<unsigned short*>(arr + 6 * Lp) + lane;
     const float* terma_b = terma + S.t_off;
     float* rev_beam = rev + G.arena_off;
     // the second half-warp's arrays start one cell past the middle: an odd
     // offset puts the two halves' strided accesses on different banks
     const int half = Lp >> 1;
-    if (max(na, nb) < half - 1) {
-        const int sub = lane >> 4;
-        tab_fwd_line<16>(P, S, G, R, terma_b, rev_beam, sub ? lb : la, sub ? i0b : i0a, sub ? nb : na, lane & 15,
-                         arr + sub * (half + 1), Lp, tab, X);
-    } else {
-        if (la >= 0) tab_fwd_line<32>(P, S, G, R, terma_b, rev_beam, la, i0a, na, lane, arr, Lp, tab, X);
-        if (lb >= 0) {
-            __syncwarp();
-            tab_fwd_line<32>(P, S, G, R, terma_b, rev_beam, lb, i0b, nb, lane, arr, Lp, tab, X);
-        }
+    const bool both = max(A.n, B.n) < half - 2;  // T takes n + 2 cells
+    const int W = both ? 16 : 32, sub = both ? lane >> 4 : 0;
+#pragma unroll 1
+    for (int k = 0; k < (both ? 1 : 2); k++) {
+        const TabLine& L = (both ? sub : k) ? B : A;
+        if (!both && L.line < 0) continue;
+        tab_fwd_line(W, P, S, G, R, terma_b, rev_beam, L, lane & (W - 1), arr + sub * (half + 1), Lp, tab, X);
+        __syncwarp();
     }
 }
 
 // One line of k_cone_T_tab on the W lanes of its group (as tab_fwd_line).
-template <int W>
-__device__ __forceinline__ void tab_adj_line(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
+__device__ __forceinline__ void tab_adj_line(int W, const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
                                              const EeRayGeom& R, const float* __restrict__ grad_beam,
-                                             float* __restrict__ terma_grad, int line, int i0, int n, int lane,
-                                             float* arr, int Lp, const float* tab, int* Y) {
+                                             float* __restrict__ terma_grad, const TabLine& L, int lane, float* arr,
+                                             int Lp, const float* tab, unsigned short* Y) {
     float* Pv = arr;
     float* Sgv = Pv + Lp;
     float* SgPv = Sgv + Lp;
@@ -1357,51 +1489,36 @@ __device__ __forceinline__ void tab_adj_line(const EeParams& P, const EeBeamSpec
     float* rho = Mv + Lp;
     float* g = rho + Lp;
     float* Tb = g + Lp;
-    float* Wk = Tb + Lp;
-    float* Uk = Wk + Lp;
-    int nn = 0, tY = 0, tZ = 0;
-    if (line >= 0 && n > 0) {
-        kept_line(R, line, tY, tZ);
-        gather_line(P, S, G, R, nullptr, tY, tZ, i0, n, lane, rho, nullptr, W);
-        nn = n;
-    }
-    __syncwarp();
-    if (nn > 0) {
-        const Brick Bv = rev_store(R);
-        const float* gin = grad_beam + R.offset + rev_line(Bv, tY, tZ);
+    const int n = L.n;
+    {
+        const float* gin = grad_beam + R.offset + rev_line(rev_store(R), L.tY, L.tZ);
         const float inv_nphi = 1.f / (float)P.nphi;
-        for (int k = lane; k < nn; k += W) {
-            g[k] = rho[k] >= 0.f ? gin[bk_x(i0 + k)] * inv_nphi : 0.f;
+        for (int k = lane; k < n; k += W) {
+            const float r = rho_at(P, sample_point(L.F, L.i0 + k));
+            rho[k] = r;
+            g[k] = r >= 0.f ? gin[bk_x(L.i0 + k)] * inv_nphi : 0.f;
             Tb[k] = 0.f;
         }
     }
     __syncwarp();
 #pragma unroll 1
     for (int dir = 0; dir < 2; dir++) {
-        if (dir == 0) tab_build_T<true, W>(rho, g, nn, lane, P.lng, Pv, Sgv, SgPv, Mv);
-        else tab_build_T<false, W>(rho, g, nn, lane, P.lng, Pv, Sgv, SgPv, Mv);
+        const bool fwd = dir == 0;
+        const int a = fwd ? L.a : max(0, n - 1 - L.e), e = fwd ? L.e : n - 1 - L.a;  // the sources in walk order
+        tab_build_T(fwd, W, rho, g, n, a, lane, P.lng, Pv, Sgv, SgPv, Mv);
         __syncwarp();
-        if (dir == 0) tab_sources<true, W>(Pv, Sgv, SgPv, Mv, nn, lane, tab_row(tab, true), Y, Wk, Uk);
-        else tab_sources<false, W>(Pv, Sgv, SgPv, Mv, nn, lane, tab_row(tab, false), Y, Wk, Uk);
-        __syncwarp();
-        for (int w = lane; w < nn; w += W) {
-            const float v = Wk[w] - (w + 1 < nn ? Uk[w + 1] : 0.f);
-            Tb[dir == 0 ? w : nn - 1 - w] += v;
-        }
+        tab_sources(fwd, W, Pv, Sgv, SgPv, Mv, n, a, e, lane, tab_row(tab, fwd), Y, Tb);
         __syncwarp();
     }
-    if (nn > 0) {
-        // transpose of the REV TERMA resample
-        const f3 gl = ld3(R.G0) + ld3(R.Gy) * (float)tY + ld3(R.Gz) * (float)tZ;
-        const f3 gx = ld3(R.Gx);
-        float* tg = terma_grad + S.t_off;
-        for (int k = lane; k < nn; k += W) {
-            const float v = Tb[k];
-            if (rho[k] < 0.f || v == 0.f) continue;
-            const f3 gp = gl + gx * (float)(i0 + k);
-            tri_brick_scatter_edge(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
-                              gp.z - (float)S.t0[2], v);
-        }
+    // transpose of the REV TERMA resample
+    float* tg = terma_grad + S.t_off;
+    const Brick Bt = brick_of(S.tn);
+    const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
+    for (int k = L.a + lane; k <= L.e; k += W) {
+        const float v = Tb[k];
+        if (rho[k] < 0.f || v == 0.f) continue;
+        const f3 p = sample_point(L.F, L.i0 + k);
+        tri_brick_scatter_edge(tg, Bt, p.x - t0.x, p.y - t0.y, p.z - t0.z, v);
     }
 }
 
@@ -1425,26 +1542,21 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_T_tab(EeParams P, const
     const EeRayGeom& R = G.ray[ray];
     int la = 2 * (blockIdx.x * TAB_WARPS + warp);
     if (la >= R.nlines) return;
-    int lb = la + 1 < R.nlines ? la + 1 : -1;
-    int i0a, na, i0b = 0, nb = 0;
-    tab_line(P, G, R, 0.f, la, i0a, na);
-    tab_line(P, G, R, 0.f, lb, i0b, nb);
-    if (la < 0 && lb < 0) return;
-    float* arr = sm + (size_t)warp * tab_adj_stride(maxL);
-    int* Y = reinterpret_cast<int*>(arr + 9 * Lp) + lane;
     const EeBeamSpec& S = specs[b];
+    const TabLine A = tab_line(P, S, G, R, 0.f, la), B = tab_line(P, S, G, R, 0.f, la + 1 < R.nlines ? la + 1 : -1);
+    if (A.n == 0 && B.n == 0) return;
+    float* arr = sm + (size_t)warp * tab_adj_stride(maxL);
+    unsigned short* Y = reinterpret_cast<unsigned short*>(arr + 7 * Lp) + lane;
     const float* grad_beam = rev_grad + G.arena_off;
     const int half = Lp >> 1;  // second half-warp's arrays at an odd offset, as k_cone_tab
-    if (max(na, nb) < half - 1) {
-        const int sub = lane >> 4;
-        tab_adj_line<16>(P, S, G, R, grad_beam, terma_grad, sub ? lb : la, sub ? i0b : i0a, sub ? nb : na,
-                         lane & 15, arr + sub * (half + 1), Lp, tab, Y);
-    } else {
-        if (la >= 0) tab_adj_line<32>(P, S, G, R, grad_beam, terma_grad, la, i0a, na, lane, arr, Lp, tab, Y);
-        if (lb >= 0) {
-            __syncwarp();
-            tab_adj_line<32>(P, S, G, R, grad_beam, terma_grad, lb, i0b, nb, lane, arr, Lp, tab, Y);
-        }
+    const bool both = max(A.n, B.n) < half - 1;
+    const int W = both ? 16 : 32, sub = both ? lane >> 4 : 0;
+#pragma unroll 1
+    for (int k = 0; k < (both ? 1 : 2); k++) {
+        const TabLine& L = (both ? sub : k) ? B : A;
+        if (!both && L.n == 0) continue;
+        tab_adj_line(W, P, S, G, R, grad_beam, terma_grad, L, lane & (W - 1), arr + sub * (half + 1), Lp, tab, Y);
+        __syncwarp();
     }
 }
 
@@ -1453,78 +1565,6 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_T_tab(EeParams P, const
 // own adjacent lines, so their segments and gathers stay close): it computes
 // its segment analytically and runs the recurrence sequentially, without
 // shuffles or shared memory.  Same operator as line_scan.
-struct LineFrame {
-    f3 gl, gx;  // patient voxel index of sample 0, and its step per sample
-};
-
-__device__ __forceinline__ f3 sample_point(const LineFrame& F, int i) { return F.gl + F.gx * (float)i; }
-
-__device__ __forceinline__ float rho_at(const EeParams& P, f3 g) {
-    return tex3D<float>(P.dens_tex, g.x + 0.5f, g.y + 0.5f, g.z + 0.5f);
-}
-
-// What a lane needs of its line.  [i0, i1]: the samples inside the BEV crop
-// box and the calc bbox by the reference's own tests (device.cu:51-70).  Every
-// test is a comparison of an affine function of i, which stays monotone in
-// FP32, so the samples that pass are one interval: the analytic segment
-// trimmed at its ends by the tests themselves, and no sample in between needs
-// them again.  [q0, q1]: the quads of [i0, i1] that hold the samples whose
-// TERMA corners can lie in the field (field_forms); q1 < q0: no such sample,
-// so neither dose nor TERMA gradient.
-struct LaneSpan {
-    int i0, i1, q0, q1;
-};
-
-__device__ __forceinline__ LaneSpan lane_span(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
-                                              const EeRayGeom& R, int tY, int tZ, LineFrame& F) {
-    const float fy = (float)tY, fz = (float)tZ;
-    F.gl = ld3(R.G0) + ld3(R.Gy) * fy + ld3(R.Gz) * fz;
-    F.gx = ld3(R.Gx);
-    LaneSpan s{0, -1, 0, -1};
-    if (lit_form(R, fy, fz) < 0.f) return s;
-    int n;
-    line_segment(P, G, R, tY, tZ, R.rev[0], s.i0, n);
-    s.i1 = s.i0 + n - 1;
-    if (n <= 0) return s;
-    // field span: the four sides, raised by more than their rounding, cut the
-    // line to one interval.  The forms hold in front of the source; beamlet_of
-    // takes |depth|, so a segment that does not stay in front of it is not
-    // restricted
-    float lo = -1e9f, hi = 1e9f;
-    const float pr = fmaf(R.front[2], fy, fmaf(R.front[3], fz, R.front[1]));
-    const bool front = fminf(fmaf(R.front[0], (float)s.i0, pr), fmaf(R.front[0], (float)s.i1, pr)) > 1e-2f * S.isodist;
-    if (front) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float al = R.side[k][0], be = fmaf(R.side[k][2], fy, fmaf(R.side[k][3], fz, R.side[k][1]));
-            if (fabsf(al) < 1e-20f) {
-                if (be < 0.f) { lo = 1e9f; hi = -1e9f; }
-            } else {
-                const float t = fminf(fmaxf(__fdividef(-be, al), -1e9f), 1e9f);
-                if (al > 0.f) lo = fmaxf(lo, t);
-                else hi = fminf(hi, t);
-            }
-        }
-    }
-    const int f0 = max(s.i0, (int)ceilf(lo - 0.01f)), f1 = min(s.i1, (int)floorf(hi + 0.01f));
-    if (f0 > f1) return s;
-    const f3 bl = ld3(R.B0) + ld3(R.By) * fy + ld3(R.Bz) * fz, bx = ld3(R.Bx);
-    auto valid = [&](int i) {
-        const f3 bev = bl + bx * (float)i, g = sample_point(F, i);
-        return !(bev.x < 0.f || bev.y < 0.f || bev.z < 0.f || bev.x >= (float)G.bev[0] || bev.y >= (float)G.bev[1] ||
-                 bev.z >= (float)G.bev[2] || g.x < (float)P.bb0[0] || g.x >= (float)(P.bb0[0] + P.bbs[0]) ||
-                 g.y < (float)P.bb0[1] || g.y >= (float)(P.bb0[1] + P.bbs[1]) || g.z < (float)P.bb0[2] ||
-                 g.z >= (float)(P.bb0[2] + P.bbs[2]));
-    };
-#pragma unroll 1
-    while (s.i0 <= s.i1 && !valid(s.i0)) s.i0++;
-#pragma unroll 1
-    while (s.i1 > s.i0 && !valid(s.i1)) s.i1--;
-    if (max(f0, s.i0) > min(f1, s.i1)) return s;
-    s.q0 = max(f0, s.i0) >> 2;
-    s.q1 = min(f1, s.i1) >> 2;
-    return s;
-}
 
 // Lane slot -> REV line for the one-lane-per-line kernels: the lanes of a
 // warp own an 8 (tY) x 4 (tZ) tile of lines, so at every sample index the
