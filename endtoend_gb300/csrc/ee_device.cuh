@@ -336,6 +336,10 @@ __device__ __forceinline__ void tri_border_scatter(float* v, int nx, int ny, int
 // the border-mode trilinear density at (pos-start)/voxel, segments shorter
 // than 1e-3 cm skipped, 5000-iteration cap.  (Nine comparisons per crossing in
 // place of the reference's validity logic: k_terma 10.0 -> 9.4 ms on 96 beams.)
+// A sample is added while the next one's fetch is under way; the order of the
+// sum stays.  Bound by the texture unit's data stage, 72 % busy on average so and
+// 66 % with one fetch in flight: 96 beams 8.07 -> 7.81 ms, 4 beams with 27
+// centres per voxel 6.29 -> 5.80.
 __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
     const f3 start = mk(P.start[0], P.start[1], P.start[2]);
     const f3 voxel = mk(P.voxel[0], P.voxel[1], P.voxel[2]);
@@ -359,7 +363,9 @@ __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
         // The parameters start at a_min >= 0 and grow, and an invalid one
         // (>= 1) is above every valid one, so "below 1 and not above the other
         // two" is the same test.
-        while (alpha < a_max && ++iter < 5000) {
+        // the next segment's length (0 below the cut) and sample position
+        auto segment = [&](float& len, f3& at) {
+            if (!(alpha < a_max && ++iter < 5000)) return false;
             const bool vy = ay < 1.f, vz = az < 1.f;
             const bool cx = ax < 1.f && ax <= ay && ax <= az;
             if (cx) { next = ax; ax += stx; }
@@ -367,17 +373,31 @@ __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
             if (cy) { next = ay; ay += sty; }
             const bool cz = vz && az <= ax && az <= ay;
             if (cz) { next = az; az += stz; }
-            if (!(cx || cy || cz)) break;  // no axis valid
+            if (!(cx || cy || cz)) return false;  // no axis valid
             const float isect = fabsf(d12 * (next - alpha));
-            if (isect >= 0.001f) {
-                const float mid = (next + alpha) * 0.5f;
-                const float fx = (src.x + mid * diff.x - start.x) * ivx;
-                const float fy = (src.y + mid * diff.y - start.y) * ivy;
-                const float fz = (src.z + mid * diff.z - start.z) * ivz;
-                rpl += isect * tex3D<float>(P.dens_tex, fx, fy, fz);
-            }
+            len = isect >= 0.001f ? isect : 0.f;
+            const float mid = (next + alpha) * 0.5f;
+            at = mk((src.x + mid * diff.x - start.x) * ivx, (src.y + mid * diff.y - start.y) * ivy,
+                    (src.z + mid * diff.z - start.z) * ivz);
             alpha = next;
+            return true;
+        };
+        float l0 = 0.f, r0 = 0.f, l1 = 0.f, r1 = 0.f;
+        f3 at;
+        for (;;) {
+            float len;
+            if (!segment(len, at)) break;
+            l0 = len;
+            r0 = tex3D<float>(P.dens_tex, at.x, at.y, at.z);
+            rpl = fmaf(l1, r1, rpl);
+            l1 = 0.f;
+            if (!segment(len, at)) break;
+            l1 = len;
+            r1 = tex3D<float>(P.dens_tex, at.x, at.y, at.z);
+            rpl = fmaf(l0, r0, rpl);
+            l0 = 0.f;
         }
+        rpl = fmaf(l1, r1, fmaf(l0, r0, rpl));
         if (iter >= 5000) iter_cap = true;
     }
     return rpl;
