@@ -2280,6 +2280,14 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, 5) k_gather(EeParams P, const 
 // 256 * 2^22 = 2^30.  The rounding error per contribution is at most
 // 2^-22 max|g| of the tile, about FP32 rounding at the tile's largest
 // gradient; the flush converts each sum back with the exact factor 1 / s.
+//
+// Bound by instruction issue (three quarters of the slots) and the conversion
+// unit, which takes 8 cycles per warp: what is the same for a tile's voxels is
+// worked out once per tile and cone, the cells come from roundings at unit
+// spacing and the quads' places from multiplications by 2^-20 reciprocals (four
+// conversions per quad and three per voxel less: six beams 0.721 -> 0.642 ms,
+// 12 beams 1.65 -> 1.48).  Five blocks per SM at 48 registers; four at 56 are
+// 2 % slower on those and 5 % faster on one beam.
 constexpr int GT_TX = 8, GT_TY = 8, GT_TZ = 4;
 // floats per footprint buffer: an 8x8x4 tile spans at most |(7,7,3)| + 2 = 13
 // REV cells per axis when the REV spacing equals the voxel size (16 along i
@@ -2290,21 +2298,22 @@ constexpr int GT_TX = 8, GT_TY = 8, GT_TZ = 4;
 constexpr int GT_BUF = 4096;
 constexpr int GT_SMEM = 2 * GT_BUF;
 
-__global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, const EeBeamSpec* __restrict__ specs,
+__global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                                    const EeBeamGeom* __restrict__ geoms,
                                                                    const float* __restrict__ dose_grad,
                                                                    float* __restrict__ rev_grad) {
     extern __shared__ int acc_all[];  // two fixed-point footprint boxes
-    // per cone: {l0 | n0 << 16, l1 | n1 << 16, l2 | n2 << 16, s0} (box origin
-    // and extent along i, tY and tZ, the box's row stride along i; all below
-    // 2^16) and {v0, v1, v2} (rev - l: the box cells inside the REV array),
-    // read with two vector loads before the scatter, and {sy, sz, offset lo,
-    // offset hi} (the REV gradient's brick strides and the cone's arena
-    // offset), read with one before the flush
-    // and {k0, k1, k2 | k each, lo | hi << 16}: the box cells inside the kept
-    // part, which the flush sends
-    __shared__ int4 s_p[EE_MAX_RAYS][4];
+    // per cone, the box of its footprint (origin l, extent n over i, tY and tZ):
+    // [0] {l0 | n0 << 16, l1 | n1 << 16, l2 | n2 << 16, row stride s0} until the
+    // second step below, then {s0, slab stride, l1 | l2 << 16, 16 l0}; [1] the
+    // REV gradient's {sy, sz, offset lo, offset hi}; [2] {rev[0], rev[1], rev[2]
+    // as floats, the constant of a voxel's cell}; [3] {k0, k1, k2 | k each, lo |
+    // hi << 16} (the box cells inside the kept part, which the flush sends), rows
+    // per slab; [4] {quads per row, its and the slab's rows' reciprocals in
+    // 2^-20, nquad | 1 << 16 where the box lies in the kept part}
+    __shared__ int4 s_p[EE_MAX_RAYS][5];
     __shared__ float4 s_A[EE_MAX_RAYS][3];
+    __shared__ int s_list[EE_MAX_RAYS], s_n;  // cones with a box
     const int b = blockIdx.z;
     const EeBeamGeom& G = geoms[b];
     if (G.status != 0 || (int)blockIdx.x >= G.tiles) return;
@@ -2373,7 +2382,7 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
             if (dark) w = 0;
         }
         int* sp = reinterpret_cast<int*>(s_p[r]);
-        sp[8 + (a == 1 ? 0 : (a == 2 ? 1 : 2))] = dim - (a == 1 ? (l & ~3) : l);
+        sp[8 + (a == 1 ? 0 : (a == 2 ? 1 : 2))] = __float_as_int((float)dim);
         if (a == 1) {
             int s0 = 0;
             if (w > 0) {
@@ -2403,6 +2412,30 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
         // (the forward gather forms q in the same order)
         s_A[r][a] = make_float4(Ar[0], Ar[1], Ar[2], -R.q0[a]);
     }
+    if (t == 0) s_n = 0;
+    __syncthreads();
+    for (int r = t; r < P.nrays; r += blockDim.x) {
+        int4* const sp = s_p[r];
+        const int4 p0 = sp[0], p3 = sp[3];
+        const int n0 = p0.x >> 16, n1 = p0.y >> 16, n2 = p0.z >> 16, s0 = p0.w;
+        if (n0 <= 0 || n1 <= 0 || n2 <= 0) continue;
+        // box cell (k0, k1, k2) over (i, tY, tZ) at k0 + s0 * (k1 + n1p * k2); rows
+        // per slab: odd, so that the slab stride s0 * n1p is 4 x odd (mod 32) and
+        // the slabs of adjacent voxels spread over the banks too; the padding rows
+        // (k1 >= n1) are never scattered to
+        const int n1p = n1 | 1, nbox = s0 * n1p * n2;
+        s_list[atomicAdd(&s_n, 1)] = nbox <= GT_BUF ? r : -1 - r;
+        auto all = [](int k, int n) { return (k & 0xffff) == 0 && (k >> 16) >= n; };
+        const int l0 = p0.x & 0xffff, l1 = p0.y & 0xffff, l2 = p0.z & 0xffff, ss = s0 * n1p;
+        sp[0] = make_int4(s0, ss, l1 | l2 << 16, 16 * l0);
+        // the box cell of a voxel from the bits of its rounded coordinates
+        sp[2].w = (int)(0u - (0x4B400000u + (unsigned)l0 + (unsigned)s0 * (0x4B400000u + (unsigned)l1) +
+                              (unsigned)ss * (0x4B400000u + (unsigned)l2)));
+        sp[3].w = n1p;
+        // floor(k / d) = k * (2^20 / d + 1) >> 20 for k < 1024, d < 1024
+        sp[4] = make_int4(s0 >> 2, (1 << 20) / (s0 >> 2) + 1, (1 << 20) / n1p + 1,
+                          nbox >> 2 | (all(p3.x, n0) && all(p3.y, n1) && all(p3.z, n2) ? 1 << 16 : 0));
+    }
     int4* const all4 = reinterpret_cast<int4*>(acc_all);
     for (int k = t; k < GT_SMEM / 4; k += blockDim.x) all4[k] = make_int4(0, 0, 0, 0);
     __syncthreads();
@@ -2416,104 +2449,92 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ) k_gather_T(EeParams P, 
     const float fx_inv = ge == 0xff ? __int_as_float(0x7fc00000) : __int_as_float((254 - se) << 23);
     const float gds = gd * fx_scale;
     int parity = 0;  // buffer of the next shared-memory cone
-    for (int r = 0; r < P.nrays; r++) {
-        const int4 p0 = s_p[r][0];
-        const int l0 = p0.x & 0xffff, n0 = p0.x >> 16, l1 = p0.y & 0xffff, n1 = p0.y >> 16, l2 = p0.z & 0xffff,
-                  n2 = p0.z >> 16;
-        const bool empty = n0 <= 0 || n1 <= 0 || n2 <= 0;
-        // box cell (k0, k1, k2) over (i, tY, tZ) at k0 + s0 * (k1 + n1p * k2)
-        const int s0 = empty ? 0 : p0.w;  // row stride of the box (>= n0, a multiple of 4)
-        // rows per slab: odd, so that the slab stride s0 * n1p is 4 x odd
-        // (mod 32) and the slabs of adjacent voxels spread over the banks
-        // too; the padding rows (k1 >= n1) are never scattered to
-        const int n1p = n1 | 1;
-        const int nbox = empty ? 0 : n1p * s0 * n2;
-        if (nbox > 0 && nbox <= GT_BUF) {
+    for (int c = 0; c < s_n; c++) {
+        const int r = s_list[c];
+        if (r >= 0) {
             // buffers alternate over the shared-memory cones: the last flush
             // of this buffer (two such cones back) was cleared by every
             // thread before the barrier of the previous cone
             int* acc = acc_all + parity * GT_BUF;
             parity ^= 1;
+            const int4 p0 = s_p[r][0], p2 = s_p[r][2];
             if (gd != 0.f) {
                 const float4 a0 = s_A[r][0], a1 = s_A[r][1], a2 = s_A[r][2];
                 const f3 q = mk(fmaf(a0.x, dx, fmaf(a0.y, dy, fmaf(a0.z, dz, a0.w))),
                                 fmaf(a1.x, dx, fmaf(a1.y, dy, fmaf(a1.z, dz, a1.w))),
                                 fmaf(a2.x, dx, fmaf(a2.y, dy, fmaf(a2.z, dz, a2.w))));
                 // the forward gather skips a cone where q is outside [0, rev)
-                if (!(q.x < 0.f || q.y < 0.f || q.z < 0.f)) {
-                    const int4 pv = s_p[r][2];  // rev - l per axis
-                    const float f0 = floorf(q.y), f1 = floorf(q.z), f2 = floorf(q.x);
-                    const int j0 = (int)f0 - l0, j1 = (int)f1 - l1, j2 = (int)f2 - l2;
-                    if (j0 < pv.x && j1 < pv.y && j2 < pv.z) {
-                        const float a0 = q.y - f0, a1 = q.z - f1, a2 = q.x - f2;
-                        // all eight corners lie in the box (its set-up above);
-                        // those past the array's end are dropped by the flush
-                        const float w0[2] = {1.f - a0, a0}, w1[2] = {1.f - a1, a1}, w2[2] = {1.f - a2, a2};
-                        int* const c = acc + j0 + s0 * (j1 + n1p * j2);
-                        const int ss = s0 * n1p;
+                if (!(q.x < 0.f || q.y < 0.f || q.z < 0.f || q.y >= __int_as_float(p2.x) ||
+                      q.z >= __int_as_float(p2.y) || q.x >= __int_as_float(p2.z))) {
+                    // floor by rounding q - 1/2 at unit spacing, off the
+                    // conversion unit; an integer q may take the cell below with
+                    // weight 1 on its upper corner (never below the box: its
+                    // origin is 0 or under the lowest q by 1e-3)
+                    const float b0 = (q.y - 0.5f) + 12582912.f, b1 = (q.z - 0.5f) + 12582912.f,
+                                b2 = (q.x - 0.5f) + 12582912.f;
+                    const float a0 = q.y - (b0 - 12582912.f), a1 = q.z - (b1 - 12582912.f),
+                                a2 = q.x - (b2 - 12582912.f);
+                    // all eight corners lie in the box (its set-up above);
+                    // those past the array's end are dropped by the flush
+                    const float w0[2] = {1.f - a0, a0}, w1[2] = {1.f - a1, a1}, w2[2] = {1.f - a2, a2};
+                    int* const cell =
+                        acc + (int)((unsigned)__float_as_int(b0) + (unsigned)p0.x * (unsigned)__float_as_int(b1) +
+                                    (unsigned)p0.y * (unsigned)__float_as_int(b2) + (unsigned)p2.w);
 #pragma unroll
-                        for (int d2 = 0; d2 < 2; d2++) {
-                            const float t2 = w2[d2] * gds;
+                    for (int d2 = 0; d2 < 2; d2++) {
+                        const float t2 = w2[d2] * gds;
 #pragma unroll
-                            for (int d1 = 0; d1 < 2; d1++) {
-                                const float t1 = w1[d1] * t2;
-                                // w * g * s rounded to an integer: the sum with
-                                // 1.5 * 2^23 has unit spacing, its low bits are
-                                // the integer (|w g s| < 2^22)
+                        for (int d1 = 0; d1 < 2; d1++) {
+                            const float t1 = w1[d1] * t2;
+                            // w * g * s rounded to an integer: the sum with
+                            // 1.5 * 2^23 has unit spacing, its low bits are
+                            // the integer (|w g s| < 2^22)
 #pragma unroll
-                                for (int d0 = 0; d0 < 2; d0++)
-                                    atomicAdd(c + d0 + d1 * s0 + d2 * ss,
-                                              __float_as_int(fmaf(w0[d0], t1, 12582912.f)) - 0x4B400000);
-                            }
+                            for (int d0 = 0; d0 < 2; d0++)
+                                atomicAdd(cell + d0 + d1 * p0.x + d2 * p0.y,
+                                          __float_as_int(fmaf(w0[d0], t1, 12582912.f)) - 0x4B400000);
                         }
                     }
                 }
             }
             __syncthreads();
-            const int4 p1 = s_p[r][1];
-            float* rb = base + (long long)(((unsigned long long)(unsigned)p1.w << 32) | (unsigned)p1.z);
-            Brick Bv;  // strides only (bk_y, bk_z)
-            Bv.sy = p1.x;
-            Bv.sz = p1.y;
+            const int4 p1 = s_p[r][1], p3 = s_p[r][3], p4 = s_p[r][4];
+            float* rb = base + (long long)(((unsigned long long)(unsigned)p1.w << 32) | (unsigned)p1.z) + p0.w;
+            const int l1 = p0.z & 0xffff, l2 = p0.z >> 16;
             // one box quad (4 samples) per iteration, quad index = kq + nq0 *
-            // (k1 + n1p * k2); (k + 0.5) / n is at least 1/(2n) away from an
-            // integer, far above the FP32 error of (k + 0.5) * rcp(n) for
-            // these sizes, so the floored quotients are exact.  A non-zero quad is one 16-byte vector
+            // (k1 + n1p * k2).  A non-zero quad is one 16-byte vector
             // reduction into the bricked REV gradient (brick rows are 16-byte
             // aligned: arena and cone offsets are multiples of 64 floats),
             // and is cleared for the buffer's next cone.
             int4* acc4 = reinterpret_cast<int4*>(acc);  // s0 is a multiple of 4
-            const int nquad = nbox >> 2;
-            const int nq0 = s0 >> 2;
-            const float invq = __frcp_rn((float)nq0), inv1 = __frcp_rn((float)n1p);
+            const int nquad = p4.w & 0xffff;
+            const bool kept = p4.w >> 16;
             for (int k = t; k < nquad; k += blockDim.x) {
                 const int4 v = acc4[k];
                 if (v.x != 0 || v.y != 0 || v.z != 0 || v.w != 0) {
                     acc4[k] = make_int4(0, 0, 0, 0);
-                    const int q1 = __float2int_rd(((float)k + 0.5f) * invq);
-                    const int kq = k - q1 * nq0;
-                    const int k2 = __float2int_rd(((float)q1 + 0.5f) * inv1);
-                    const int k1 = q1 - k2 * n1p;
+                    const int q1 = k * p4.y >> 20, kq = k - q1 * p4.x;
+                    const int k2 = q1 * p4.z >> 20, k1 = q1 - k2 * p3.w;
                     // rows and slabs past the array's end and quads that
                     // start past it hold the forward's border corners (0), and
                     // cells outside the kept part are not read: cleared, not
                     // sent; a quad that starts inside ends in its last brick,
                     // whose padding nothing reads
-                    const int4 pk = s_p[r][3];
-                    if (4 * kq >= (pk.x & 0xffff) && 4 * kq < (pk.x >> 16) && k1 >= (pk.y & 0xffff) &&
-                        k1 < (pk.y >> 16) && k2 >= (pk.z & 0xffff) && k2 < (pk.z >> 16))
-                        red_v4(rb + bk_x(l0 + 4 * kq) + bk_y(Bv, l1 + k1) + bk_z(Bv, l2 + k2), (float)v.x * fx_inv,
-                               (float)v.y * fx_inv, (float)v.z * fx_inv, (float)v.w * fx_inv);
+                    if (kept || (4 * kq >= (p3.x & 0xffff) && 4 * kq < (p3.x >> 16) && k1 >= (p3.y & 0xffff) &&
+                                 k1 < (p3.y >> 16) && k2 >= (p3.z & 0xffff) && k2 < (p3.z >> 16))) {
+                        const int y = l1 + k1, z = l2 + k2;
+                        red_v4(rb + (64 * kq + (y >> 2) * p1.x + ((y & 3) << 2) + (z >> 2) * p1.y + ((z & 3) << 4)),
+                               (float)v.x * fx_inv, (float)v.y * fx_inv, (float)v.z * fx_inv, (float)v.w * fx_inv);
+                    }
                 }
             }
-        } else if (nbox > GT_BUF && gd != 0.f) {
+        } else if (gd != 0.f) {
             // footprint too large for a shared buffer (a REV spacing finer
             // than the voxels): scatter directly
-            const EeRayGeom& R = G.ray[r];
-            const float4 a0 = s_A[r][0], a1 = s_A[r][1], a2 = s_A[r][2];
-            const f3 q = mk(fmaf(a0.x, dx, fmaf(a0.y, dy, fmaf(a0.z, dz, a0.w))),
-                            fmaf(a1.x, dx, fmaf(a1.y, dy, fmaf(a1.z, dz, a1.w))),
-                            fmaf(a2.x, dx, fmaf(a2.y, dy, fmaf(a2.z, dz, a2.w))));
+            const EeRayGeom& R = G.ray[-1 - r];
+            const f3 q = mk(fmaf(R.A[0], dx, fmaf(R.A[1], dy, fmaf(R.A[2], dz, -R.q0[0]))),
+                            fmaf(R.A[3], dx, fmaf(R.A[4], dy, fmaf(R.A[5], dz, -R.q0[1]))),
+                            fmaf(R.A[6], dx, fmaf(R.A[7], dy, fmaf(R.A[8], dz, -R.q0[2]))));
             if (!(q.y >= (float)R.rev[0] || q.z >= (float)R.rev[1] || q.x >= (float)R.rev[2] || q.x < 0.f ||
                   q.y < 0.f || q.z < 0.f) &&
                 lit_form(R, q.z, q.x) >= 0.5f * EE_LIT_READ)  // a line around the voxel can be lit, so all are kept
