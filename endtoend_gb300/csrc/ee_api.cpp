@@ -203,7 +203,8 @@ struct ee_context {
     // per-call scratch
     DevBuf<EeBeamSpec> d_specs;
     DevBuf<EeBeamGeom> d_geoms;
-    DevBuf<float> terma, unit, terma_grad;
+    DevBuf<float> terma, unit;
+    DevBuf<float4> terma_grad;  // a chunk's quads
     DevBuf<float> rev;  // a chunk's REV dose, then (adjoint) its REV gradient
     ConeBufs cone;
     DevBuf<int> bl_idx;
@@ -307,7 +308,7 @@ void terma_box(const EeParams& P, EeBeamSpec& S, int t0[3], int tn[3]) {
 }
 
 void build_specs(const EeParams& P, const ee_beam* beams, int nbeams, EeBeamSpec* out) {
-    long long off = 0, toff = 0;
+    long long off = 0, toff = 0, qoff = 0;
     for (int b = 0; b < nbeams; b++) {
         const ee_beam& B = beams[b];
         double az, zen;
@@ -335,6 +336,8 @@ void build_specs(const EeParams& P, const ee_beam* beams, int nbeams, EeBeamSpec
         terma_box(P, S, S.t0, S.tn);
         S.t_off = toff;
         toff += ee_brick_vol(S.tn);
+        S.q_off = qoff;
+        qoff += ee_quad_vol(S.tn);
     }
 }
 
@@ -411,7 +414,9 @@ constexpr int kTermaBeams = 32768;  // beams per launch: a grid's z extent
 
 struct ChunkDims {
     long long rev_total = 0, max_tvol = 1;
+    long long q0 = 0, quads = 0;  // TERMA gradient: first quad of the chunk's first beam, and their number
     int max_line = 1, max_lines = 1, max_rows = 1, max_tiles = 1;
+    long long bytes() const { return 4 * rev_total + 16 * quads; }
 };
 
 // The lane cones' work space for a set of chunks: the longest line, the lists
@@ -493,7 +498,6 @@ int pipeline(ee_context* c, const PipeArgs& A) {
     if (adj) {
         EE_CUDA(grow(c, c->unit, tvol_total));
         EE_CUDA(grow(c, c->bl_idx, tvol_total));
-        EE_CUDA(grow(c, c->terma_grad, tvol_total + 4));  // +4: vector-reduction padding
     }
     EE_CUDA(cudaMemcpyAsync(c->d_specs.p, c->h_specs.p, sizeof(EeBeamSpec) * n, cudaMemcpyHostToDevice, s));
     c->last_info.clear();
@@ -523,17 +527,20 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         EeBeamGeomHead& G = hg[b];
         if (G.status != 0) return fail(G.status, "beam %d: %s", b, status_text(G.status));
         c->last_info.push_back(beam_info(c->h_specs.p[b], G));
-        // a beam's share of the budget: its REV arena; the lane cones' scratch
-        // takes a quarter at most
+        // a beam's share of the budget: its REV arena and TERMA gradient; the
+        // lane cones' scratch takes a quarter at most
+        const long long quads = adj ? ee_quad_vol(c->h_specs.p[b].tn) : 0;
         if (starts.empty() || b - starts.back() >= kTermaBeams ||
-            4 * (dims.back().rev_total + G.store_total) > c->max_batch_bytes / 4 * 3) {
+            dims.back().bytes() + 4 * G.store_total + 16 * quads > c->max_batch_bytes / 4 * 3) {
             starts.push_back(b);
             dims.push_back(ChunkDims());
+            dims.back().q0 = c->h_specs.p[b].q_off;
         }
         ChunkDims& D = dims.back();
         G.arena_off = D.rev_total;
         G.arena_cap = G.store_total;
         D.rev_total += G.store_total;
+        D.quads += quads;
         D.max_tvol = std::max(D.max_tvol, tvol_of(c->h_specs.p[b]));
         D.max_line = std::max(D.max_line, G.max_line);
         D.max_lines = std::max(D.max_lines, G.max_lines);
@@ -549,6 +556,11 @@ int pipeline(ee_context* c, const PipeArgs& A) {
     long long rev_max = 0;
     for (auto& D : dims) rev_max = std::max(rev_max, D.rev_total);
     EE_CUDA(grow(c, c->rev, rev_max + 4));  // +4: vector-reduction padding
+    if (adj) {
+        long long quads = 0;
+        for (auto& D : dims) quads = std::max(quads, D.quads);
+        EE_CUDA(grow(c, c->terma_grad, quads));
+    }
     EeConeWork work;
     if (c->P.mode == EE_KERNEL_EXP) {
         int max_line = 1;
@@ -594,22 +606,23 @@ int pipeline(ee_context* c, const PipeArgs& A) {
     long long nfl_all = 0;
     for (int b = 0; b < n; b++) nfl_all += (long long)A.beams[b].fmap_size[0] * A.beams[b].fmap_size[1];
     EE_CUDA(cudaMemsetAsync(A.d_fgrad, 0, sizeof(float) * nfl_all, s));
-    EE_CUDA(cudaMemsetAsync(c->terma_grad.p, 0, sizeof(float) * tvol_total, s));
     for (int k = 0; k < nchunks; k++) {
         const int b0 = starts[k], nb = starts[k + 1] - b0;
         const EeBeamSpec* dsp = c->d_specs.p + b0;
         const EeBeamGeom* dge = c->d_geoms.p + b0;
         const ChunkDims& D = dims[k];
         if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
+        EE_CUDA(cudaMemsetAsync(c->terma_grad.p, 0, sizeof(float4) * D.quads, s));
+        float4* const tg = c->terma_grad.p - D.q0;  // a beam's quads at its q_off
         EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev.p, nb, D.max_lines, s));
         EE_CUDA(staged(c, EE_STAGE_GATHER_T, 1, [&] {
             return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev.p, nb, D.max_tiles, s);
         }));
         EE_CUDA(staged(c, EE_STAGE_CONE_T, cone_launches, [&] {
-            return ee_launch_cone_T(c->P, dsp, dge, c->rev.p, work, c->terma_grad.p, nb, D.max_lines, D.max_line, s);
+            return ee_launch_cone_T(c->P, dsp, dge, c->rev.p, work, tg, nb, D.max_lines, D.max_line, s);
         }));
         EE_CUDA(staged(c, EE_STAGE_TERMA_T, 1, [&] {
-            return ee_launch_terma_T(c->P, dsp, dge, c->unit.p, c->bl_idx.p, c->terma_grad.p, A.d_fgrad, nb,
+            return ee_launch_terma_T(c->P, dsp, dge, c->unit.p, c->bl_idx.p, tg, A.d_fgrad, nb,
                                      D.max_tvol, s);
         }));
     }
@@ -815,7 +828,8 @@ struct ee_plan {
     long long tvol_total = 0, max_tvol = 1, rev_max = 0, nfl = 0;
     DevBuf<EeBeamSpec> d_specs;
     DevBuf<EeBeamGeom> d_geoms;
-    DevBuf<float> terma, unit, terma_grad, rev;
+    DevBuf<float> terma, unit, rev;
+    DevBuf<float4> terma_grad;
     DevBuf<int> bl_idx;
     ConeBufs cone;
     EeConeWork work;
@@ -866,17 +880,18 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
     }
     if (!pl->adjoint) return cudaSuccess;
     PL(cudaMemsetAsync(pl->d_fgrad, 0, sizeof(float) * pl->nfl, s));
-    PL(cudaMemsetAsync(pl->terma_grad.p, 0, sizeof(float) * pl->tvol_total, s));
     for (int k = 0; k < nchunks; k++) {
         const int b0 = pl->starts[k], nb = pl->starts[k + 1] - b0;
         const EeBeamSpec* dsp = pl->d_specs.p + b0;
         const EeBeamGeom* dge = pl->d_geoms.p + b0;
         const ChunkDims& D = pl->dims[k];
         if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
+        PL(cudaMemsetAsync(pl->terma_grad.p, 0, sizeof(float4) * D.quads, s));
+        float4* const tg = pl->terma_grad.p - D.q0;  // a beam's quads at its q_off
         PL(ee_launch_rev_zero(P, dsp, dge, pl->rev.p, nb, D.max_lines, s));
         PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev.p, nb, D.max_tiles, s));
-        PL(ee_launch_cone_T(P, dsp, dge, pl->rev.p, pl->work, pl->terma_grad.p, nb, D.max_lines, D.max_line, s));
-        PL(ee_launch_terma_T(P, dsp, dge, pl->unit.p, pl->bl_idx.p, pl->terma_grad.p, pl->d_fgrad, nb, D.max_tvol, s));
+        PL(ee_launch_cone_T(P, dsp, dge, pl->rev.p, pl->work, tg, nb, D.max_lines, D.max_line, s));
+        PL(ee_launch_terma_T(P, dsp, dge, pl->unit.p, pl->bl_idx.p, tg, pl->d_fgrad, nb, D.max_tvol, s));
     }
 #undef PL
     return cudaSuccess;
@@ -1274,17 +1289,20 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
     for (int b = 0; b < nbeams; b++) {
         EeBeamSpec& S = pl->specs[b];
         PlanBound B = plan_bound(c, S);
-        // the REV arena in three quarters of the budget, as pipeline()
+        // the arenas in three quarters of the budget, as pipeline()
+        const long long quads = pl->adjoint ? ee_quad_vol(S.tn) : 0;
         if (pl->starts.empty() || b - pl->starts.back() >= kTermaBeams ||
-            4 * (pl->dims.back().rev_total + B.rev) > c->max_batch_bytes / 4 * 3) {
+            pl->dims.back().bytes() + 4 * B.rev + 16 * quads > c->max_batch_bytes / 4 * 3) {
             pl->starts.push_back(b);
             pl->dims.push_back(ChunkDims());
+            pl->dims.back().q0 = S.q_off;
         }
         ChunkDims& D = pl->dims.back();
         S.plan_off = D.rev_total;
         S.plan_cap = B.rev;
         S.t_off = pl->tvol_total;
         D.rev_total += B.rev;
+        D.quads += quads;
         D.max_tvol = std::max(D.max_tvol, tvol_of(S));
         D.max_line = std::max(D.max_line, B.max_line);
         D.max_lines = std::max(D.max_lines, B.max_lines);
@@ -1310,7 +1328,9 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
     if (pl->adjoint) {
         EE_CUDA(pl->unit.ensure(pl->tvol_total));
         EE_CUDA(pl->bl_idx.ensure(pl->tvol_total));
-        EE_CUDA(pl->terma_grad.ensure(pl->tvol_total + 4));
+        long long quads = 0;
+        for (auto& D : pl->dims) quads = std::max(quads, D.quads);
+        EE_CUDA(pl->terma_grad.ensure(quads));
     }
     EE_CUDA(cudaMemcpyAsync(pl->d_specs.p, pl->specs.data(), sizeof(EeBeamSpec) * nbeams, cudaMemcpyHostToDevice, s));
     pl->status.resize(nbeams);
@@ -1358,7 +1378,7 @@ int ee_plan_info(ee_plan* pl, int* lane_block, long long* device_bytes, int* nch
     if (nchunks) *nchunks = (int)pl->starts.size() - 1;
     if (device_bytes) {
         long long b = 4ll * (pl->tvol_total + pl->rev_max) + pl->cone.bytes();
-        if (pl->adjoint) b += 4ll * 3 * pl->tvol_total;
+        if (pl->adjoint) b += 4ll * 2 * pl->tvol_total + 16ll * pl->terma_grad.n;
         *device_bytes = b;
     }
     return EE_OK;
@@ -1523,9 +1543,9 @@ long long ee_internal_context_bytes(ee_context* c) {
     std::lock_guard<std::mutex> lk(c->mu);
     long long b = 0;
     b += 4ll * (c->density.n + c->cumkern.n + c->expp.n + c->terma.n + c->unit.n + c->rev.n +
-                c->terma_grad.n + c->io_fluence.n + c->io_dose.n + c->io_grad.n + c->xf.n + c->xg.n + c->spread_w.n +
+                c->io_fluence.n + c->io_dose.n + c->io_grad.n + c->xf.n + c->xg.n + c->spread_w.n +
                 c->bl_idx.n);
-    b += 8ll * c->acc.n + c->cone.bytes();
+    b += 8ll * c->acc.n + 16ll * c->terma_grad.n + c->cone.bytes();
     b += (long long)sizeof(EeBeamSpec) * c->d_specs.n + (long long)sizeof(EeBeamGeom) * c->d_geoms.n;
     if (c->dens_array) b += 4ll * c->density.n;
     return b;

@@ -58,6 +58,14 @@ inline __host__ __device__ long long ee_brick_vol(const int tn[3]) {
     return 64ll * ((tn[0] + 3) >> 2) * ((tn[1] + 3) >> 2) * ((tn[2] + 3) >> 2);
 }
 
+// The adjoint scatters each sample's TERMA gradient into quads: the four corners
+// of a cell in (x, y) at one z as one float4, for the cells from one before the
+// box to its last voxel in x and y, bricked over (n0 + 1, n1 + 1, n2).  A voxel's
+// gradient is the sum of one value of each of its four cells.
+inline __host__ __device__ long long ee_quad_vol(const int tn[3]) {
+    return 64ll * ((tn[0] + 4) >> 2) * ((tn[1] + 4) >> 2) * ((tn[2] + 3) >> 2);
+}
+
 // The forward gather's warp patch: EE_GATHER_PX x EE_GATHER_PY x EE_GATHER_PZ
 // patient voxels (32 lanes); a warp owns a group of PY x PZ patient rows.
 constexpr int EE_GATHER_PX = 8, EE_GATHER_PY = 2, EE_GATHER_PZ = 2;
@@ -82,6 +90,7 @@ struct EeBeamSpec {
     int t0[3];             // origin (full-grid voxel index)
     int tn[3];             // size
     long long t_off;       // element offset in the TERMA arena (a multiple of 64: bricks, below)
+    long long q_off;       // first quad of the beam's TERMA gradient (ee_quad_vol)
     // FP64 copies for re-deciding the beamlet of voxels whose FP32 fluence-map
     // coordinate lands within 1e-4 of a beamlet boundary
     double srcd[3];
@@ -273,7 +282,7 @@ cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const E
 cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
                                const float* dose_grad, float* rev_grad, int nbeams, int max_tiles, cudaStream_t s);
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
-                             const EeConeWork& work, float* terma_grad, int nbeams, int max_lines, int max_line,
+                             const EeConeWork& work, float4* terma_grad, int nbeams, int max_lines, int max_line,
                              cudaStream_t s);
 // zeros on every line's segment of a chunk's REV gradient arena (before
 // ee_launch_gather_T; the forward cone kernels zero their own arena)
@@ -285,7 +294,7 @@ bool ee_debug_poison();
 // per-beam status words of a geometry array (strided copy), for plans
 cudaError_t ee_copy_status(const EeBeamGeom* geoms, int* status_host, int nbeams, cudaStream_t s);
 cudaError_t ee_launch_terma_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
-                              const float* unit_terma, const int* beamlet_idx, const float* terma_grad,
+                              const float* unit_terma, const int* beamlet_idx, const float4* terma_grad,
                               float* fluence_grad, int nbeams, long long max_tvol, cudaStream_t s);
 // EndtoEnd loss pieces
 cudaError_t ee_launch_loss_grad(const float* dose, const float* ptv_w, const float* ptv_t, const float* oar_w,

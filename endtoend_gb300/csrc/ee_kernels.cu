@@ -1480,7 +1480,7 @@ __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_tab(EeParams P, const E
 // One line of k_cone_T_tab on the W lanes of its group (as tab_fwd_line).
 __device__ __forceinline__ void tab_adj_line(int W, const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
                                              const EeRayGeom& R, const float* __restrict__ grad_beam,
-                                             float* __restrict__ terma_grad, const TabLine& L, int lane, float* arr,
+                                             float4* __restrict__ terma_grad, const TabLine& L, int lane, float* arr,
                                              int Lp, const float* tab, unsigned short* Y) {
     float* Pv = arr;
     float* Sgv = Pv + Lp;
@@ -1511,14 +1511,14 @@ __device__ __forceinline__ void tab_adj_line(int W, const EeParams& P, const EeB
         __syncwarp();
     }
     // transpose of the REV TERMA resample
-    float* tg = terma_grad + S.t_off;
-    const Brick Bt = brick_of(S.tn);
+    float4* tg = terma_grad + S.q_off;
+    const Brick Bt = quads_of(S.tn);
     const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
     for (int k = L.a + lane; k <= L.e; k += W) {
         const float v = Tb[k];
         if (rho[k] < 0.f || v == 0.f) continue;
         const f3 p = sample_point(L.F, L.i0 + k);
-        tri_brick_scatter_edge(tg, Bt, p.x - t0.x, p.y - t0.y, p.z - t0.z, v);
+        quad_scatter(tg, Bt, p.x - t0.x, p.y - t0.y, p.z - t0.z, v);
     }
 }
 
@@ -1527,7 +1527,7 @@ __device__ __forceinline__ void tab_adj_line(int W, const EeParams& P, const EeB
 __global__ void __launch_bounds__(TAB_WARPS * 32) k_cone_T_tab(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                                const EeBeamGeom* __restrict__ geoms,
                                                                const float* __restrict__ rev_grad,
-                                                               float* __restrict__ terma_grad, int maxL) {
+                                                               float4* __restrict__ terma_grad, int maxL) {
     extern __shared__ float4 sm4[];
     float* sm = reinterpret_cast<float*>(sm4);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1891,13 +1891,14 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
 // part and scatters Tbar into the TERMA-box gradient.  Only the quads [q0, q1]
 // of the field span have a TERMA gradient: pass A stops below q0, pass B
 // above q1, and outside the span each only updates Z, with the densities of
-// the texture; the scratch holds the span alone.  One 24 x 24 beam 0.428 ->
-// 0.242 ms, 20 beams of 128^2 pixels 8.1 -> 2.9 ms; of that 0.265 -> 0.242 by
-// scattering interior samples without tests per corner row and those at the
-// box's faces in one loop per quad.
+// the texture; the scratch holds the span alone.  A quad is loaded while the one
+// before it is worked on.  Bound by the reductions into the TERMA gradient
+// (half of the time) and by latency: one 24 x 24 beam 0.428 -> 0.143 ms, 20
+// beams of 128^2 pixels 8.1 -> 2.6 ms, of which 0.247 -> 0.143 and 2.93 -> 2.64
+// by reducing into quads (quad_scatter) and loading ahead.
 __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec* __restrict__ specs,
                                             const EeBeamGeom* __restrict__ geoms, const float* __restrict__ rev_grad,
-                                            float* __restrict__ terma_grad, int b, int ray, int slot,
+                                            float4* __restrict__ terma_grad, int b, int ray, int slot,
                                             float4* __restrict__ sA) {
     const EeBeamGeom& G = geoms[b];
     const EeRayGeom& R = G.ray[ray];
@@ -1932,19 +1933,29 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
         h1 = hm1; h2 = hm2;
         return e;
     };
+    // a quad's densities and gradients; the walks load a quad while they work on
+    // the one before it
+    auto load = [&](int q, float (&r)[4], float4& g) {
+        g = *reinterpret_cast<const float4*>(gin + 64 * q);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int i = 4 * q + j;
+            r[j] = rho_at(P, sample_point(F, i));
+            if (i < s.i0 || i > s.i1) r[j] = -1.f;
+        }
+    };
     {   // pass A, down from i1
         begin(RC.row_fwd);
+        float rn[4];
+        float4 gn4;
+        load(s.i1 >> 2, rn, gn4);
 #pragma unroll 1
         for (int q = s.i1 >> 2; q >= s.q0; q--) {
-            const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
-            const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
+            const float gl[4] = {gn4.x, gn4.y, gn4.z, gn4.w};
             float rl[4], e[4];
 #pragma unroll
-            for (int j = 3; j >= 0; j--) {
-                const int i = 4 * q + j;
-                rl[j] = rho_at(P, sample_point(F, i));
-                if (i < s.i0 || i > s.i1) rl[j] = -1.f;
-            }
+            for (int j = 0; j < 4; j++) rl[j] = rn[j];
+            if (q > s.q0) load(q - 1, rn, gn4);
 #pragma unroll
             for (int j = 3; j >= 0; j--) e[j] = step(rl[j], gl[j]);
             if (q <= s.q1) {
@@ -1970,37 +1981,28 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
 #pragma unroll
             for (int j = 0; j < 4; j++) step(rl[j], gl[j]);
         }
-        float* tg = terma_grad + S.t_off;
-        const Brick Bt = brick_of(S.tn);
+        float4* tg = terma_grad + S.q_off;
+        const Brick Bt = quads_of(S.tn);
         const f3 t0 = mk((float)S.t0[0], (float)S.t0[1], (float)S.t0[2]);
+        float4 n01 = sA[0], n23 = sA[32], n4 = *reinterpret_cast<const float4*>(gin + 64 * s.q0);
 #pragma unroll 1
         for (int q = s.q0; q <= s.q1; q++) {
-            const float4* sq = sA + 64 * (q - s.q0);
-            const float4 s01 = sq[0], s23 = sq[32];
-            const float4 g4 = *reinterpret_cast<const float4*>(gin + 64 * q);
+            const float4 s01 = n01, s23 = n23, g4 = n4;
+            if (q < s.q1) {
+                const float4* sq = sA + 64 * (q + 1 - s.q0);
+                n01 = sq[0];
+                n23 = sq[32];
+                n4 = *reinterpret_cast<const float4*>(gin + 64 * (q + 1));
+            }
             const float al[4] = {s01.x, s01.z, s23.x, s23.z}, rl[4] = {s01.y, s01.w, s23.y, s23.w};
             const float gl[4] = {g4.x, g4.y, g4.z, g4.w};
-            float tot[4];
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const float e = al[j] + step(rl[j], gl[j]);
-                tot[j] = rl[j] >= 0.f ? e : 0.f;
-            }
-            unsigned edge = 0;  // samples with corners outside the TERMA box
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const f3 g = sample_point(F, 4 * q + j), p = mk(g.x - t0.x, g.y - t0.y, g.z - t0.z);
-                int ci, cj, ck;
-                const bool cell = brick_cell(Bt, p.x, p.y, p.z, ci, cj, ck);
-                if (tot[j] != 0.f && cell) tri_brick_scatter_cell(tg, Bt, p.x, p.y, p.z, tot[j], ci, cj, ck);
-                edge |= tot[j] != 0.f && !cell ? 1u << j : 0u;
-            }
-#pragma unroll 1
-            for (; edge; edge &= edge - 1) {
-                const int w = __ffs((int)edge) - 1;
-                const f3 g = sample_point(F, 4 * q + w);
-                const float e = w == 0 ? tot[0] : w == 1 ? tot[1] : w == 2 ? tot[2] : tot[3];
-                tri_brick_scatter_edge(tg, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z, e);
+                const float tot = al[j] + step(rl[j], gl[j]);
+                if (rl[j] >= 0.f && tot != 0.f) {
+                    const f3 g = sample_point(F, 4 * q + j);
+                    quad_scatter(tg, Bt, g.x - t0.x, g.y - t0.y, g.z - t0.z, tot);
+                }
             }
         }
     }
@@ -2009,7 +2011,7 @@ __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec*
 __global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / EE_CONE_BLOCK_WARPS)
     k_cone_T_lane(EeParams P, const EeBeamSpec* __restrict__ specs, const EeBeamGeom* __restrict__ geoms,
                   const float* __restrict__ rev_grad, EeConeWork W, int nbeams, int cap,
-                  float* __restrict__ terma_grad) {
+                  float4* __restrict__ terma_grad) {
     cone_tiles_run(P, W, nbeams, cap, [&](int b, int ray, int slot, float4* scratch) {
         cone_T_line(P, specs, geoms, rev_grad, terma_grad, b, ray, slot, scratch);
     });
@@ -2020,7 +2022,7 @@ __global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / E
 __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                             const EeBeamGeom* __restrict__ geoms,
                                                             const float* __restrict__ rev_grad,
-                                                            float* __restrict__ terma_grad, int maxL) {
+                                                            float4* __restrict__ terma_grad, int maxL) {
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ray = blockIdx.y, b = blockIdx.z;
@@ -2078,12 +2080,12 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
     // transpose of the REV TERMA resample
     const f3 gl = ld3(R.G0) + ld3(R.Gy) * (float)tY + ld3(R.Gz) * (float)tZ;
     const f3 gx = ld3(R.Gx);
-    float* tg = terma_grad + S.t_off;
+    float4* tg = terma_grad + S.q_off;
     for (int k = lane; k < n; k += 32) {
         float v = Tb[k];
         if (rho[k] < 0.f || v == 0.f) continue;
         f3 gp = gl + gx * (float)(i0 + k);
-        tri_brick_scatter_edge(tg, brick_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
+        quad_scatter(tg, quads_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
                            gp.z - (float)S.t0[2], v);
     }
 }
@@ -2538,7 +2540,7 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams 
             if (!(q.y >= (float)R.rev[0] || q.z >= (float)R.rev[1] || q.x >= (float)R.rev[2] || q.x < 0.f ||
                   q.y < 0.f || q.z < 0.f) &&
                 lit_form(R, q.z, q.x) >= 0.5f * EE_LIT_READ)  // a line around the voxel can be lit, so all are kept
-                tri_brick_scatter_edge(base + R.offset, rev_store(R), q.y, q.z, q.x, gd);
+                tri_brick_scatter(base + R.offset, rev_store(R), q.y, q.z, q.x, gd);
         }
     }
 }
@@ -2553,7 +2555,7 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams 
 // share a beamlet add once.  The fluence enters linearly, as in the ss = 1
 // adjoint (a centre whose beamlet has zero fluence still has its slope).
 __global__ void __launch_bounds__(256) k_terma_T_ss(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                    const float* __restrict__ terma_grad, float* __restrict__ fgrad) {
+                                                    const float4* __restrict__ terma_grad, float* __restrict__ fgrad) {
     const int b = blockIdx.z;
     const EeBeamSpec& S = specs[b];
     const long long bvol = ee_brick_vol(S.tn);
@@ -2566,7 +2568,7 @@ __global__ void __launch_bounds__(256) k_terma_T_ss(EeParams P, const EeBeamSpec
     const int yr = (int)(bxy / nbx) * 4 + ((w >> 2) & 3);
     const int zr = (int)(brick / ((long long)nbx * nby)) * 4 + (w >> 4);
     if (xr >= S.tn[0] || yr >= S.tn[1] || zr >= S.tn[2]) return;
-    const float g = terma_grad[S.t_off + v];
+    const float g = quad_value(terma_grad + S.q_off, quads_of(S.tn), xr, yr, zr);
     if (g == 0.f) return;
     const int x = S.t0[0] + xr, y = S.t0[1] + yr, z = S.t0[2] + zr;
     const f3 src = ld3(S.src);
@@ -2606,7 +2608,7 @@ constexpr int TT_HIST = 4096, TT_VPT = 4;
 
 __global__ void __launch_bounds__(256) k_terma_T(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                  const float* __restrict__ unit, const int* __restrict__ bl_idx,
-                                                 const float* __restrict__ terma_grad, float* __restrict__ fluence_grad) {
+                                                 const float4* __restrict__ terma_grad, float* __restrict__ fluence_grad) {
     __shared__ float hist[TT_HIST];
     const int b = blockIdx.z;
     const EeBeamSpec& S = specs[b];
@@ -2615,6 +2617,15 @@ __global__ void __launch_bounds__(256) k_terma_T(EeParams P, const EeBeamSpec* _
     if (v0 >= tvol) return;
     const int t = threadIdx.x, nfl = S.fmap[0] * S.fmap[1];
     float* fg = fluence_grad + S.fl_off;
+    const Brick Q = quads_of(S.tn);
+    const int nbx = (S.tn[0] + 3) >> 2, nby = (S.tn[1] + 3) >> 2;
+    const float4* const tq = terma_grad + S.q_off;
+    auto grad = [&](long long v) {  // of bricked box element v, inside the box
+        const unsigned brick = (unsigned)(v >> 6), row = brick / nbx;
+        const int w = (int)(v & 63);
+        return quad_value(tq, Q, (int)(brick - row * nbx) * 4 + (w & 3), (int)(row % nby) * 4 + ((w >> 2) & 3),
+                          (int)(row / nby) * 4 + (w >> 4));
+    };
     if (nfl > TT_HIST) {
         for (int j = 0; j < TT_VPT; j++) {
             const long long v = v0 + j * 256 + t;
@@ -2623,7 +2634,7 @@ __global__ void __launch_bounds__(256) k_terma_T(EeParams P, const EeBeamSpec* _
             if (v < tvol) {
                 const long long o = S.t_off + v;
                 bl = bl_idx[o];
-                if (bl >= 0) val = unit[o] * terma_grad[o];
+                if (bl >= 0) val = unit[o] * grad(v);
             }
             const unsigned peers = __match_any_sync(FULL, bl);
             const int leader = __ffs(peers) - 1;
@@ -2642,7 +2653,7 @@ __global__ void __launch_bounds__(256) k_terma_T(EeParams P, const EeBeamSpec* _
             const long long o = S.t_off + v;
             const int bl = bl_idx[o];
             if (bl >= 0) {
-                const float val = unit[o] * terma_grad[o];
+                const float val = unit[o] * grad(v);
                 if (val != 0.f) atomicAdd(hist + bl, val);
             }
         }
@@ -2804,7 +2815,7 @@ cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const
 }
 
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
-                             const EeConeWork& work, float* terma_grad, int nbeams, int max_lines, int max_line,
+                             const EeConeWork& work, float4* terma_grad, int nbeams, int max_lines, int max_line,
                              cudaStream_t s) {
     if (P.mode == 1 && work.scratch) {
         const int cap = ee_cone_tiles_cap(max_lines);
@@ -2830,7 +2841,7 @@ cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const E
 }
 
 cudaError_t ee_launch_terma_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
-                              const float* unit_terma, const int* beamlet_idx, const float* terma_grad,
+                              const float* unit_terma, const int* beamlet_idx, const float4* terma_grad,
                               float* fluence_grad, int nbeams, long long max_tvol, cudaStream_t s) {
     (void)geoms;
     if (P.ss > 1) {  // supersampled TERMA: recompute the sub-voxel beamlets
