@@ -52,34 +52,35 @@ __device__ __forceinline__ void merge_crop_box(EeBeamGeom& G, bool nz, f3 bi, bo
     }
 }
 
-// TERMA without supersampling.  Threads take the box's voxels brick by brick
-// (4x4x4, ee_brick_vol), two bricks per block.  A voxel needs a ray trace when it
-// has a beamlet (beamlet_of, cudaSiddon.cu:143-165) whose fluence is
-// positive, or any beamlet when the unit TERMA is kept for the adjoint; the
-// rest are written at once.  The box is the field's axis-aligned hull, so
-// warps at the field's edge hold both kinds: the voxels to trace are first
-// gathered into a shared list in box order, and the block's leading threads
-// trace them, so the Siddon loops run with full warps (measured 10 % faster
-// than tracing in place).  Each voxel's arithmetic is unchanged.  The crop
-// box (host.cu:442-459) is reduced from the traced voxels with non-zero
-// TERMA: min/max of BEV indices as ordered-int keys, one merge per warp.
-// Bound by the texture unit's data stage (half its cycles busy on average and
-// three quarters on the busiest SM) and by the uneven ray lengths: 128 threads
-// per block free their place sooner than 256 (96 beams of 8^2..40^2 beamlets
-// on 200 x 200 x 160: 9.42 -> 8.99 ms).  40 resident warps per SM: 48
-// registers, no spills.
+// TERMA without supersampling.  A block takes ITEMS of the box's voxels brick by
+// brick (4x4x4, ee_brick_vol).  A voxel needs a ray trace when it has a beamlet
+// (beamlet_of, cudaSiddon.cu:143-165) whose fluence is positive, or any beamlet
+// when the unit TERMA is kept for the adjoint; the rest are written at once.  The
+// box is the field's axis-aligned hull, so warps at the field's edge hold both
+// kinds: the voxels to trace are first gathered into a shared list, a warp's in
+// box order, and the warps take 32 of them at a time, so the Siddon loops run
+// with full warps.  Each voxel's arithmetic is unchanged.  The crop box
+// (host.cu:442-459) is reduced from the traced voxels with non-zero TERMA:
+// min/max of BEV indices as ordered-int keys, one merge per 32 voxels.
+// Bound by the texture unit's data stage, where the rays' uneven lengths leave
+// it busy: 96 beams of 8^2..40^2 beamlets on 200 x 200 x 160 9.42 ms with 256
+// threads per block of 256 voxels, 8.99 with 128 of 128, 7.8 with two fetches in
+// flight, 6.3 with 512 voxels per 128 threads (ee_launch_terma: the rule).  40
+// resident warps per SM: 48 registers, no spills.
 constexpr int TERMA_BLOCK = 128;
 
-__global__ void __launch_bounds__(TERMA_BLOCK, 1280 / TERMA_BLOCK) k_terma(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                   EeBeamGeom* __restrict__ geoms, const float* __restrict__ fluence,
-                                                   float* __restrict__ terma, float* __restrict__ unit,
-                                                   int* __restrict__ bl_idx) {
-    __shared__ int s_v[TERMA_BLOCK], s_bl[TERMA_BLOCK], s_wcnt[TERMA_BLOCK / 32];
-    __shared__ float s_fl[TERMA_BLOCK];
+template <int ITEMS>
+__global__ void __launch_bounds__(TERMA_BLOCK, 1280 / TERMA_BLOCK)
+    k_terma(EeParams P, const EeBeamSpec* __restrict__ specs, EeBeamGeom* __restrict__ geoms,
+            const float* __restrict__ fluence, float* __restrict__ terma, float* __restrict__ unit,
+            int* __restrict__ bl_idx) {
+    __shared__ int s_bl[ITEMS], s_n, s_next;
+    __shared__ float s_fl[ITEMS];
+    __shared__ unsigned short s_v[ITEMS];
     const int b = blockIdx.z;
     const EeBeamSpec& S = specs[b];
     const long long bvol = ee_brick_vol(S.tn);
-    const long long vb = (long long)blockIdx.x * TERMA_BLOCK;
+    const long long vb = (long long)blockIdx.x * ITEMS;
     if (vb >= bvol) return;
     const int nbx = (S.tn[0] + 3) >> 2, nby = (S.tn[1] + 3) >> 2;
     // box indices of bricked box element v
@@ -91,74 +92,83 @@ __global__ void __launch_bounds__(TERMA_BLOCK, 1280 / TERMA_BLOCK) k_terma(EePar
         yr = (int)(bxy / nbx) * 4 + ((w >> 2) & 3);
         zr = (int)(brick / ((long long)nbx * nby)) * 4 + (w >> 4);
     };
-    const long long v = vb + threadIdx.x;
-    bool need = false;
-    int bl = -1;
-    float fl = 0.f;
-    if (v < bvol) {
-        int xr, yr, zr;
-        coords(v, xr, yr, zr);
-        // padding of the last bricks: never sampled, kept zero
-        const bool inbox = xr < S.tn[0] && yr < S.tn[1] && zr < S.tn[2];
-        if (inbox) {
-            const int x = S.t0[0] + xr, y = S.t0[1] + yr, z = S.t0[2] + zr;
-            const f3 vox = mk(P.start[0] + x * P.voxel[0], P.start[1] + y * P.voxel[1], P.start[2] + z * P.voxel[2]);
-            bl = beamlet_of(S, vox);
-            if (bl == -2) bl = beamlet_of_fp64(P, S, x, y, z);
-            if (bl >= 0) {
-                fl = __ldg(fluence + S.fl_off + bl);
-                need = fl > 0.f || unit;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        s_n = 0;
+        s_next = TERMA_BLOCK;
+    }
+    __syncthreads();
+    // the list of voxels to trace, a warp's in box order
+#pragma unroll 1
+    for (int c = threadIdx.x; c < ITEMS; c += TERMA_BLOCK) {
+        const long long v = vb + c;
+        bool need = false;
+        int bl = -1;
+        float fl = 0.f;
+        if (v < bvol) {
+            int xr, yr, zr;
+            coords(v, xr, yr, zr);
+            // padding of the last bricks: never sampled, kept zero
+            const bool inbox = xr < S.tn[0] && yr < S.tn[1] && zr < S.tn[2];
+            if (inbox) {
+                const int x = S.t0[0] + xr, y = S.t0[1] + yr, z = S.t0[2] + zr;
+                const f3 vox = mk(P.start[0] + x * P.voxel[0], P.start[1] + y * P.voxel[1], P.start[2] + z * P.voxel[2]);
+                bl = beamlet_of(S, vox);
+                if (bl == -2) bl = beamlet_of_fp64(P, S, x, y, z);
+                if (bl >= 0) {
+                    fl = __ldg(fluence + S.fl_off + bl);
+                    need = fl > 0.f || unit;
+                }
+            }
+            if (!need) {
+                terma[S.t_off + v] = 0.f;
+                if (unit) unit[S.t_off + v] = 0.f;
+                if (bl_idx) bl_idx[S.t_off + v] = bl;
             }
         }
-        if (!need) {
-            terma[S.t_off + v] = 0.f;
-            if (unit) unit[S.t_off + v] = 0.f;
-            if (bl_idx) bl_idx[S.t_off + v] = bl;
+        const unsigned m = __ballot_sync(FULL, need);
+        int p = 0;
+        if (lane == 0 && m) p = atomicAdd(&s_n, __popc(m));
+        p = __shfl_sync(FULL, p, 0) + __popc(m & ((1u << lane) - 1u));
+        if (need) {
+            s_v[p] = (unsigned short)c;
+            s_bl[p] = bl;
+            s_fl[p] = fl;
         }
     }
-    // the list of voxels to trace, in box order
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned m = __ballot_sync(FULL, need);
-    if (lane == 0) s_wcnt[warp] = __popc(m);
     __syncthreads();
-    int off = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < TERMA_BLOCK / 32; w++) {
-        const int c = s_wcnt[w];
-        off += w < warp ? c : 0;
-        total += c;
-    }
-    if (need) {
-        const int p = off + __popc(m & ((1u << lane) - 1u));
-        s_v[p] = threadIdx.x;
-        s_bl[p] = bl;
-        s_fl[p] = fl;
-    }
-    __syncthreads();
-    if (warp * 32 >= total) return;
-    bool nz = false, cap = false;
-    f3 bi = mk(0.f, 0.f, 0.f);
-    if ((int)threadIdx.x < total) {
-        const long long vt = vb + s_v[threadIdx.x];
-        int xr, yr, zr;
-        coords(vt, xr, yr, zr);
-        const int x = S.t0[0] + xr, y = S.t0[1] + yr, z = S.t0[2] + zr;
-        const f3 vox = mk(P.start[0] + x * P.voxel[0], P.start[1] + y * P.voxel[1], P.start[2] + z * P.voxel[2]);
-        const f3 src = ld3(S.src);
-        const float flt = s_fl[threadIdx.x];
-        const float rpl = siddon_rpl(P, vox, src, cap);
-        const float u = terma_per_fluence(P, rpl, vox, src, S.sad);
-        const float t = flt > 0.f ? flt * u : 0.f;
-        terma[S.t_off + vt] = t;
-        if (unit) unit[S.t_off + vt] = u;
-        if (bl_idx) bl_idx[S.t_off + vt] = s_bl[threadIdx.x];
-        if (t != 0.f) {
-            nz = true;
-            // crop box works on calc-bbox-relative indices (host.cu:445-448)
-            bi = mv(S.MB, mk((float)(x - P.bb0[0]), (float)(y - P.bb0[1]), (float)(z - P.bb0[2])));
+    const int total = s_n;
+    // 32 voxels to each warp, then the next 32 to the warp that is done
+#pragma unroll 1
+    for (int k0 = threadIdx.x & ~31; k0 < total;) {
+        const int k = k0 + lane;
+        bool nz = false, cap = false;
+        f3 bi = mk(0.f, 0.f, 0.f);
+        if (k < total) {
+            const long long vt = vb + s_v[k];
+            int xr, yr, zr;
+            coords(vt, xr, yr, zr);
+            const int x = S.t0[0] + xr, y = S.t0[1] + yr, z = S.t0[2] + zr;
+            const f3 vox = mk(P.start[0] + x * P.voxel[0], P.start[1] + y * P.voxel[1], P.start[2] + z * P.voxel[2]);
+            const f3 src = ld3(S.src);
+            const float flt = s_fl[k];
+            const float rpl = siddon_rpl(P, vox, src, cap);
+            const float u = terma_per_fluence(P, rpl, vox, src, S.sad);
+            const float t = flt > 0.f ? flt * u : 0.f;
+            terma[S.t_off + vt] = t;
+            if (unit) unit[S.t_off + vt] = u;
+            if (bl_idx) bl_idx[S.t_off + vt] = s_bl[k];
+            if (t != 0.f) {
+                nz = true;
+                // crop box works on calc-bbox-relative indices (host.cu:445-448)
+                bi = mv(S.MB, mk((float)(x - P.bb0[0]), (float)(y - P.bb0[1]), (float)(z - P.bb0[2])));
+            }
         }
+        merge_crop_box(geoms[b], nz, bi, cap);
+        if (ITEMS == TERMA_BLOCK) return;
+        if (lane == 0) k0 = atomicAdd(&s_next, 32);
+        k0 = __shfl_sync(FULL, k0, 0);
     }
-    merge_crop_box(geoms[b], nz, bi, cap);
 }
 
 // TERMA with supersampling (ss > 1, cudaSiddon.cu:248-258, 297-306): each
@@ -2686,9 +2696,20 @@ cudaError_t ee_launch_terma(const EeParams& P, const EeBeamSpec* specs, EeBeamGe
     if (P.ss > 1)
         k_terma_ss<<<dim3(grid1(max_tvol, 64), 1, nbeams), 256, 0, s>>>(P, specs, geoms, fluence, terma, unit,
                                                                         beamlet_idx);
-    else
-        k_terma<<<dim3(grid1(max_tvol, TERMA_BLOCK), 1, nbeams), TERMA_BLOCK, 0, s>>>(P, specs, geoms, fluence, terma,
-                                                                                      unit, beamlet_idx);
+    else {
+        // Voxels per block: larger blocks waste fewer lanes, smaller ones spread
+        // the rays of a small call over the chip.  128, 256, 512: one 24 x 24 beam
+        // 0.114, 0.133, 0.186 ms (4.2 M voxels), three 0.285, 0.293, 0.326, six
+        // 0.406, 0.389, 0.393, twelve 1.06, 0.93, 0.91, 96 8.0, 6.8, 6.3 (1024: 6.1).
+        const long long all = max_tvol * nbeams;
+        auto run = [&](auto kernel, int items) {
+            kernel<<<dim3(grid1(max_tvol, items), 1, nbeams), TERMA_BLOCK, 0, s>>>(P, specs, geoms, fluence, terma, unit,
+                                                                                beamlet_idx);
+        };
+        if (all < 18000000) run(k_terma<128>, 128);
+        else if (all < 40000000) run(k_terma<256>, 256);
+        else run(k_terma<512>, 512);
+    }
     return cudaGetLastError();
 }
 
@@ -2707,8 +2728,8 @@ cudaError_t ee_launch_geometry(const EeParams& P, const EeBeamSpec* specs, EeBea
 // on the large batches (128 KB and more: 4 % and up; 64 KB: the three engines
 // gain nothing on the batches).
 cudaError_t ee_kernel_setup() {
-    const void* const fn[] = {(const void*)k_terma, (const void*)k_cone_tiles, (const void*)k_cone_lane,
-                              (const void*)k_cone_T_lane};
+    const void* const fn[] = {(const void*)k_terma<128>,  (const void*)k_terma<256>,  (const void*)k_terma<512>,
+                              (const void*)k_cone_tiles, (const void*)k_cone_lane, (const void*)k_cone_T_lane};
     for (const void* f : fn) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
         if (e != cudaSuccess) return e;
