@@ -180,9 +180,12 @@ __global__ void __launch_bounds__(TERMA_BLOCK, 1280 / TERMA_BLOCK)
 // centres' order.  Neighbouring lanes then trace rays a fraction of a voxel
 // apart, so a warp's density fetches share their texels, which is what the
 // texture unit is bound by: 4 beams at ss = 3 8.00 ms with a thread per voxel
-// that traces its 27 centres in turn, 6.29 ms here.  (Unit TERMA and beamlets
-// are not kept: k_terma_T_ss recomputes the sub-voxel beamlets.)
-constexpr int TS_ITEMS = 1024;
+// that traces its 27 centres in turn, 6.29 ms here, 5.80 with two fetches in
+// flight, 5.60 with 2048 centres at a time, which hold all of ss = 3, instead of
+// 1024 (ss = 2: 2.01 -> 1.96; 32 centres at a time to the next free warp: the
+// same).  (Unit TERMA and beamlets are not kept: k_terma_T_ss recomputes the
+// sub-voxel beamlets.)
+constexpr int TS_ITEMS = 2048;
 
 __global__ void __launch_bounds__(256, 4) k_terma_ss(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                      EeBeamGeom* __restrict__ geoms, const float* __restrict__ fluence,
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(256, 4) k_terma_ss(EeParams P, const EeBeamSpe
         const int n = min(TS_ITEMS, 64 * nsub - i0);
         if (t == 0) s_n = 0;
         __syncthreads();
-        for (int k = t; k < TS_ITEMS; k += 256) {
+        for (int k = t; k < ((n + 255) & ~255); k += 256) {
             float fl = 0.f;
             f3 p;
             if (k < n && centre(i0 + k, p)) {
