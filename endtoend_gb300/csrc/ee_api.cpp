@@ -155,17 +155,19 @@ struct PinBuf {
 struct ConeBufs {
     DevBuf<float4> scratch;
     DevBuf<int> counts, tiles;
+    DevBuf<unsigned char> touched;
     static size_t scratch_size(int max_line, long long limit) {
         return (size_t)64 * ee_cone_quads(max_line) * ee_cone_warps(max_line, limit);
     }
     bool fits(int max_line, long long segments, long long ntiles, long long limit) const {
         return scratch.n >= scratch_size(max_line, limit) && counts.n >= (size_t)(1 + segments) &&
-               tiles.n >= (size_t)ntiles;
+               tiles.n >= (size_t)ntiles && touched.n >= (size_t)ntiles;
     }
     cudaError_t ensure(int max_line, long long segments, long long ntiles, long long limit) {
         cudaError_t e = scratch.ensure(scratch_size(max_line, limit));
         if (e == cudaSuccess) e = counts.ensure((size_t)(1 + segments));
         if (e == cudaSuccess) e = tiles.ensure((size_t)ntiles);
+        if (e == cudaSuccess) e = touched.ensure((size_t)ntiles);
         return e;
     }
     EeConeWork work(int max_line, long long limit) const {
@@ -173,15 +175,17 @@ struct ConeBufs {
         w.scratch = scratch.p;
         w.counts = counts.p;
         w.tiles = tiles.p;
+        w.touched = touched.p;
         w.quads = ee_cone_quads(max_line);
         w.warps = ee_cone_warps(max_line, limit);
         return w;
     }
-    long long bytes() const { return 16ll * scratch.n + 4ll * (counts.n + tiles.n); }
+    long long bytes() const { return 16ll * scratch.n + 4ll * (counts.n + tiles.n) + touched.n; }
     void release() {
         scratch.release();
         counts.release();
         tiles.release();
+        touched.release();
     }
 };
 
@@ -614,9 +618,9 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
         EE_CUDA(cudaMemsetAsync(c->terma_grad.p, 0, sizeof(float4) * D.quads, s));
         float4* const tg = c->terma_grad.p - D.q0;  // a beam's quads at its q_off
-        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev.p, nb, D.max_lines, s));
+        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev.p, work, nb, D.max_lines, s));
         EE_CUDA(staged(c, EE_STAGE_GATHER_T, 1, [&] {
-            return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev.p, nb, D.max_tiles, s);
+            return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev.p, work, nb, D.max_lines, D.max_tiles, s);
         }));
         EE_CUDA(staged(c, EE_STAGE_CONE_T, cone_launches, [&] {
             return ee_launch_cone_T(c->P, dsp, dge, c->rev.p, work, tg, nb, D.max_lines, D.max_line, s);
@@ -888,8 +892,8 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
         if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
         PL(cudaMemsetAsync(pl->terma_grad.p, 0, sizeof(float4) * D.quads, s));
         float4* const tg = pl->terma_grad.p - D.q0;  // a beam's quads at its q_off
-        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev.p, nb, D.max_lines, s));
-        PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev.p, nb, D.max_tiles, s));
+        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev.p, pl->work, nb, D.max_lines, s));
+        PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev.p, pl->work, nb, D.max_lines, D.max_tiles, s));
         PL(ee_launch_cone_T(P, dsp, dge, pl->rev.p, pl->work, tg, nb, D.max_lines, D.max_line, s));
         PL(ee_launch_terma_T(P, dsp, dge, pl->unit.p, pl->bl_idx.p, tg, pl->d_fgrad, nb, D.max_tvol, s));
     }

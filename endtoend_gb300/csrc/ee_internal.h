@@ -258,6 +258,7 @@ struct EeConeWork {
     int quads = 0;         // quads of samples per warp
     int* counts = nullptr; // [0] tiles taken; [1 + segment] tiles listed, segment = beam * nrays + cone in list order
     int* tiles = nullptr;  // [segment][tiles_cap] tiles of 8 x 4 lines
+    unsigned char* touched = nullptr;  // [beam * nrays + cone][tiles_cap] tiles that the adjoint gather adds to
 };
 constexpr int EE_CONE_BLOCK_WARPS = 2, EE_CONE_SM_WARPS = 24, EE_CONE_MAX_WARPS = 152 * EE_CONE_SM_WARPS;
 inline int ee_cone_quads(int max_line) { return (max_line + 3) / 4 + 2; }
@@ -280,14 +281,15 @@ cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const E
                              float* dose, int nbeams, int dose_mode, int max_rows, cudaStream_t s);
 // adjoint
 cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
-                               const float* dose_grad, float* rev_grad, int nbeams, int max_tiles, cudaStream_t s);
+                               const float* dose_grad, float* rev_grad, const EeConeWork& work, int nbeams,
+                               int max_lines, int max_tiles, cudaStream_t s);
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
                              const EeConeWork& work, float4* terma_grad, int nbeams, int max_lines, int max_line,
                              cudaStream_t s);
 // zeros on every line's segment of a chunk's REV gradient arena (before
 // ee_launch_gather_T; the forward cone kernels zero their own arena)
 cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,
-                               int nbeams, int max_lines, cudaStream_t s);
+                               const EeConeWork& work, int nbeams, int max_lines, cudaStream_t s);
 // test option: EE_DEBUG_POISON=1 fills scratch with NaN where the engine
 // relies on its kernels, not on a clear, to write every sample it reads
 bool ee_debug_poison();

@@ -1603,8 +1603,12 @@ __device__ __forceinline__ int list_cone(const EeParams& P, int y) {
 
 // The tiles of 8 x 4 lines that may hold a line with lit forms of at least
 // `least` in the dilated crop box: the lane cones' work lists, a block per
-// beam and cone.
+// beam and cone.  touched (adjoint): tiles that the gather added to; the
+// gradient of the others' lines is zero (20 beams of 128^2 pixels with a
+// target-and-organs gradient: adjoint cone 2.64 -> 0.80 ms; dense gradients
+// unchanged).
 __global__ void __launch_bounds__(256) k_cone_tiles(EeParams P, const EeBeamGeom* __restrict__ geoms, float least,
+                                                    const unsigned char* __restrict__ touched,
                                                     int* __restrict__ counts, int* __restrict__ tiles, int cap) {
     __shared__ int s_n;
     const int b = blockIdx.y, seg = b * P.nrays + blockIdx.x;
@@ -1613,11 +1617,14 @@ __global__ void __launch_bounds__(256) k_cone_tiles(EeParams P, const EeBeamGeom
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
     if (G.status == 0) {
-        const EeRayGeom& R = G.ray[list_cone(P, blockIdx.x)];
+        const int cone = list_cone(P, blockIdx.x);
+        const EeRayGeom& R = G.ray[cone];
+        const unsigned char* const hit = touched ? touched + (size_t)(b * P.nrays + cone) * cap : nullptr;
         const int nty = (R.sn[1] + 7) >> 3, n = nty * ((R.sn[2] + 3) >> 2);
         for (int t0 = 0; t0 < n; t0 += 256) {
             const int tile = t0 + threadIdx.x;
             bool live = tile < n;
+            const bool added = !hit || (live && hit[tile]);
             if (live) {
                 const float cy = (float)(R.so[1] + (tile % nty) * 8) + 3.5f, cz = (float)(R.so[2] + (tile / nty) * 4) + 1.5f;
 #pragma unroll
@@ -1638,7 +1645,7 @@ __global__ void __launch_bounds__(256) k_cone_tiles(EeParams P, const EeBeamGeom
                         e = fminf(e, fmaxf(lo * R.iB[k], hi * R.iB[k]));
                     }
                 }
-                if (a > e + 3.f) live = false;
+                if (a > e + 3.f || !added) live = false;
             }
             const unsigned m = __ballot_sync(FULL, live);
             int base = 0;
@@ -1870,8 +1877,11 @@ __global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / E
 template <int LANE_BLOCK>
 __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                          const EeBeamGeom* __restrict__ geoms,
-                                                         float* __restrict__ rev_grad) {
+                                                         float* __restrict__ rev_grad,
+                                                         unsigned char* __restrict__ touched, int cap) {
     const int ray = blockIdx.y, b = blockIdx.z;
+    if (const int t = blockIdx.x * LANE_BLOCK + threadIdx.x; touched && t < cap)  // none yet
+        touched[(size_t)(b * P.nrays + ray) * cap + t] = 0;
     const EeBeamGeom& G = geoms[b];
     if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
@@ -1908,7 +1918,8 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
 // before it is worked on.  Bound by the reductions into the TERMA gradient
 // (half of the time) and by latency: one 24 x 24 beam 0.428 -> 0.143 ms, 20
 // beams of 128^2 pixels 8.1 -> 2.6 ms, of which 0.247 -> 0.143 and 2.93 -> 2.64
-// by reducing into quads (quad_scatter) and loading ahead.
+// by reducing into quads (quad_scatter) and loading ahead; 0.8 where only the
+// tiles with a gradient are listed (k_cone_tiles).
 __device__ __forceinline__ void cone_T_line(const EeParams& P, const EeBeamSpec* __restrict__ specs,
                                             const EeBeamGeom* __restrict__ geoms, const float* __restrict__ rev_grad,
                                             float4* __restrict__ terma_grad, int b, int ray, int slot,
@@ -2316,7 +2327,8 @@ constexpr int GT_SMEM = 2 * GT_BUF;
 __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                                    const EeBeamGeom* __restrict__ geoms,
                                                                    const float* __restrict__ dose_grad,
-                                                                   float* __restrict__ rev_grad) {
+                                                                   float* __restrict__ rev_grad,
+                                                                   unsigned char* __restrict__ touched, int cap) {
     extern __shared__ int acc_all[];  // two fixed-point footprint boxes
     // per cone, the box of its footprint (origin l, extent n over i, tY and tZ):
     // [0] {l0 | n0 << 16, l1 | n1 << 16, l2 | n2 << 16, row stride s0} until the
@@ -2329,6 +2341,9 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams 
     __shared__ int4 s_p[EE_MAX_RAYS][5];
     __shared__ float4 s_A[EE_MAX_RAYS][3];
     __shared__ int s_list[EE_MAX_RAYS], s_n;  // cones with a box
+    // line tiles of the box's kept lines: first and end in tY and tZ, tiles per row
+    __shared__ ushort2 s_tile[EE_MAX_RAYS][2];
+    __shared__ unsigned short s_nty[EE_MAX_RAYS];
     const int b = blockIdx.z;
     const EeBeamGeom& G = geoms[b];
     if (G.status != 0 || (int)blockIdx.x >= G.tiles) return;
@@ -2416,6 +2431,12 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams 
         const int d = a == 1 ? 0 : (a == 2 ? 1 : 2);
         sp[d] = l | (max(w, 0) << 16);
         sp[12 + d] = max(0, R.so[d] - l) | max(0, R.so[d] + R.sn[d] - l) << 16;
+        if (d > 0) {
+            const int first = max(l - R.so[d], 0), end = max(min(l + max(w, 0) - R.so[d], R.sn[d]), 0);
+            const int by = d == 1 ? 3 : 2;
+            s_tile[r][d - 1] = first < end ? make_ushort2(first >> by, ((end - 1) >> by) + 1) : make_ushort2(0, 0);
+            if (d == 1) s_nty[r] = (unsigned short)((R.sn[1] + 7) >> 3);
+        }
         if (a == 0) {
             const Brick Bv = rev_store(R);
             sp[4] = Bv.sy;
@@ -2466,6 +2487,13 @@ __global__ void __launch_bounds__(GT_TX * GT_TY * GT_TZ, 5) k_gather_T(EeParams 
     int parity = 0;  // buffer of the next shared-memory cone
     for (int c = 0; c < s_n; c++) {
         const int r = s_list[c];
+        if (touched && t >= GT_TX * GT_TY * GT_TZ - 32) {  // a warp's worth of the block marks the box's line tiles
+            const int k = r >= 0 ? r : -1 - r;
+            unsigned char* const hit = touched + (size_t)(b * P.nrays + k) * cap;
+            const ushort2 ty = s_tile[k][0], tz = s_tile[k][1];
+            for (int z = tz.x + ((t & 31) >> 3); z < tz.y; z += 4)
+                for (int y = ty.x + (t & 7); y < ty.y; y += 8) hit[y + s_nty[k] * z] = 1;
+        }
         if (r >= 0) {
             // buffers alternate over the shared-memory cones: the last flush
             // of this buffer (two such cones back) was cleared by every
@@ -2780,7 +2808,7 @@ cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeB
                            cudaStream_t s) {
     if (P.mode == 1 && work.scratch) {  // exp kernel: one lane per line
         const int cap = ee_cone_tiles_cap(max_lines);
-        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, EE_LIT_READ, work.counts, work.tiles, cap);
+        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, EE_LIT_READ, nullptr, work.counts, work.tiles, cap);
         k_cone_lane<<<work.warps / EE_CONE_BLOCK_WARPS, EE_CONE_BLOCK_WARPS * 32, 0, s>>>(P, specs, geoms, terma, rev,
                                                                                         work, nbeams, cap);
         return cudaGetLastError();
@@ -2802,8 +2830,9 @@ cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeB
 }
 
 cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,
-                               int nbeams, int max_lines, cudaStream_t s) {
-    k_rev_zero<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, specs, geoms, rev_grad);
+                               const EeConeWork& work, int nbeams, int max_lines, cudaStream_t s) {
+    k_rev_zero<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, specs, geoms, rev_grad, work.touched,
+                                                                                 ee_cone_tiles_cap(max_lines));
     return cudaGetLastError();
 }
 
@@ -2829,12 +2858,14 @@ cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const E
 }
 
 cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
-                               const float* dose_grad, float* rev_grad, int nbeams, int max_tiles, cudaStream_t s) {
+                               const float* dose_grad, float* rev_grad, const EeConeWork& work, int nbeams,
+                               int max_lines, int max_tiles, cudaStream_t s) {
     const size_t smem = sizeof(float) * GT_SMEM;
     cudaError_t e = smem_attr((const void*)k_gather_T, smem);
     if (e != cudaSuccess) return e;
     dim3 grid(max(1, max_tiles), 1, nbeams);
-    k_gather_T<<<grid, GT_TX * GT_TY * GT_TZ, smem, s>>>(P, specs, geoms, dose_grad, rev_grad);
+    k_gather_T<<<grid, GT_TX * GT_TY * GT_TZ, smem, s>>>(P, specs, geoms, dose_grad, rev_grad, work.touched,
+                                                        ee_cone_tiles_cap(max_lines));
     return cudaGetLastError();
 }
 
@@ -2843,7 +2874,7 @@ cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const E
                              cudaStream_t s) {
     if (P.mode == 1 && work.scratch) {
         const int cap = ee_cone_tiles_cap(max_lines);
-        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, 0.f, work.counts, work.tiles, cap);
+        k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, 0.f, work.touched, work.counts, work.tiles, cap);
         k_cone_T_lane<<<work.warps / EE_CONE_BLOCK_WARPS, EE_CONE_BLOCK_WARPS * 32, 0, s>>>(
             P, specs, geoms, rev_grad, work, nbeams, cap, terma_grad);
         return cudaGetLastError();
