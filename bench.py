@@ -461,12 +461,11 @@ def run_reference(args, ws, rank):
 
 
 # DRAM bytes (read + write) per crop-box voxel of each stage, from ncu
-# captures of the chain kernels on eight beams of this workload (dram__bytes
-# of one call's launches / sum of V_beam = 12.37 M; k_gather_T and
-# k_cone_T_lane captured again with their current forms); roofline.traffic
-# scales the dominant stage's figure to the profiled step.
-DRAM_BYTES_PER_VBEAM = {"terma": 1.0, "cone": 251.9, "gather": 51.7, "gather_T": 102.3, "cone_T": 230.3,
-                        "terma_T": 3.5, "geometry": 0.0}
+# captures of the chain kernels on four beams of 8^2..40^2 beamlets on this
+# phantom (rate x time of one launch each / sum of V_beam = 5.76 M);
+# roofline.traffic scales the dominant stage's figure to the profiled step.
+DRAM_BYTES_PER_VBEAM = {"terma": 8.5, "cone": 109.6, "gather": 55.7, "gather_T": 65.4, "cone_T": 77.4,
+                        "terma_T": 9.1, "geometry": 0.0}
 
 
 def algorithmic_bytes(infos):

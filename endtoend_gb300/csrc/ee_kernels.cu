@@ -1,21 +1,23 @@
 // ee_kernels.cu -- sm_103a kernels of the CCCS beam-dose engine.
 //
 // Stages per beam (forward):
-//   k_terma     Siddon radiological path + polyenergetic TERMA, one thread per
-//               calc-bbox voxel, fused with the crop-box min/max reduction.
+//   k_terma     Siddon radiological path + polyenergetic TERMA of the voxels
+//               of the beam's TERMA box, with the crop-box min/max reduction.
 //               Restates CCCS/DoseCalcAlgo/cudaSiddon.cu:20-308 and the host
 //               extent scan CCCS/dosecalc-beam/nvbbRayConvolve_host.cu:429-499.
 //   k_geometry  crop box -> BEV box, findREV for every cone, affine maps
 //               (host.cu:460-499, :75-155).
-//   k_cone_*    one warp per collapsed-cone line: trilinear gather of density
-//               and TERMA along the rotated line into shared memory
-//               (nvbbRayConvolve_device.cu:11-80), then the bidirectional line
-//               convolution (device.cu:87-218): EE_KERNEL_EXP as two warp-shuffle
-//               affine scans, EE_KERNEL_TABLE as the reference walk.
+//   k_cone_*    resample of density and TERMA along the rotated lines
+//               (nvbbRayConvolve_device.cu:11-80) and the bidirectional line
+//               convolution (device.cu:87-218): EE_KERNEL_EXP one lane per line
+//               over lists of line tiles (k_cone_tiles, k_cone_lane),
+//               EE_KERNEL_TABLE window sums of two lines per warp (k_cone_tab),
+//               the step-by-step walk and the allocation-free path one warp per
+//               line (k_cone).
 //   k_gather    patient voxel <- sum over cones of the trilinear REV dose
 //               (device.cu:222-261), all cones of all beams of the batch in
 //               registers, one write per voxel.
-// Adjoint: k_gather_T (scatter), k_cone_T (reverse scans + TERMA scatter),
+// Adjoint: k_gather_T (scatter), k_cone_T_* (reverse scans + TERMA scatter),
 // k_terma_T (per-beamlet reduction).
 #include "ee_internal.h"
 #include <algorithm>
