@@ -925,12 +925,7 @@ int ee_create(int device, ee_context** out) {
         delete c;
         return fail(EE_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
     }
-    e = ee_kernel_setup();
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(c->stream);
-        delete c;
-        return fail(EE_ERR_CUDA, "kernel attributes: %s", cudaGetErrorString(e));
-    }
+    ee_kernel_setup();
     c->P.mode = EE_KERNEL_TABLE;
     c->P.ss = 1;
     *out = c;

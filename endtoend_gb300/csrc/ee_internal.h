@@ -268,8 +268,8 @@ inline int ee_cone_warps(int max_line, long long limit) {
     return (int)(n < 152 ? 152 : (n > EE_CONE_MAX_WARPS ? EE_CONE_MAX_WARPS : n)) & ~(EE_CONE_BLOCK_WARPS - 1);
 }
 inline int ee_cone_tiles_cap(int max_lines) { return max_lines / 32 + 1; }
-// kernel attributes of the current device; before the first launch on it
-cudaError_t ee_kernel_setup();
+// kernel preferences of the current device; before the first launch on it
+void ee_kernel_setup();
 // the cones write every sample that k_gather reads; without work space (exp
 // mode) the warp-per-line kernel runs
 cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* terma,

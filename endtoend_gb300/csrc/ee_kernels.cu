@@ -2760,14 +2760,12 @@ cudaError_t ee_launch_geometry(const EeParams& P, const EeBeamSpec* specs, EeBea
 // beams of 8^2..40^2 beamlets 26.9 against 27.3 ms; one engine alone loses 1 %
 // on the large batches (128 KB and more: 4 % and up; 64 KB: the three engines
 // gain nothing on the batches).
-cudaError_t ee_kernel_setup() {
+void ee_kernel_setup() {
     const void* const fn[] = {(const void*)k_terma<128>,  (const void*)k_terma<256>,  (const void*)k_terma<512>,
                               (const void*)k_cone_tiles, (const void*)k_cone_lane, (const void*)k_cone_T_lane};
-    for (const void* f : fn) {
-        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    for (const void* f : fn)
+        if (cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 40) != cudaSuccess)
+            (void)cudaGetLastError();  // a preference: the launches do not depend on it
 }
 
 static size_t cone_smem(int maxL) { return sizeof(float) * ((size_t)CONE_WARPS * 3 * maxL + 2 * EE_MAX_RADII + EE_MAX_RADII); }
