@@ -272,6 +272,12 @@ __device__ __forceinline__ Brick quads_of(const int* tn) {
     return B;
 }
 
+// Offset of row z of the quads: unsigned, since a box near the 2^31 voxels that a
+// volume may have has more quads than that.
+__device__ __forceinline__ unsigned quad_z(const Brick& Q, int z) {
+    return (unsigned)(z >> 2) * (unsigned)Q.sz + ((unsigned)(z & 3) << 4);
+}
+
 // Transpose of tri_border: scatter g with the trilinear weights, one 16-byte
 // reduction per z corner.  Corners outside the box in x or y fall on values that
 // quad_value does not read, those in z are left out.  Against a reduction per
@@ -282,16 +288,16 @@ __device__ __forceinline__ void quad_scatter(float4* v, const Brick& Q, float x,
     if (!(x > -1.f && x < (float)Q.n0 && y > -1.f && y < (float)Q.n1 && z > -1.f && z < (float)Q.n2)) return;
     const int i = __float2int_rd(x), j = __float2int_rd(y), k = __float2int_rd(z);
     const float ax = x - (float)i, ay = y - (float)j, az = z - (float)k;
-    float4* const p = v + (bk_x(i + 1) + bk_y(Q, j + 1));
+    const unsigned p = (unsigned)(bk_x(i + 1) + bk_y(Q, j + 1));
     const float g1 = ay * g, g0 = g - g1, g01 = ax * g0, g00 = g0 - g01, g11 = ax * g1, g10 = g1 - g11;
     const float bz = az, cz = 1.f - az;
-    if (k >= 0) red_v4(reinterpret_cast<float*>(p + bk_z(Q, k)), cz * g00, cz * g01, cz * g10, cz * g11);
-    if (k + 1 < Q.n2) red_v4(reinterpret_cast<float*>(p + bk_z(Q, k + 1)), bz * g00, bz * g01, bz * g10, bz * g11);
+    if (k >= 0) red_v4(reinterpret_cast<float*>(v + (p + quad_z(Q, k))), cz * g00, cz * g01, cz * g10, cz * g11);
+    if (k + 1 < Q.n2) red_v4(reinterpret_cast<float*>(v + (p + quad_z(Q, k + 1))), bz * g00, bz * g01, bz * g10, bz * g11);
 }
 
 // The gradient of voxel (x, y, z) of the box from its four cells.
 __device__ __forceinline__ float quad_value(const float4* __restrict__ v, const Brick& Q, int x, int y, int z) {
-    const float4* const p = v + bk_z(Q, z);
+    const float4* const p = v + quad_z(Q, z);
     const int x0 = bk_x(x), x1 = bk_x(x + 1), y0 = bk_y(Q, y), y1 = bk_y(Q, y + 1);
     return (__ldg(&p[x1 + y1].x) + __ldg(&p[x0 + y1].y)) + (__ldg(&p[x1 + y0].z) + __ldg(&p[x0 + y0].w));
 }
