@@ -618,7 +618,7 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         if (ee_debug_poison()) EE_CUDA(cudaMemsetAsync(c->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
         EE_CUDA(cudaMemsetAsync(c->terma_grad.p, 0, sizeof(float4) * D.quads, s));
         float4* const tg = c->terma_grad.p - D.q0;  // a beam's quads at its q_off
-        EE_CUDA(ee_launch_rev_zero(c->P, dsp, dge, c->rev.p, work, nb, D.max_lines, s));
+        EE_CUDA(ee_launch_rev_zero(c->P, dge, c->rev.p, work, nb, D.max_lines, s));
         EE_CUDA(staged(c, EE_STAGE_GATHER_T, 1, [&] {
             return ee_launch_gather_T(c->P, dsp, dge, dgrad, c->rev.p, work, nb, D.max_lines, D.max_tiles, s);
         }));
@@ -892,7 +892,7 @@ cudaError_t plan_enqueue(ee_plan* pl, cudaStream_t s) {
         if (ee_debug_poison()) PL(cudaMemsetAsync(pl->rev.p, 0xFF, sizeof(float) * D.rev_total, s));
         PL(cudaMemsetAsync(pl->terma_grad.p, 0, sizeof(float4) * D.quads, s));
         float4* const tg = pl->terma_grad.p - D.q0;  // a beam's quads at its q_off
-        PL(ee_launch_rev_zero(P, dsp, dge, pl->rev.p, pl->work, nb, D.max_lines, s));
+        PL(ee_launch_rev_zero(P, dge, pl->rev.p, pl->work, nb, D.max_lines, s));
         PL(ee_launch_gather_T(P, dsp, dge, pl->d_grad, pl->rev.p, pl->work, nb, D.max_lines, D.max_tiles, s));
         PL(ee_launch_cone_T(P, dsp, dge, pl->rev.p, pl->work, tg, nb, D.max_lines, D.max_line, s));
         PL(ee_launch_terma_T(P, dsp, dge, pl->unit.p, pl->bl_idx.p, tg, pl->d_fgrad, nb, D.max_tvol, s));

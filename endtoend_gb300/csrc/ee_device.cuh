@@ -4,6 +4,7 @@
 // the beamlet lookup and the polyenergetic TERMA of one point.
 #pragma once
 #include "ee_internal.h"
+#include "ee_lines.cuh"
 #include <cfloat>
 
 namespace {
@@ -23,20 +24,6 @@ __device__ __forceinline__ float key2f(int k) { return __int_as_float(k >= 0 ? k
 __device__ __forceinline__ float snap_ceilf(float v) {
     float r = rintf(v);
     return fabsf(v - r) <= 1e-3f ? r : ceilf(v);
-}
-
-struct f3 {
-    float x, y, z;
-};
-__device__ __forceinline__ f3 mk(float x, float y, float z) { return {x, y, z}; }
-__device__ __forceinline__ f3 operator+(f3 a, f3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ f3 operator-(f3 a, f3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ f3 operator*(f3 a, float s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ f3 ld3(const float* p) { return {p[0], p[1], p[2]}; }
-__device__ __forceinline__ f3 mv(const float* M, f3 v) {
-    return {M[0] * v.x + M[1] * v.y + M[2] * v.z, M[3] * v.x + M[4] * v.y + M[5] * v.z,
-            M[6] * v.x + M[7] * v.y + M[8] * v.z};
 }
 
 // tex3D<float> with linear filtering, unnormalised coordinates and border

@@ -288,8 +288,8 @@ cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const E
                              cudaStream_t s);
 // zeros on every line's segment of a chunk's REV gradient arena (before
 // ee_launch_gather_T; the forward cone kernels zero their own arena)
-cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,
-                               const EeConeWork& work, int nbeams, int max_lines, cudaStream_t s);
+cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamGeom* geoms, float* rev_grad, const EeConeWork& work,
+                               int nbeams, int max_lines, cudaStream_t s);
 // test option: EE_DEBUG_POISON=1 fills scratch with NaN where the engine
 // relies on its kernels, not on a clear, to write every sample it reads
 bool ee_debug_poison();

@@ -385,14 +385,6 @@ __device__ void kept_part(const EeBeamGeom& G, EeRayGeom& R, bool bounded) {
     R.nlines = R.sn[1] * R.sn[2];
 }
 
-// The least of a cone's lit forms at lateral REV point (tY, tZ).
-__device__ __forceinline__ float lit_form(const EeRayGeom& R, float tY, float tZ) {
-    float f = 1e30f;
-#pragma unroll
-    for (int k = 0; k < 4; k++) f = fminf(f, fmaf(R.lit[k][0], tY, fmaf(R.lit[k][1], tZ, R.lit[k][2])));
-    return f;
-}
-
 // Lit form k of the cone as an affine form of the crop-box-relative patient
 // index (dx, dy, dz): >= 0 where one of the four lines around the voxel can be
 // lit (a cell per axis added).
@@ -537,68 +529,6 @@ __global__ void k_geometry(EeParams P, const EeBeamSpec* __restrict__ specs, EeB
 
 
 // ------------------------------------------------------- cone: gather ----
-// Samples of REV line (tY, tZ) that can be valid: the line's intersection
-// with the BEV crop box and the calc bbox (both convex, so one segment),
-// widened by one sample for rounding.  Outside it every sample is a sentinel
-// (-3 outside the BEV box, -2 outside the bbox, device.cu:51-70) and its dose
-// is zero, so neither the gather nor the scans visit it.
-__device__ __forceinline__ void line_segment(const EeParams& P, const EeBeamGeom& G, const EeRayGeom& R, int tY,
-                                             int tZ, int L, int& i0, int& n) {
-    const f3 bl = ld3(R.B0) + ld3(R.By) * (float)tY + ld3(R.Bz) * (float)tZ;
-    const f3 gl = ld3(R.G0) + ld3(R.Gy) * (float)tY + ld3(R.Gz) * (float)tZ;
-    const float c[6] = {bl.x, bl.y, bl.z, gl.x, gl.y, gl.z};
-    const float im[6] = {R.iB[0], R.iB[1], R.iB[2], R.iG[0], R.iG[1], R.iG[2]};
-    const float lo[6] = {0.f, 0.f, 0.f, (float)P.bb0[0], (float)P.bb0[1], (float)P.bb0[2]};
-    const float hi[6] = {(float)G.bev[0], (float)G.bev[1], (float)G.bev[2], (float)(P.bb0[0] + P.bbs[0]),
-                         (float)(P.bb0[1] + P.bbs[1]), (float)(P.bb0[2] + P.bbs[2])};
-    float a = 0.f, b = (float)(L - 1);
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        if (im[k] == 0.f) {
-            if (c[k] < lo[k] - 1e-3f || c[k] > hi[k] + 1e-3f) { n = 0; i0 = 0; return; }
-        } else {
-            float t0 = (lo[k] - c[k]) * im[k], t1 = (hi[k] - c[k]) * im[k];
-            a = fmaxf(a, fminf(t0, t1));
-            b = fminf(b, fmaxf(t0, t1));
-        }
-    }
-    if (!(a <= b + 2.f)) { n = 0; i0 = 0; return; }
-    i0 = max(R.so[0], (int)floorf(a) - 1);
-    int i1 = min(R.so[0] + R.sn[0] - 1, (int)ceilf(b) + 1);
-    n = max(0, i1 - i0 + 1);
-}
-
-// Samples of a REV line that k_gather can read (and k_gather_T can add to):
-// k_gather visits voxels within 2 BEV voxels of the crop box and reads the
-// REV cells within one REV step (per axis) of each voxel's REV point, i.e.
-// within sum_k |B[a][k]| BEV units per axis a.  So the line's intersection
-// with the crop box dilated by 2 + sum_k |B[a][k]| (+0.05, +1 sample each
-// side) holds every sample either kernel touches; samples outside it are
-// never read and need no zero.  z1 < z0: none.
-__device__ __forceinline__ void line_read_span(const EeBeamGeom& G, const EeRayGeom& R, int tY, int tZ, int L,
-                                               int& z0, int& z1) {
-    const f3 bl = ld3(R.B0) + ld3(R.By) * (float)tY + ld3(R.Bz) * (float)tZ;
-    const float c[3] = {bl.x, bl.y, bl.z};
-    float a = 0.f, b = (float)(L - 1);
-    z0 = 0;
-    z1 = -1;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const float D = 2.05f + fabsf(R.Bx[k]) + fabsf(R.By[k]) + fabsf(R.Bz[k]);
-        const float lo = -D, hi = (float)G.bev[k] + D, im = R.iB[k];
-        if (im == 0.f) {
-            if (c[k] < lo || c[k] > hi) return;
-        } else {
-            const float t0 = (lo - c[k]) * im, t1 = (hi - c[k]) * im;
-            a = fmaxf(a, fminf(t0, t1));
-            b = fminf(b, fmaxf(t0, t1));
-        }
-    }
-    if (!(a <= b + 2.f)) return;
-    z0 = max(R.so[0], (int)floorf(a) - 1);
-    z1 = min(R.so[0] + R.sn[0] - 1, (int)ceilf(b) + 1);
-}
-
 // Line `line` of a cone's kept part (R.nlines).
 __device__ __forceinline__ void kept_line(const EeRayGeom& R, int line, int& tY, int& tZ) {
     tZ = line / R.sn[1];
@@ -623,18 +553,18 @@ __device__ __forceinline__ void zero_outside_segment(float* out, const Brick& Bv
 __device__ __forceinline__ void gather_line(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
                                             const EeRayGeom& R, const float* __restrict__ terma_b, int tY, int tZ,
                                             int i0, int n, int lane, float* rho, float* T, int stride = 32) {
-    const f3 bl = ld3(R.B0) + ld3(R.By) * (float)tY + ld3(R.Bz) * (float)tZ;
-    const f3 gl = ld3(R.G0) + ld3(R.Gy) * (float)tY + ld3(R.Gz) * (float)tZ;
+    const f3 bl = line_point(R.B0, R.By, R.Bz, (float)tY, (float)tZ);
+    const f3 gl = line_point(R.G0, R.Gy, R.Gz, (float)tY, (float)tZ);
     const f3 bx = ld3(R.Bx), gx = ld3(R.Gx);
     const float bsx = (float)G.bev[0], bsy = (float)G.bev[1], bsz = (float)G.bev[2];
     const float b0x = (float)P.bb0[0], b0y = (float)P.bb0[1], b0z = (float)P.bb0[2];
     const float b1x = (float)(P.bb0[0] + P.bbs[0]), b1y = (float)(P.bb0[1] + P.bbs[1]), b1z = (float)(P.bb0[2] + P.bbs[2]);
     for (int k = lane; k < n; k += stride) {
         const float fi = (float)(i0 + k);
-        f3 bev = bl + bx * fi;
+        f3 bev = along(bl, bx, fi);
         float r = -3.f, t = 0.f;
         if (!(bev.x < 0.f || bev.y < 0.f || bev.z < 0.f || bev.x >= bsx || bev.y >= bsy || bev.z >= bsz)) {
-            f3 g = gl + gx * fi;
+            f3 g = along(gl, gx, fi);
             if (g.x < b0x || g.x >= b1x || g.y < b0y || g.y >= b1y || g.z < b0z || g.z >= b1z) {
                 r = -2.f;
             } else {
@@ -878,77 +808,8 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone(EeParams P, const EeBe
     for (int k = lane; k < n; k += 32) out[bk_x(i0 + k)] = D[k];
 }
 
-struct LineFrame {
-    f3 gl, gx;  // patient voxel index of sample 0, and its step per sample
-};
-
-__device__ __forceinline__ f3 sample_point(const LineFrame& F, int i) { return F.gl + F.gx * (float)i; }
-
 __device__ __forceinline__ float rho_at(const EeParams& P, f3 g) {
     return tex3D<float>(P.dens_tex, g.x + 0.5f, g.y + 0.5f, g.z + 0.5f);
-}
-
-// What a lane needs of its line.  [i0, i1]: the samples inside the BEV crop
-// box and the calc bbox by the reference's own tests (device.cu:51-70).  Every
-// test is a comparison of an affine function of i, which stays monotone in
-// FP32, so the samples that pass are one interval: the analytic segment
-// trimmed at its ends by the tests themselves, and no sample in between needs
-// them again.  [q0, q1]: the quads of [i0, i1] that hold the samples whose
-// TERMA corners can lie in the field (field_forms); q1 < q0: no such sample,
-// so neither dose nor TERMA gradient.
-struct LaneSpan {
-    int i0, i1, q0, q1;
-};
-
-__device__ __forceinline__ LaneSpan lane_span(const EeParams& P, const EeBeamSpec& S, const EeBeamGeom& G,
-                                              const EeRayGeom& R, int tY, int tZ, LineFrame& F) {
-    const float fy = (float)tY, fz = (float)tZ;
-    F.gl = ld3(R.G0) + ld3(R.Gy) * fy + ld3(R.Gz) * fz;
-    F.gx = ld3(R.Gx);
-    LaneSpan s{0, -1, 0, -1};
-    if (lit_form(R, fy, fz) < 0.f) return s;
-    int n;
-    line_segment(P, G, R, tY, tZ, R.rev[0], s.i0, n);
-    s.i1 = s.i0 + n - 1;
-    if (n <= 0) return s;
-    // field span: the four sides, raised by more than their rounding, cut the
-    // line to one interval.  The forms hold in front of the source; beamlet_of
-    // takes |depth|, so a segment that does not stay in front of it is not
-    // restricted
-    float lo = -1e9f, hi = 1e9f;
-    const float pr = fmaf(R.front[2], fy, fmaf(R.front[3], fz, R.front[1]));
-    const bool front = fminf(fmaf(R.front[0], (float)s.i0, pr), fmaf(R.front[0], (float)s.i1, pr)) > 1e-2f * S.isodist;
-    if (front) {
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float al = R.side[k][0], be = fmaf(R.side[k][2], fy, fmaf(R.side[k][3], fz, R.side[k][1]));
-            if (fabsf(al) < 1e-20f) {
-                if (be < 0.f) { lo = 1e9f; hi = -1e9f; }
-            } else {
-                const float t = fminf(fmaxf(__fdividef(-be, al), -1e9f), 1e9f);
-                if (al > 0.f) lo = fmaxf(lo, t);
-                else hi = fminf(hi, t);
-            }
-        }
-    }
-    const int f0 = max(s.i0, (int)ceilf(lo - 0.01f)), f1 = min(s.i1, (int)floorf(hi + 0.01f));
-    if (f0 > f1) return s;
-    const f3 bl = ld3(R.B0) + ld3(R.By) * fy + ld3(R.Bz) * fz, bx = ld3(R.Bx);
-    auto valid = [&](int i) {
-        const f3 bev = bl + bx * (float)i, g = sample_point(F, i);
-        return !(bev.x < 0.f || bev.y < 0.f || bev.z < 0.f || bev.x >= (float)G.bev[0] || bev.y >= (float)G.bev[1] ||
-                 bev.z >= (float)G.bev[2] || g.x < (float)P.bb0[0] || g.x >= (float)(P.bb0[0] + P.bbs[0]) ||
-                 g.y < (float)P.bb0[1] || g.y >= (float)(P.bb0[1] + P.bbs[1]) || g.z < (float)P.bb0[2] ||
-                 g.z >= (float)(P.bb0[2] + P.bbs[2]));
-    };
-#pragma unroll 1
-    while (s.i0 <= s.i1 && !valid(s.i0)) s.i0++;
-#pragma unroll 1
-    while (s.i1 > s.i0 && !valid(s.i1)) s.i1--;
-    if (max(f0, s.i0) > min(f1, s.i1)) return s;
-    s.q0 = max(f0, s.i0) >> 2;
-    s.q1 = min(f1, s.i1) >> 2;
-    return s;
 }
 
 // ------------------------------------- cone: exact table scan, O(n nr) ----
@@ -1871,14 +1732,14 @@ __global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / E
     });
 }
 
-// Zero the samples of the chunk's REV gradient arena that the adjoint cone
-// reads, before k_gather_T adds into it: the quads of [i0, i1] of every line
-// with a field span.  k_gather_T also adds into the rest; those cells are
-// never read, so they need no zero.  A warp's 16-byte stores cover two whole
-// bricks.
+// Zero the samples of the chunk's REV gradient arena that the adjoint cones
+// may read, before k_gather_T adds into it: the quads of each line's
+// line_clear_span, which holds the samples that the cones find for themselves
+// whatever their own end tests decide (the arena holds the forward's dose
+// before that).  k_gather_T also adds into the rest; those cells are never
+// read, so they need no zero.  A warp's 16-byte stores cover two whole bricks.
 template <int LANE_BLOCK>
-__global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBeamSpec* __restrict__ specs,
-                                                         const EeBeamGeom* __restrict__ geoms,
+__global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBeamGeom* __restrict__ geoms,
                                                          float* __restrict__ rev_grad,
                                                          unsigned char* __restrict__ touched, int cap) {
     const int ray = blockIdx.y, b = blockIdx.z;
@@ -1890,18 +1751,7 @@ __global__ void __launch_bounds__(LANE_BLOCK) k_rev_zero(EeParams P, const EeBea
     int tY, tZ;
     if (!lane_line(R, blockIdx.x * LANE_BLOCK + threadIdx.x, tY, tZ)) return;
     int i0, i1;
-    if (P.mode == EE_KERNEL_EXP) {
-        LineFrame F;
-        const LaneSpan s = lane_span(P, specs[b], G, R, tY, tZ, F);
-        if (s.q1 < s.q0) return;
-        i0 = s.i0;
-        i1 = s.i1;
-    } else {
-        if (lit_form(R, (float)tY, (float)tZ) < 0.f) return;
-        int n;
-        line_segment(P, G, R, tY, tZ, R.rev[0], i0, n);
-        i1 = i0 + n - 1;
-    }
+    line_clear_span(P, G, R, tY, tZ, i0, i1);
     float* row = rev_grad + G.arena_off + R.offset + rev_line(rev_store(R), tY, tZ);
     for (int ib = i0 & ~3; ib <= i1; ib += 4)
         *reinterpret_cast<float4*>(row + bk_x(ib)) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -2104,13 +1954,12 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
     }
     __syncwarp();
     // transpose of the REV TERMA resample
-    const f3 gl = ld3(R.G0) + ld3(R.Gy) * (float)tY + ld3(R.Gz) * (float)tZ;
-    const f3 gx = ld3(R.Gx);
+    const LineFrame F{line_point(R.G0, R.Gy, R.Gz, (float)tY, (float)tZ), ld3(R.Gx)};
     float4* tg = terma_grad + S.q_off;
     for (int k = lane; k < n; k += 32) {
         float v = Tb[k];
         if (rho[k] < 0.f || v == 0.f) continue;
-        f3 gp = gl + gx * (float)(i0 + k);
+        f3 gp = sample_point(F, i0 + k);
         quad_scatter(tg, quads_of(S.tn), gp.x - (float)S.t0[0], gp.y - (float)S.t0[1],
                            gp.z - (float)S.t0[2], v);
     }
@@ -2829,9 +2678,9 @@ cudaError_t ee_launch_cone(const EeParams& P, const EeBeamSpec* specs, const EeB
     return cudaGetLastError();
 }
 
-cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, float* rev_grad,
-                               const EeConeWork& work, int nbeams, int max_lines, cudaStream_t s) {
-    k_rev_zero<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, specs, geoms, rev_grad, work.touched,
+cudaError_t ee_launch_rev_zero(const EeParams& P, const EeBeamGeom* geoms, float* rev_grad, const EeConeWork& work,
+                               int nbeams, int max_lines, cudaStream_t s) {
+    k_rev_zero<128><<<dim3(grid1(max_lines, 128), P.nrays, nbeams), 128, 0, s>>>(P, geoms, rev_grad, work.touched,
                                                                                  ee_cone_tiles_cap(max_lines));
     return cudaGetLastError();
 }
