@@ -1312,6 +1312,11 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
         pl->rev_max = std::max(pl->rev_max, D.rev_total);
     }
     pl->starts.push_back(nbeams);
+    for (size_t k = 0; k < pl->dims.size(); k++)
+        for (int b = pl->starts[k]; b < pl->starts[k + 1]; b++) {
+            pl->specs[b].plan_lines = pl->dims[k].max_lines;
+            pl->specs[b].plan_line = pl->dims[k].max_line;
+        }
     pl->nfl = total_fluence(beams, nbeams);
     EE_CUDA(pl->d_specs.ensure(nbeams));
     EE_CUDA(pl->d_geoms.ensure(nbeams));

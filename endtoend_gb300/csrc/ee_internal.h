@@ -104,10 +104,19 @@ struct EeBeamSpec {
     // plan_cap == 0: the arena is sized after the geometry read-back
     long long plan_off;
     long long plan_cap;
+    int plan_lines;  // line slots per cone that the planned tile lists hold
+    int plan_line;   // samples per line that the planned cone scratch holds
     // element offset of this beam's dose (and dose-gradient) volume: grouped
     // outputs of the request server; 0 otherwise
     long long out_off;
 };
+
+// Whether a beam's sizes, as the device finds them, fit what was planned for it.
+// The lists and the scratch are indexed by the device's own sizes, so a bound
+// that failed would be written past; such a beam gets a status instead.
+inline __host__ __device__ bool ee_plan_holds(const EeBeamSpec& S, long long store, int max_lines, int max_line) {
+    return S.plan_cap == 0 || (store <= S.plan_cap && max_lines <= S.plan_lines && max_line <= S.plan_line);
+}
 
 // Per-cone geometry of one beam, computed on the device.
 struct EeRayGeom {

@@ -523,7 +523,7 @@ __global__ void k_geometry(EeParams P, const EeBeamSpec* __restrict__ specs, EeB
         if (all > 2147483647ll) G.status = 4;  // EE_ERR_REV_SIZE
         G.max_line = ml;
         G.max_lines = mls;
-        if (G.arena_cap > 0 && off > G.arena_cap) G.status = 8;
+        if (!ee_plan_holds(S, off, mls, ml)) G.status = 8;  // EE_ERR_CAPACITY
     }
 }
 
