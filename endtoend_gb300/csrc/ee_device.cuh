@@ -341,6 +341,11 @@ __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
             alpha = next;
             return true;
         };
+        // a segment below the cut is fetched with the others but not added: the
+        // density there may be infinite, and 0 times that is not 0
+        auto add = [&](float len, float rho) {
+            if (len > 0.f) rpl = fmaf(len, rho, rpl);
+        };
         float l0 = 0.f, r0 = 0.f, l1 = 0.f, r1 = 0.f;
         f3 at;
         for (;;) {
@@ -348,15 +353,16 @@ __device__ float siddon_rpl(const EeParams& P, f3 vox, f3 src, bool& iter_cap) {
             if (!segment(len, at)) break;
             l0 = len;
             r0 = tex3D<float>(P.dens_tex, at.x, at.y, at.z);
-            rpl = fmaf(l1, r1, rpl);
+            add(l1, r1);
             l1 = 0.f;
             if (!segment(len, at)) break;
             l1 = len;
             r1 = tex3D<float>(P.dens_tex, at.x, at.y, at.z);
-            rpl = fmaf(l0, r0, rpl);
+            add(l0, r0);
             l0 = 0.f;
         }
-        rpl = fmaf(l1, r1, fmaf(l0, r0, rpl));
+        add(l0, r0);
+        add(l1, r1);
         if (iter >= 5000) iter_cap = true;
     }
     return rpl;
