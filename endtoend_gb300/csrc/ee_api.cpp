@@ -156,28 +156,26 @@ struct ConeBufs {
     DevBuf<float4> scratch;
     DevBuf<int> counts, tiles;
     DevBuf<unsigned char> touched;
-    static size_t scratch_size(int max_line, long long limit) {
-        return (size_t)64 * ee_cone_quads(max_line) * ee_cone_warps(max_line, limit);
-    }
-    bool fits(int max_line, long long segments, long long ntiles, long long limit) const {
-        return scratch.n >= scratch_size(max_line, limit) && counts.n >= (size_t)(1 + segments) &&
+    static size_t scratch_size(int max_line, int warps) { return (size_t)64 * ee_cone_quads(max_line) * warps; }
+    bool fits(int max_line, long long segments, long long ntiles, int warps) const {
+        return scratch.n >= scratch_size(max_line, warps) && counts.n >= (size_t)(1 + segments) &&
                tiles.n >= (size_t)ntiles && touched.n >= (size_t)ntiles;
     }
-    cudaError_t ensure(int max_line, long long segments, long long ntiles, long long limit) {
-        cudaError_t e = scratch.ensure(scratch_size(max_line, limit));
+    cudaError_t ensure(int max_line, long long segments, long long ntiles, int warps) {
+        cudaError_t e = scratch.ensure(scratch_size(max_line, warps));
         if (e == cudaSuccess) e = counts.ensure((size_t)(1 + segments));
         if (e == cudaSuccess) e = tiles.ensure((size_t)ntiles);
         if (e == cudaSuccess) e = touched.ensure((size_t)ntiles);
         return e;
     }
-    EeConeWork work(int max_line, long long limit) const {
+    EeConeWork work(int max_line, int warps) const {
         EeConeWork w;
         w.scratch = scratch.p;
         w.counts = counts.p;
         w.tiles = tiles.p;
         w.touched = touched.p;
         w.quads = ee_cone_quads(max_line);
-        w.warps = ee_cone_warps(max_line, limit);
+        w.warps = warps;
         return w;
     }
     long long bytes() const { return 16ll * scratch.n + 4ll * (counts.n + tiles.n) + touched.n; }
@@ -570,11 +568,12 @@ int pipeline(ee_context* c, const PipeArgs& A) {
         int max_line = 1;
         long long segs = 1, ntiles = 1;
         cone_sizes(c->P.nrays, starts, dims, max_line, segs, ntiles);
-        if (!c->cone.fits(max_line, segs, ntiles, c->max_batch_bytes)) {
+        const int warps = ee_cone_warps(max_line, c->max_batch_bytes, 4 * rev_max);
+        if (!c->cone.fits(max_line, segs, ntiles, warps)) {
             EE_CUDA(cudaStreamSynchronize(s));  // queued kernels may still use the old buffers
-            EE_CUDA(c->cone.ensure(max_line, segs, ntiles, c->max_batch_bytes));
+            EE_CUDA(c->cone.ensure(max_line, segs, ntiles, warps));
         }
-        work = c->cone.work(max_line, c->max_batch_bytes);
+        work = c->cone.work(max_line, warps);
     }
 
     // ---- forward, chunk by chunk
@@ -1326,8 +1325,9 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
         int max_line = 1;
         long long segs = 1, ntiles = 1;
         cone_sizes(c->P.nrays, pl->starts, pl->dims, max_line, segs, ntiles);
-        EE_CUDA(pl->cone.ensure(max_line, segs, ntiles, c->max_batch_bytes));
-        pl->work = pl->cone.work(max_line, c->max_batch_bytes);
+        const int warps = ee_cone_warps(max_line, c->max_batch_bytes, 4 * pl->rev_max);
+        EE_CUDA(pl->cone.ensure(max_line, segs, ntiles, warps));
+        pl->work = pl->cone.work(max_line, warps);
     }
     if (pl->adjoint) {
         EE_CUDA(pl->unit.ensure(pl->tvol_total));

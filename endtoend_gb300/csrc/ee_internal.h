@@ -271,9 +271,14 @@ struct EeConeWork {
 };
 constexpr int EE_CONE_BLOCK_WARPS = 2, EE_CONE_SM_WARPS = 24, EE_CONE_MAX_WARPS = 152 * EE_CONE_SM_WARPS;
 inline int ee_cone_quads(int max_line) { return (max_line + 3) / 4 + 2; }
-// resident warps whose scratch stays within a quarter of `limit` bytes
-inline int ee_cone_warps(int max_line, long long limit) {
-    const long long per = 1024ll * ee_cone_quads(max_line), n = limit / 4 / per;
+// Resident warps whose scratch stays within a quarter of `limit` bytes.  A beam
+// whose arena alone exceeds the other three quarters is taken all the same;
+// `arena`: bytes of the largest chunk's, and then the scratch may be as large.
+// With the quarter in that case too, a limit of 1 MB left one warp per SM: a 24 x
+// 24 beam on 200 x 200 x 160, dose and adjoint, 1.91 ms, so 0.62 (0.61 with a
+// limit of 512 MB).
+inline int ee_cone_warps(int max_line, long long limit, long long arena) {
+    const long long per = 1024ll * ee_cone_quads(max_line), n = (arena > limit / 4 * 3 ? arena : limit / 4) / per;
     return (int)(n < 152 ? 152 : (n > EE_CONE_MAX_WARPS ? EE_CONE_MAX_WARPS : n)) & ~(EE_CONE_BLOCK_WARPS - 1);
 }
 inline int ee_cone_tiles_cap(int max_lines) { return max_lines / 32 + 1; }
