@@ -321,20 +321,23 @@ __device__ __forceinline__ f3 bl_rev_point(const BlGrid& G, const BlPillar& Q, c
 // one add per warp or so and not one per sample.  Bound by the instructions of
 // the tests.  A thread per REV sample (0.2 % of them are in a beamlet) took
 // 272 us per direction of about 110 beamlets on 200 x 200 x 160 at 2 mm, a warp
-// per unit 27 us; this takes 5.2 us.
+// per unit 27 us; this takes 5.2 us.  `slices` warps share the candidates of 32
+// units (ee_bl_source_slices).
 constexpr int BL_SRC_WARPS = 4, BL_SRC_BUF = 128;
 
 __global__ void __launch_bounds__(BL_SRC_WARPS * 32)
     k_bl_sources(const EeBeamSpec* __restrict__ spec, BlGrid G, const BlPillar* __restrict__ pil,
-                 const BlRayDev* __restrict__ rays, BlQueue W, float4* __restrict__ band, int* __restrict__ status) {
+                 const BlRayDev* __restrict__ rays, BlQueue W, int slices, float4* __restrict__ band,
+                 int* __restrict__ status) {
     // per warp and unit: box origin (tX, tY, tZ), sizes along tX and tY, first candidate
     __shared__ int s_unit[BL_SRC_WARPS][6][32];
     __shared__ int s_v[BL_SRC_WARPS][BL_SRC_BUF], s_line[BL_SRC_WARPS][BL_SRC_BUF];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int u0 = (blockIdx.y * BL_SRC_WARPS + warp) * 32, unit = u0 + lane, j = blockIdx.x, r = blockIdx.z;
+    const int part = blockIdx.y * BL_SRC_WARPS + warp, slice = part % slices;
+    const int u0 = part / slices * 32, unit = u0 + lane, j = blockIdx.x, r = blockIdx.z;
     const BlRayDev& R = rays[r];
     const BlPillar& Q = pil[j];
-    if (unit == 0) {
+    if (unit == 0 && slice == 0) {
         float n0 = -R.MK[7], n1 = R.MK[1];  // n = (-e_tY, e_tZ), e the pillar axis
         const float l = sqrtf(n0 * n0 + n1 * n1);
         if (l > 1e-3f) { n0 /= l; n1 /= l; }
@@ -416,11 +419,12 @@ __global__ void __launch_bounds__(BL_SRC_WARPS * 32)
         nv = nl = 0;
         __syncwarp();
     };
-    for (int k0 = 0; k0 < total; k0 += 32) {
+    const int per = ((total + slices - 1) / slices + 31) & ~31, stop = min(total, (slice + 1) * per);
+    for (int k0 = slice * per; k0 < stop; k0 += 32) {
         const int k = k0 + lane;
         bool take = false, fresh = false;
         int v = 0, line = 0;
-        if (k < total) {
+        if (k < stop) {
             int u = 0;  // the last unit that starts at or before k (units without candidates share a start)
 #pragma unroll
             for (int o = 16; o; o >>= 1)
@@ -1439,8 +1443,9 @@ int ee_beamlet_run(const EeParams& P, const EeRayConst* rays, cudaStream_t s, vo
             Qu.nlines = W.lines.p + 1;
             Qu.src = W.queue.p;
             Qu.line = W.line_list.p;
-            k_bl_sources<<<dim3(m, pd[1] / (32 * BL_SRC_WARPS) + 1, ng), BL_SRC_WARPS * 32, 0, s>>>(
-                W.spec.p, G, W.pil.p, W.rays.p, Qu, W.band.p, W.status.p);
+            const int slices = ee_bl_source_slices(nsrc / m / (pd[1] + 2.0), (long long)m * ng * (pd[1] / 32 + 1));
+            k_bl_sources<<<dim3(m, (pd[1] / 32 + 1) * slices / BL_SRC_WARPS + 1, ng), BL_SRC_WARPS * 32, 0, s>>>(
+                W.spec.p, G, W.pil.p, W.rays.p, Qu, slices, W.band.p, W.status.p);
             BL_CUDA(cudaGetLastError());
             k_bl_terma<<<152 * 8, 256, 0, s>>>(P, W.spec.p, G, W.pil.p, W.rays.p, W.fluence.p, Qu, W.status.p);
             BL_CUDA(cudaGetLastError());

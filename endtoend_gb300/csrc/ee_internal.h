@@ -326,6 +326,20 @@ struct EeBeamletOptions {
     int max_rev[3];       // REV size limit that triggers re-batching (argparser.h:29: 500^3)
     long long scratch_bytes = 0;  // the context's scratch budget: directions whose REV arrays share a launch
 };
+// Warps that share the candidate samples of 32 units of a pillar's depth
+// (k_bl_sources).  `area` cells of footprint are about 3 area candidates per
+// unit, so as many steps of a warp for its 32 units; `warps`: the launch's
+// without a split.  More than 64 steps are split, and down to 8 (the boxes cost
+// about as much) while the launch has fewer than 16 warps per SM.  One beamlet of
+// 8 cm on 64^3 at 2.5 mm: 53 ms with one warp per 32 units, 3.5 split (a thread
+// per sample of the packed grid: 10.1); of 4 cm on 200 x 200 x 160 at 2 mm, a
+// direction per launch: 303 ms, 7.8 (14.5).  A batch's usual hundred beamlets of
+// a voxel or two stay whole.
+inline int ee_bl_source_slices(double area, long long warps) {
+    const double steps = 3.0 * area;
+    const double few = std::fmin(steps / 8, 152.0 * 16.0 / (double)warps), n = std::fmax(steps / 64, few);
+    return n < 1 ? 1 : (n > 4096 ? 4096 : (int)n);
+}
 int ee_beamlet_run(const EeParams& P, const EeRayConst* rays, cudaStream_t s, void** ws, const EeBeamletOptions& opt,
                    const ee_beam& beam, const EeBeamSpec& S, const float* fluence_host, float thresh, ee_csr* out);
 void ee_beamlet_free(void* ws);
