@@ -1393,16 +1393,20 @@ int ee_beamlet_run(const EeParams& P, const EeRayConst* rays, cudaStream_t s, vo
             }
             nsrc += (w[0] + 2.0) * (w[1] + 2.0) * (pd[1] + 2.0);
         }
-        // directions in groups whose REV arrays fit the scratch budget
+        // directions in groups whose buffers fit the scratch budget: the REV
+        // arrays, flags and bits of the lines, the lists of sources and lines
         for (int r0 = 0; r0 < nrays;) {
             int r1 = r0;
-            long long samples = 0, ints = 2, nlines = 0, maxL = 1;
+            long long samples = 0, ints = 2, nlines = 0, maxL = 1, bytes = 0;
             for (; r1 < nrays; r1++) {
                 const int* z = revs[k][r1].size;
-                const long long lines = (long long)z[1] * z[2], n = lines * z[0];
-                if (r1 > r0 && (samples + n) * (long long)sizeof(float) > opt.scratch_bytes) break;
+                const long long lines = (long long)z[1] * z[2], n = lines * z[0], flags = lines * (1 + (z[0] + 31) / 32);
+                const long long more = 4 * (n + flags) + (long long)sizeof(int2) * ((long long)nsrc + 1 + lines) +
+                                       (long long)sizeof(BlRayDev) + (long long)sizeof(float4) * m;
+                if (r1 > r0 && bytes + more > opt.scratch_bytes) break;
+                bytes += more;
                 samples += n;
-                ints += lines * (1 + (z[0] + 31) / 32);
+                ints += flags;
                 nlines += lines;
                 maxL = std::max<long long>(maxL, z[0]);
             }
