@@ -418,7 +418,10 @@ struct ChunkDims {
     long long rev_total = 0, max_tvol = 1;
     long long q0 = 0, quads = 0;  // TERMA gradient: first quad of the chunk's first beam, and their number
     int max_line = 1, max_lines = 1, max_rows = 1, max_tiles = 1;
-    long long bytes() const { return 4 * rev_total + 16 * quads; }
+    // bytes with one more beam of such sizes, as the chunk's beam number `beams`
+    long long bytes_with(long long rev, long long quad, int lines, int lists, int beams) const {
+        return ee_chunk_bytes(rev_total + rev, quads + quad, (long long)lists * (beams + 1), std::max(max_lines, lines));
+    }
 };
 
 // The lane cones' work space for a set of chunks: the longest line, the lists
@@ -525,15 +528,17 @@ int pipeline(ee_context* c, const PipeArgs& A) {
     EE_CUDA(cudaStreamSynchronize(s));
     std::vector<int> starts;
     std::vector<ChunkDims> dims;
+    const int lists = c->P.mode == EE_KERNEL_EXP ? c->P.nrays : 0;  // per beam
     for (int b = 0; b < n; b++) {
         EeBeamGeomHead& G = hg[b];
         if (G.status != 0) return fail(G.status, "beam %d: %s", b, status_text(G.status));
         c->last_info.push_back(beam_info(c->h_specs.p[b], G));
-        // a beam's share of the budget: its REV arena and TERMA gradient; the
-        // lane cones' scratch takes a quarter at most
+        // a beam's share of the budget: its REV arena, TERMA gradient and tile
+        // lists; the lane cones' scratch takes a quarter at most
         const long long quads = adj ? ee_quad_vol(c->h_specs.p[b].tn) : 0;
         if (starts.empty() || b - starts.back() >= kTermaBeams ||
-            dims.back().bytes() + 4 * G.store_total + 16 * quads > c->max_batch_bytes / 4 * 3) {
+            dims.back().bytes_with(G.store_total, quads, G.max_lines, lists, b - starts.back()) >
+                c->max_batch_bytes / 4 * 3) {
             starts.push_back(b);
             dims.push_back(ChunkDims());
             dims.back().q0 = c->h_specs.p[b].q_off;
@@ -1290,7 +1295,8 @@ int ee_plan_create(ee_context* c, const ee_beam* beams, int nbeams, const float*
         // the arenas in three quarters of the budget, as pipeline()
         const long long quads = pl->adjoint ? ee_quad_vol(S.tn) : 0;
         if (pl->starts.empty() || b - pl->starts.back() >= kTermaBeams ||
-            pl->dims.back().bytes() + 4 * B.rev + 16 * quads > c->max_batch_bytes / 4 * 3) {
+            pl->dims.back().bytes_with(B.rev, quads, B.max_lines, expm ? c->P.nrays : 0, b - pl->starts.back()) >
+                c->max_batch_bytes / 4 * 3) {
             pl->starts.push_back(b);
             pl->dims.push_back(ChunkDims());
             pl->dims.back().q0 = S.q_off;

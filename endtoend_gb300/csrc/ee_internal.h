@@ -282,6 +282,12 @@ inline int ee_cone_warps(int max_line, long long limit, long long arena) {
     return (int)(n < 152 ? 152 : (n > EE_CONE_MAX_WARPS ? EE_CONE_MAX_WARPS : n)) & ~(EE_CONE_BLOCK_WARPS - 1);
 }
 inline int ee_cone_tiles_cap(int max_lines) { return max_lines / 32 + 1; }
+// Bytes of a chunk that its scratch limit counts, apart from the warps' scratch:
+// REV arena, TERMA gradient, and the lists of the lane cones with a count, the
+// tiles and their marks.
+inline long long ee_chunk_bytes(long long rev, long long quads, long long lists, int max_lines) {
+    return 4 * rev + 16 * quads + lists * (4 + 5ll * ee_cone_tiles_cap(max_lines));
+}
 // kernel preferences of the current device; before the first launch on it
 void ee_kernel_setup();
 // the cones write every sample that k_gather reads; without work space (exp
