@@ -26,49 +26,6 @@ __device__ __forceinline__ float snap_ceilf(float v) {
     return fabsf(v - r) <= 1e-3f ? r : ceilf(v);
 }
 
-// tex3D<float> with linear filtering, unnormalised coordinates and border
-// addressing, written as an explicit FP32 trilinear gather.  (x,y,z) are
-// texel-space coordinates after the -0.5 texel-centre shift.
-__device__ __forceinline__ float tri_border(const float* __restrict__ v, int nx, int ny, int nz, float x, float y,
-                                            float z) {
-    // all eight texels outside (or a NaN coordinate): the border value 0
-    if (!(x > -1.f && x < (float)nx && y > -1.f && y < (float)ny && z > -1.f && z < (float)nz)) return 0.f;
-    float fx = floorf(x), fy = floorf(y), fz = floorf(z);
-    int i = (int)fx, j = (int)fy, k = (int)fz;
-    float ax = x - fx, ay = y - fy, az = z - fz;
-    long long sxy = (long long)nx * ny;
-    if (i >= 0 && j >= 0 && k >= 0 && i + 1 < nx && j + 1 < ny && k + 1 < nz) {
-        const float* p = v + i + (long long)nx * j + sxy * k;
-        float c000 = __ldg(p), c100 = __ldg(p + 1), c010 = __ldg(p + nx), c110 = __ldg(p + nx + 1);
-        float c001 = __ldg(p + sxy), c101 = __ldg(p + sxy + 1), c011 = __ldg(p + sxy + nx), c111 = __ldg(p + sxy + nx + 1);
-        float c00 = c000 + ax * (c100 - c000), c10 = c010 + ax * (c110 - c010);
-        float c01 = c001 + ax * (c101 - c001), c11 = c011 + ax * (c111 - c011);
-        float c0 = c00 + ay * (c10 - c00), c1 = c01 + ay * (c11 - c01);
-        return c0 + az * (c1 - c0);
-    }
-    float acc = 0.f;
-#pragma unroll
-    for (int dk = 0; dk < 2; dk++) {
-        int kk = k + dk;
-        if (kk < 0 || kk >= nz) continue;
-        float wz = dk ? az : 1.f - az;
-#pragma unroll
-        for (int dj = 0; dj < 2; dj++) {
-            int jj = j + dj;
-            if (jj < 0 || jj >= ny) continue;
-            float wy = dj ? ay : 1.f - ay;
-#pragma unroll
-            for (int di = 0; di < 2; di++) {
-                int ii = i + di;
-                if (ii < 0 || ii >= nx) continue;
-                float wx = di ? ax : 1.f - ax;
-                acc += wx * wy * wz * __ldg(v + ii + (long long)nx * jj + sxy * kk);
-            }
-        }
-    }
-    return acc;
-}
-
 // Vector reduction of four floats into a 16-byte aligned quad of global
 // memory (red.global.add.v4.f32, sm_90+): no value comes back, unlike an
 // atomicAdd whose result the caller ignores.
@@ -128,11 +85,12 @@ __device__ __forceinline__ bool brick_cell(const Brick& B, float x, float y, flo
     return (unsigned)i < (unsigned)(B.n0 - 1) && (unsigned)j < (unsigned)(B.n1 - 1) && (unsigned)k < (unsigned)(B.n2 - 1);
 }
 
-// tri_border on a bricked box at a point whose corners all lie in it: the same
-// weights and order.  The corners are addressed from the first one by per-axis
+// tex3D<float> with linear filtering, unnormalised coordinates and border
+// addressing, as an explicit FP32 gather from a bricked box, at a point (the
+// texel-centre shift of -0.5 taken) whose corners all lie in the box.  The corners are addressed from the first one by per-axis
 // steps (+1, +4, +16 inside a brick; +61, +sy - 12, +sz - 48 across a brick
 // face), which with one range test per axis saves the forward cone 7 % against a
-// brick offset per corner and tri_border's tests.
+// brick offset per corner with a test each.
 __device__ __forceinline__ float tri_brick_cell(const float* __restrict__ v, const Brick& B, float x, float y, float z,
                                                 int i, int j, int k) {
     const float ax = x - (float)i, ay = y - (float)j, az = z - (float)k;
@@ -147,7 +105,7 @@ __device__ __forceinline__ float tri_brick_cell(const float* __restrict__ v, con
     return c0 + az * (c1 - c0);
 }
 
-// tri_border on a bricked box at any other point: the corner values that
+// The same at any other point: the corner values that
 // exist, weighted; 0 from one cell outside the box on.  Callers keep it out of
 // their unrolled samples: there it was a quarter of the forward cone's code and
 // a third of the gather's, more than the instruction cache holds.
@@ -179,7 +137,7 @@ __device__ __forceinline__ float tri_brick_edge(const float* __restrict__ v, con
     return acc;
 }
 
-// tri_border on a bricked box.
+// The same at any point.
 __device__ __forceinline__ float tri_brick(const float* __restrict__ v, const Brick& B, float x, float y, float z) {
     int i, j, k;
     return brick_cell(B, x, y, z, i, j, k) ? tri_brick_cell(v, B, x, y, z, i, j, k) : tri_brick_edge(v, B, x, y, z);
@@ -265,7 +223,7 @@ __device__ __forceinline__ unsigned quad_z(const Brick& Q, int z) {
     return (unsigned)(z >> 2) * (unsigned)Q.sz + ((unsigned)(z & 3) << 4);
 }
 
-// Transpose of tri_border: scatter g with the trilinear weights, one 16-byte
+// Transpose of tri_brick: scatter g with the trilinear weights, one 16-byte
 // reduction per z corner.  Corners outside the box in x or y fall on values that
 // quad_value does not read, those in z are left out.  Against a reduction per
 // (y, z) corner row into the voxels, and a second one where the row crosses a

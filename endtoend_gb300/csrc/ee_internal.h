@@ -303,6 +303,7 @@ cudaError_t ee_launch_gather(const EeParams& P, const EeBeamSpec* specs, const E
 cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms,
                                const float* dose_grad, float* rev_grad, const EeConeWork& work, int nbeams,
                                int max_lines, int max_tiles, cudaStream_t s);
+// (exp mode: with work space only)
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
                              const EeConeWork& work, float4* terma_grad, int nbeams, int max_lines, int max_line,
                              cudaStream_t s);

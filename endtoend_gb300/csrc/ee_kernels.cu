@@ -653,64 +653,6 @@ __device__ __forceinline__ void line_scan(const float* rho, const float* T, int 
     }
 }
 
-// Transpose of line_scan<FWD> for the TERMA adjoint.  With g_i the incoming
-// REV-dose gradient (already / nphi, zero at sentinels) and im the forward
-// walk's previous sample of i,
-//   Z_i = c g_i + h_i^2 Z_{i+1}         (walking opposite to FWD),
-//   Tbar_im += c g_i (1 - h_im) + Z_{i+1} h_i (1 - h_im h_i),
-// with the same chunked scan.  im is the next sample of this walk, so its
-// h is computed once and carried.
-template <bool FWD>
-__device__ __forceinline__ void line_scan_T(const float* rho, const float* g, int n, int lane, float delr,
-                                            const float* prm, float* Tb) {
-    const float c1 = prm[0] / prm[1], c2 = prm[2] / prm[3];
-    const float e1 = -0.5f * prm[1] * delr, e2 = -0.5f * prm[3] * delr;
-    const int cs = ((n + 31) >> 5) | 1;
-    const int v0 = min(n, lane * cs), v1 = min(n, v0 + cs);
-    // pass 1: compose Z -> h^2 Z + c g over the chunk
-    float F1 = 1.f, U1 = 0.f, F2 = 1.f, U2 = 0.f;
-    for (int v = v0; v < v1; v++) {
-        const int i = FWD ? n - 1 - v : v;
-        const float r = rho[i];
-        float gi = 0.f, h1 = 1.f, h2 = 1.f;
-        if (r >= 0.f) { gi = g[i]; h1 = __expf(e1 * r); h2 = __expf(e2 * r); }
-        const float f1 = h1 * h1, f2 = h2 * h2;
-        U1 = fmaf(f1, U1, c1 * gi); F1 *= f1;
-        U2 = fmaf(f2, U2, c2 * gi); F2 *= f2;
-    }
-    warp_affine_scan(lane, F1, U1, F2, U2);
-    float Z1 = __shfl_up_sync(FULL, U1, 1), Z2 = __shfl_up_sync(FULL, U2, 1);
-    if (lane == 0) { Z1 = 0.f; Z2 = 0.f; }
-    // pass 2: replay, emitting the TERMA-gradient contributions
-    float h1 = 1.f, h2 = 1.f, gi = 0.f;
-    bool vi = false;
-    if (v0 < v1) {
-        const int i = FWD ? n - 1 - v0 : v0;
-        const float r = rho[i];
-        if (r >= 0.f) { vi = true; gi = g[i]; h1 = __expf(e1 * r); h2 = __expf(e2 * r); }
-    }
-    for (int v = v0; v < v1; v++) {
-        const int i = FWD ? n - 1 - v : v;
-        const int im = FWD ? i - 1 : i + 1;
-        float hm1 = 1.f, hm2 = 1.f, gm = 0.f;
-        bool vm = false;
-        if (im >= 0 && im < n) {
-            const float rm = rho[im];
-            if (rm >= 0.f) { vm = true; gm = g[im]; hm1 = __expf(e1 * rm); hm2 = __expf(e2 * rm); }
-        }
-        if (vm) {
-            const float c = c1 * gi * (1.f - hm1) + Z1 * h1 * (1.f - hm1 * h1) + c2 * gi * (1.f - hm2) +
-                            Z2 * h2 * (1.f - hm2 * h2);
-            Tb[im] += c;  // each im has exactly one i per pass
-        }
-        (void)vi;
-        Z1 = fmaf(h1 * h1, Z1, c1 * gi);
-        Z2 = fmaf(h2 * h2, Z2, c2 * gi);
-        // the next step's sample is im
-        h1 = hm1; h2 = hm2; gi = gm; vi = vm;
-    }
-}
-
 // --------------------------------------------------- cone: table walk ----
 // RowConvolve walk (device.cu:126-211) over shared memory with exact FP32
 // linear interpolation of the cumulative kernel between radial boundaries.
@@ -1893,7 +1835,7 @@ __global__ void __launch_bounds__(EE_CONE_BLOCK_WARPS * 32, EE_CONE_SM_WARPS / E
     });
 }
 
-// Adjoint of k_cone followed by the transpose of the REV TERMA resample:
+// Adjoint of k_cone with the table walk, followed by the transpose of the REV TERMA resample:
 // terma_grad (bbox grid) += R_T^T C^T rev_grad.
 __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const EeBeamSpec* __restrict__ specs,
                                                             const EeBeamGeom* __restrict__ geoms,
@@ -1905,15 +1847,13 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
     const EeBeamGeom& G = geoms[b];
     float* tabK = sm + (size_t)CONE_WARPS * 3 * maxL;
     float* tabR = tabK + 2 * EE_MAX_RADII;
-    if (P.mode != EE_KERNEL_EXP) {
-        const EeRayConst& RC = P.rays[ray];
-        for (int k = threadIdx.x; k < P.nradii; k += blockDim.x) {
-            tabK[k] = P.cumkern[RC.row_fwd * P.nradii + k];
-            tabK[EE_MAX_RADII + k] = P.cumkern[RC.row_rev * P.nradii + k];
-            tabR[k] = P.radii[k];
-        }
-        __syncthreads();
+    const EeRayConst& RC = P.rays[ray];
+    for (int k = threadIdx.x; k < P.nradii; k += blockDim.x) {
+        tabK[k] = P.cumkern[RC.row_fwd * P.nradii + k];
+        tabK[EE_MAX_RADII + k] = P.cumkern[RC.row_rev * P.nradii + k];
+        tabR[k] = P.radii[k];
     }
+    __syncthreads();
     if (G.status != 0) return;
     const EeRayGeom& R = G.ray[ray];
     const int line = blockIdx.x * CONE_WARPS + warp;
@@ -1939,17 +1879,10 @@ __global__ void __launch_bounds__(CONE_WARPS * 32) k_cone_T(EeParams P, const Ee
         Tb[k] = 0.f;
     }
     __syncwarp();
-    const EeRayConst& RC = P.rays[ray];
-    if (P.mode == EE_KERNEL_EXP) {
-        line_scan_T<true>(rho, g, n, lane, P.lng, P.expp + 4 * RC.row_fwd, Tb);
-        __syncwarp();
-        line_scan_T<false>(rho, g, n, lane, P.lng, P.expp + 4 * RC.row_rev, Tb);
-    } else {
-        for (int k = lane; k < n; k += 32) {
-            if (rho[k] >= 0.f && g[k] != 0.f) {
-                table_walk(rho, nullptr, n, k, -1, tabK, tabR, P.nradii, P.lng, Tb, g[k]);
-                table_walk(rho, nullptr, n, k, +1, tabK + EE_MAX_RADII, tabR, P.nradii, P.lng, Tb, g[k]);
-            }
+    for (int k = lane; k < n; k += 32) {
+        if (rho[k] >= 0.f && g[k] != 0.f) {
+            table_walk(rho, nullptr, n, k, -1, tabK, tabR, P.nradii, P.lng, Tb, g[k]);
+            table_walk(rho, nullptr, n, k, +1, tabK + EE_MAX_RADII, tabR, P.nradii, P.lng, Tb, g[k]);
         }
     }
     __syncwarp();
@@ -2721,7 +2654,8 @@ cudaError_t ee_launch_gather_T(const EeParams& P, const EeBeamSpec* specs, const
 cudaError_t ee_launch_cone_T(const EeParams& P, const EeBeamSpec* specs, const EeBeamGeom* geoms, const float* rev_grad,
                              const EeConeWork& work, float4* terma_grad, int nbeams, int max_lines, int max_line,
                              cudaStream_t s) {
-    if (P.mode == 1 && work.scratch) {
+    if (P.mode == EE_KERNEL_EXP) {
+        if (!work.scratch) return cudaErrorInvalidValue;  // no warp-per-line form of the exp adjoint
         const int cap = ee_cone_tiles_cap(max_lines);
         k_cone_tiles<<<dim3(P.nrays, nbeams), 256, 0, s>>>(P, geoms, 0.f, work.touched, work.counts, work.tiles, cap);
         k_cone_T_lane<<<work.warps / EE_CONE_BLOCK_WARPS, EE_CONE_BLOCK_WARPS * 32, 0, s>>>(
