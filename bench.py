@@ -461,11 +461,12 @@ def run_reference(args, ws, rank):
 
 
 # DRAM bytes (read + write) per crop-box voxel of each stage, from ncu
-# captures of the chain kernels on four beams of 8^2..40^2 beamlets on this
-# phantom (rate x time of one launch each / sum of V_beam = 5.76 M);
-# roofline.traffic scales the dominant stage's figure to the profiled step.
-DRAM_BYTES_PER_VBEAM = {"terma": 8.5, "cone": 109.6, "gather": 55.7, "gather_T": 65.4, "cone_T": 77.4,
-                        "terma_T": 9.1, "geometry": 0.0}
+# captures of the chain kernels under `--profile-case exp --profile-beams 4`
+# (four beams spread over the batch; rate x time of one launch each / sum of
+# V_beam = 4.58 M); roofline.traffic scales the dominant stage's figure to the
+# profiled step.
+DRAM_BYTES_PER_VBEAM = {"terma": 13.0, "cone": 238.3, "gather": 95.4, "gather_T": 154.2, "cone_T": 185.9,
+                        "terma_T": 15.4, "geometry": 0.0}
 
 
 def algorithmic_bytes(infos):
@@ -728,7 +729,7 @@ def main():
             "plain": {"value": plain, "unit": UNIT, "beams": npl, "p50_ms": float(np.percentile(lat_ms, 50)),
                       "p99_ms": float(np.percentile(lat_ms, 99))},
             "batched_over_plain": value / plain,
-            "pipeline": {"value": pipeline_value, "unit": UNIT, "note": "same batch, direct call (host geometry read-back per chunk)"},
+            "pipeline": {"value": pipeline_value, "unit": UNIT, "note": "same batch, direct call (one host geometry read-back)"},
             "table_measured_6x": table,
             "plan": plan_info,
             "serving": serving,

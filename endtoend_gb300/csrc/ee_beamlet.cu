@@ -11,7 +11,8 @@
 // column.
 //
 // GB300 organisation:
-//   k_bl_sources one warp per (pillar, unit of depth): the few REV samples
+//   k_bl_sources one warp, or several where beamlets are wide or few, per
+//                direction, pillar and 32 units of depth: the REV samples
 //                around that piece of the beamlet's footprint, each with the
 //                reference's pillar lookup and beamlet test; samples inside
 //                are queued and marked on their line (the reference looks at
@@ -308,7 +309,7 @@ __device__ __forceinline__ f3 bl_rev_point(const BlGrid& G, const BlPillar& Q, c
     return mk(fmaf(-R.rs[0], R.rcp[0], r.x), fmaf(-R.rs[1], R.rcp[1], r.y), fmaf(-R.rs[2], R.rcp[2], r.z));
 }
 
-// Pass 1, one warp per direction, pillar and 32 units of pillar depth.  A
+// Pass 1, `slices` warps per direction, pillar and 32 units of pillar depth.  A
 // unit's candidates are the REV samples in the box around that piece of the
 // beamlet's footprint (3^3 to 4^3 for a beamlet of a voxel or two): each lane
 // sets one unit's box up, and the warp then walks the candidates of all its
@@ -321,8 +322,7 @@ __device__ __forceinline__ f3 bl_rev_point(const BlGrid& G, const BlPillar& Q, c
 // one add per warp or so and not one per sample.  Bound by the instructions of
 // the tests.  A thread per REV sample (0.2 % of them are in a beamlet) took
 // 272 us per direction of about 110 beamlets on 200 x 200 x 160 at 2 mm, a warp
-// per unit 27 us; this takes 5.2 us.  `slices` warps share the candidates of 32
-// units (ee_bl_source_slices).
+// per unit 27 us; this takes 5.2 us.
 constexpr int BL_SRC_WARPS = 4, BL_SRC_BUF = 128;
 
 __global__ void __launch_bounds__(BL_SRC_WARPS * 32)

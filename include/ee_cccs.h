@@ -227,7 +227,9 @@ int ee_beam_dose_noalloc(ee_context *ctx, const ee_beam *beam, const float *d_fl
  * chain into one CUDA graph.
  * ee_plan_launch replays that graph on the context stream with no host
  * synchronisation (new fluence / gradient values are read from the same
- * buffers); ee_plan_status then reports per-beam failures. */
+ * buffers); ee_plan_status then reports per-beam failures.
+ * ee_plan_info: threads per block of the cone kernels (*lane_block: the same
+ * for every plan), device bytes of the plan's buffers and chunks of beams. */
 typedef struct ee_plan ee_plan;
 int ee_plan_create(ee_context *ctx, const ee_beam *beams, int nbeams, const float *d_fluence, float *d_dose,
                    const float *d_dose_grad, float *d_fluence_grad, ee_plan **plan);
